@@ -456,3 +456,42 @@ def test_materialisation_depth_boundaries(native, oracle, monkeypatch, depth):
             finally:
                 eng.close()
             assert_same(out, want, g, src, f"depth={depth} narrow={narrow} pinned={pinned} W={words}")
+
+
+def _caterpillar(native, n):
+    """A spine whose vertices carry six leaves each: degree 8, about two edges
+    per vertex -- a road-like graph with more out-edges than one round of a
+    frontier vertex's lanes takes."""
+    spine = (n + 6) // 7
+    e = [(i, i + 1) for i in range(spine - 1)]
+    e += [(i % spine, v) for i, v in enumerate(range(spine, n))]
+    return native.CsrGraph.from_edge_list(n, e + [(v, u) for u, v in e])
+
+
+@pytest.mark.parametrize("graph", ["small_grid", "wide_grid", "caterpillar"])
+def test_cta_block_forms(native, gpu_engine, oracle, graph):
+    """Every block form of the CTA path (chosen by the sources per SM and the
+    vertex count), at the source counts where it changes, with and without
+    edge records, rows and statistics."""
+    torch = pytest.importorskip("torch")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = {"small_grid": lambda: native.Grid2D(33, 31).graph,
+         "wide_grid": lambda: native.Grid2D(2, 16384).graph,  # V = 32,768: the wide form
+         "caterpillar": lambda: _caterpillar(native, 2000)}[graph]()
+    counts = [1, sms + 1] if graph == "wide_grid" else [1, sms, sms + 1, 3 * sms, 3 * sms + 1]
+    for S in counts:
+        src = np.random.default_rng(S).integers(0, g.num_vertices, S).astype(np.uint32)
+        want = oracle.ms_bfs_threaded(g.num_vertices, g.row_offsets, g.col_indices, src)
+        got = gpu_engine.run_ms_bfs_with_method(native.GpuBfsMethod.WorkgroupPersistentBfs, g, src)
+        assert gpu_engine.last_stats["path"] == 4
+        assert_same(got, want, g, src, f"{graph} S={S}")
+    st = gpu_engine.run_ms_bfs_stats(g, src)
+    rows = want.reshape(S, -1).astype(np.int64)
+    assert np.array_equal(st["distance_sum"].astype(np.int64), rows.sum(1))  # connected graphs
+    assert np.array_equal(st["eccentricity"], rows.max(1))
+    assert (st["reached"] == g.num_vertices).all()
+    # no edge records: the same structure with one hub beyond road-like degrees
+    hub = native.star_graph(600)
+    src = np.arange(0, 600, 7, dtype=np.uint32)
+    got = gpu_engine.run_ms_bfs_with_method(native.GpuBfsMethod.WorkgroupPersistentBfs, hub, src)
+    assert_same(got, oracle.ms_bfs_fifo(600, hub.row_offsets, hub.col_indices, src), hub, src, "star")

@@ -28,128 +28,256 @@ namespace cg = cooperative_groups;
 namespace msbfs {
 
 constexpr uint32_t CTA_DIST_MAX = 0xffffffffu;
-// Latency form's block (ms; road 339x338 + 5,000 edges S=256 / S=1, grid
-// 64x64 S=64): 512 threads 1.216 / 0.964 / 0.123, 256 threads 1.148 /
-// 0.912 / 0.109, 128 threads 1.402 / 1.275 / 0.109. A level of a few
-// hundred frontier vertices keeps 256 threads busy, and a smaller block's
-// barrier costs less.
-#ifndef MSBFS_CTA_LAT_THREADS
-#define MSBFS_CTA_LAT_THREADS 256
-#endif
-constexpr int CTA_THREADS = MSBFS_CTA_LAT_THREADS;
-// Global-bitmap mode (graphs whose bitmap does not fit shared memory, e.g.
-// road 1448 x 1448) keeps 512-thread blocks: its frontiers are wider.
-constexpr int CTA_GB_THREADS = 512;
-// Two forms. The latency form: blocks of CTA_THREADS threads, 3 resident
-// per SM (4 edge records in flight, the shortest level latency). The
-// throughput form, for calls with more sources than 3 blocks per SM can
-// hold: CTA_TPUT_THREADS threads and CTA_TPUT_MINB resident blocks per SM
-// (2 records in flight): many-source calls are bound by how many BFSs run
-// at once, single ones by the per-level latency chain.
-constexpr int CTA_MINB_LATENCY = 3;
-// Road 339x338 + 5,000 edges, S=2048 (threads x blocks per SM, ms): 512 x 4
-// 5.41, 384 x 5 4.92, 256 x 6 5.16, 256 x 7 4.46, 256 x 8 4.78, 128 x 12
-// 6.68, 128 x 16 6.78. Each block waits at one barrier per level while a
-// few of its warps walk a frontier of a few hundred vertices: smaller blocks
-// put more sources in flight, until too few threads share a level's work.
+constexpr uint32_t CTA_FULL = 0xffffffffu;
+// Block forms of cta_bfs_kernel: threads, resident blocks per SM it is built
+// for, lanes per frontier vertex. One block walks a whole level between two
+// barriers, so a call of few sources wants every frontier vertex in one
+// sweep of the block, a call of many wants many blocks per SM. The form is
+// chosen by the blocks an SM will hold (the call's sources per SM, at most
+// what the bitmaps leave room for). ms a pass, three calls in flight:
+//   one block per SM    road 339x338 S=1 / road 1000x1000 S=250 / grid 64x64
+//     CTA_WIDE          S=64: 1,024 threads x 4 lanes 0.197 / 5.62 / 0.031,
+//     CTA_SMALL         512 x 4 0.233 / 7.68 / 0.028, 256 x 4 0.38 / - /
+//                       0.030, 1,024 x 2 0.240 / - / 0.038 (a small graph's
+//                       frontier fits 128 vertices, and its barrier is cheaper)
+//   two or three        road 339x338 S=256: 512 x 2 0.445, 512 x 4 0.498,
+//     CTA_MID           256 x 2 0.445 (alone 0.99 against 0.89), 1,024 x 4 0.60
+//   four or more        road 339x338 S=2,048: 256 threads x 2 lanes x 8 blocks
+//     CTA_TPUT          2.84, 192 x 2 x 9 2.80, 256 x 1 x 7 3.07, 256 x 2 x 7
+//                       2.90, 256 x 4 x 7 3.11, 128 x 2 x 14 3.60
+// Global-bitmap mode (graphs whose bitmap does not fit shared memory) uses
+// CTA_MID and CTA_TPUT.
 #ifndef MSBFS_CTA_TPUT_THREADS
 #define MSBFS_CTA_TPUT_THREADS 256
 #endif
 #ifndef MSBFS_CTA_TPUT_MINB
-#define MSBFS_CTA_TPUT_MINB 7
+#define MSBFS_CTA_TPUT_MINB 8
 #endif
-constexpr int CTA_TPUT_THREADS = MSBFS_CTA_TPUT_THREADS;
-constexpr int CTA_MINB_THROUGHPUT = MSBFS_CTA_TPUT_MINB;
-static_assert(CTA_MINB_THROUGHPUT > CTA_MINB_LATENCY, "the throughput form holds more blocks");
+enum : int { CTA_WIDE = 0, CTA_SMALL = 1, CTA_MID = 2, CTA_TPUT = 3 };
+template <int FORM>
+struct CtaForm {
+  static constexpr int THREADS = FORM == CTA_WIDE ? 1024 : FORM == CTA_TPUT ? MSBFS_CTA_TPUT_THREADS : 512;
+  static constexpr int MINB = FORM == CTA_WIDE ? 1 : FORM == CTA_TPUT ? MSBFS_CTA_TPUT_MINB : 3;
+  static constexpr int LPV = FORM <= CTA_SMALL ? 4 : 2;
+};
+// Vertices from which one block per SM is the wide one: about the graph whose
+// frontiers (of the order of the square root) exceed the small one's sweep.
+constexpr size_t CTA_WIDE_VERTICES = 32768;
+constexpr size_t CTA_MID_BLOCKS = 3;  // most blocks per SM of the middle form
 // Global-bitmap mode keeps its per-block scratch (queue slab + bitmap) within
 // this many bytes by shrinking the grid.
 constexpr size_t CTA_GLOBAL_SCRATCH_BYTES = 4ull << 30;
-// Frontier entries per shared-memory queue half (16 KB of vertex ids, 32 KB
-// of edge ranges).
+// Frontier entries per shared-memory queue half (16 KB).
 constexpr uint32_t CTA_SMEM_QUEUE = 4096;
-// Cluster form: threads of rank 0 (which walks every frontier) and edge
-// records each keeps in flight. Road 1448 x 1448, one source: 1,024 threads
-// and 4 records 9.8 ms, 1,024 and 2 10.6 ms, 512 and 4 12.3 ms (global-bitmap
-// mode 17.6 ms).
+// Cluster form: threads of rank 0 (which walks every frontier) and lanes per
+// frontier vertex. Road 1448 x 1448, S=64, ms a pass: 1 lane 6.79, 2 lanes
+// 6.99, 4 lanes 7.32 (one edge at a time, with a visited test before each
+// atomic 9.09). 512 threads were a quarter slower than 1,024.
 #ifndef MSBFS_CTA_CLUSTER_THREADS
 #define MSBFS_CTA_CLUSTER_THREADS 1024
 #endif
 constexpr int CTA_CLUSTER_THREADS = MSBFS_CTA_CLUSTER_THREADS;
-#ifndef MSBFS_CTA_CLUSTER_ER_BATCH
-#define MSBFS_CTA_CLUSTER_ER_BATCH 4
-#endif
-constexpr int CTA_CLUSTER_ER_BATCH = MSBFS_CTA_CLUSTER_ER_BATCH;
+constexpr int CTA_CLUSTER_LPV = 1;
+
+// Frontier entries. ER: the graph carries edge records, 8 bytes per edge
+// {target, target's edge range packed as begin << 4 | count} (built once per
+// road-like graph: at most 8 out-edges, fewer than 2^28 edges), and a queue
+// entry is the packed edge range of a frontier vertex instead of its id.
+// Expanding a vertex then costs one dependent L2 round trip per level (its
+// edge records) instead of three (queue entry, offsets, adjacency): on a
+// ~4,000-level road graph the per-level latency chain is what a traversal's
+// time is made of.
+//
+// Queue: the first `qh` entries of a level's frontier sit in shared memory
+// (two halves, by level parity), the rest in one global slab of V words per
+// block. The frontiers of consecutive levels are disjoint vertex sets, so
+// |F_L| + |F_L+1| <= V: in the slab even levels sit at the front and odd
+// levels at the back.
+// Shared-memory accesses by 32-bit address: through generic pointers (a queue
+// entry may also sit in the slab) each would pay the generic path's latency.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t r;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
+  return r;
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t x) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(x) : "memory");
+}
+__device__ __forceinline__ uint32_t atoms_or(uint32_t a, uint32_t x) {
+  uint32_t r;
+  asm volatile("atom.shared.or.b32 %0, [%1], %2;" : "=r"(r) : "r"(a), "r"(x) : "memory");
+  return r;
+}
+__device__ __forceinline__ uint32_t atoms_add(uint32_t a, uint32_t x) {
+  uint32_t r;
+  asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(r) : "r"(a), "r"(x) : "memory");
+  return r;
+}
+
+template <bool ER>
+struct CtaQueue {
+  uint32_t sq;     // shared-memory address of the halves
+  uint32_t* slab;  // global memory
+  uint32_t qh, V;
+  const uint32_t* off;
+  __device__ __forceinline__ uint32_t* slab_at(uint32_t lv, uint32_t i) const {
+    return (lv & 1) ? slab + (V - 1 - i) : slab + i;
+  }
+  __device__ __forceinline__ uint32_t half(uint32_t lv) const {
+    return sq + ((lv & 1) ? 4 * qh : 0);
+  }
+  // The frontier of level 0 (the halves may hold nothing: qh == 0).
+  __device__ __forceinline__ void put_source(uint32_t u) const {
+    uint32_t x = u;
+    if constexpr (ER) {
+      const uint32_t b = __ldg(off + u);
+      x = b << 4 | (__ldg(off + u + 1) - b);
+    }
+    if (qh)
+      sts32(sq, x);
+    else
+      slab[0] = x;
+  }
+};
+
+// Expands the n_in frontier entries of `level`: LPV lanes take one vertex,
+// each BATCH of its edges per round. Each step of a round -- edge records,
+// bitmap atomics, queue places -- is issued for all edges
+// before the next step needs a result, so a level is one pass through that
+// latency chain, not one pass per edge. `mark(v, bit)` sets v's visited bit
+// and returns the bitmap word as it was (testing the bit first only adds a
+// step: road 339x338 S=2,048 3.25 -> 3.08 ms without it). New vertices get their places in the next frontier with one shared-memory atomicAdd per
+// warp and round (ballot prefix sums). A level with few vertices is bound by
+// the length of this instruction sequence (about 6 cycles an instruction
+// with one warp per scheduler), hence the straight-line common case: queue
+// entries read without a per-lane branch while the frontier fits the
+// shared-memory half (its length is a multiple of 32, so a warp's entries
+// past n_in are still inside it).
+template <bool ER, int THREADS, int LPV, int BATCH, typename Mark>
+__device__ __forceinline__ void cta_expand(const CtaParams& p, const CtaQueue<ER>& q,
+                                           uint32_t level, uint32_t n_in, uint32_t cnt,
+                                           uint32_t* row, Mark&& mark) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t sub = lane % LPV;
+  const uint32_t nd = level + 1;
+  const uint32_t hin = q.half(level), hout = q.half(nd);
+  for (uint32_t base = (threadIdx.x - lane) / LPV; base < n_in; base += THREADS / LPV) {
+    const uint32_t i = base + lane / LPV;
+    uint32_t x = 0, e = 0, n = 0;
+    if (n_in <= q.qh) {
+      x = lds32(hin + 4 * i);
+    } else if (i < n_in) {
+      if (i < q.qh)
+        x = lds32(hin + 4 * i);
+      else
+        x = *q.slab_at(level, i);
+    }
+    if constexpr (ER) {
+      e = x >> 4;
+      n = i < n_in ? x & 15u : 0u;
+    } else if (i < n_in) {
+      e = __ldg(q.off + x);
+      n = __ldg(q.off + x + 1) - e;
+    }
+    for (;;) {
+      uint32_t v[BATCH], nx[BATCH], was[BATCH];
+      bool fresh[BATCH];
+#pragma unroll
+      for (int k = 0; k < BATCH; ++k) {
+        v[k] = nx[k] = 0;
+        fresh[k] = sub + k * LPV < n;
+        if (fresh[k]) {
+          if constexpr (ER) {
+            const uint2 r = __ldg(p.erec + e + sub + k * LPV);
+            v[k] = r.x;
+            nx[k] = r.y;
+          } else {
+            v[k] = nx[k] = __ldg(p.idx + e + sub + k * LPV);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < BATCH; ++k) {
+        was[k] = 0;
+        if (fresh[k]) was[k] = mark(v[k], __funnelshift_l(0u, 1u, v[k]));
+      }
+      uint32_t total, before;  // of the warp, of the lower lanes
+      uint32_t lt;
+      asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+#pragma unroll
+      for (int k = 0; k < BATCH; ++k)
+        fresh[k] = fresh[k] && !(was[k] & __funnelshift_l(0u, 1u, v[k]));
+      if constexpr (BATCH == 1) {
+        const uint32_t b0 = __ballot_sync(CTA_FULL, fresh[0]);
+        total = __popc(b0);
+        before = __popc(b0 & lt);
+      } else {
+        static_assert(BATCH <= 7, "counts of three bits");
+        uint32_t c = 0;
+#pragma unroll
+        for (int k = 0; k < BATCH; ++k) c += fresh[k] ? 1u : 0u;
+        const uint32_t b0 = __ballot_sync(CTA_FULL, c & 1u), b1 = __ballot_sync(CTA_FULL, c & 2u);
+        total = __popc(b0) + 2 * __popc(b1);
+        before = __popc(b0 & lt) + 2 * __popc(b1 & lt);
+        if constexpr (BATCH >= 4) {
+          const uint32_t b2 = __ballot_sync(CTA_FULL, c & 4u);
+          total += 4 * __popc(b2);
+          before += 4 * __popc(b2 & lt);
+        }
+      }
+      if (total) {
+        uint32_t pos = 0;
+        if (lane == 0) pos = atoms_add(cnt, total);
+        pos = __shfl_sync(CTA_FULL, pos, 0) + before;
+#pragma unroll
+        for (int k = 0; k < BATCH; ++k) {
+          if (!fresh[k]) continue;
+          if (row) row[v[k]] = nd;
+          if (pos < q.qh)
+            sts32(hout + 4 * pos, nx[k]);
+          else
+            *q.slab_at(nd, pos) = nx[k];
+          ++pos;
+        }
+      }
+      if (!__any_sync(CTA_FULL, n > LPV * BATCH)) break;
+      e += LPV * BATCH;
+      n -= min(n, (uint32_t)(LPV * BATCH));
+    }
+  }
+}
 
 // GB: the visited bitmap lives in an L2-resident global slab per block (for
 // graphs whose bitmap does not fit shared memory) instead of shared memory.
 //
-// ER: the graph carries edge records {target, target's first edge, target's
-// end edge} (built once per road-like graph), and a queue entry holds the
-// edge range of a frontier vertex instead of its id. Expanding a vertex then
-// costs one dependent L2 round trip per level (its edge records) instead of
-// three (queue entry, offsets, adjacency): on a ~4,000-level road graph the
-// per-level latency chain is what a traversal's time is made of.
-//
-// Queue: the first p.qh entries of a level's frontier sit in shared memory
-// (two halves, by level parity), the rest in one global slab of V words per
-// block (vertex ids: an ER reader looks their offsets up). The frontiers of
-// consecutive levels are disjoint vertex sets, so |F_L| + |F_L+1| <= V: in
-// the slab even levels sit at the front and odd levels at the back.
 // Counters: level L appends through s_cnt[L % 3]; thread 0 clears
 // s_cnt[(L+1) % 3] during level L (last read right after the barrier of
-// level L-2), so a level needs one block barrier.
-template <bool GB, bool ER, int THREADS, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB) cta_bfs_kernel(CtaParams p) {
-  constexpr int CTA_ER_BATCH = MINB >= CTA_MINB_THROUGHPUT ? 2 : 4;
+// level L-2), so a level needs one block barrier. The per-source statistics
+// follow from the frontier sizes, which every thread knows.
+template <bool GB, bool ER, int FORM>
+__global__ void __launch_bounds__(CtaForm<FORM>::THREADS, CtaForm<FORM>::MINB)
+    cta_bfs_kernel(CtaParams p) {
+  constexpr int THREADS = CtaForm<FORM>::THREADS, LPV = CtaForm<FORM>::LPV;
   extern __shared__ __align__(16) uint32_t smem_dyn[];
   __shared__ uint32_t s_src_idx;
   __shared__ uint32_t s_cnt[3];
-  __shared__ unsigned long long s_sum;
-  __shared__ uint32_t s_reached;
   const uint32_t V = p.V;
   const uint32_t words = (V + 31) / 32;
-  const uint32_t QH = p.qh;
   uint32_t* bits = GB ? p.gbits + (size_t)blockIdx.x * words : smem_dyn;
-  // queue halves after the bitmap, 8-byte aligned: ER entries are (eb, ee)
-  uint32_t* sq = smem_dyn + (GB ? 0 : (words + 1) / 2 * 2);
-  uint2* sq2 = reinterpret_cast<uint2*>(sq);
-  uint32_t* slab = p.gqueue + (size_t)blockIdx.x * V;
-  auto slab_at = [&](uint32_t lv, uint32_t i) -> uint32_t* {
-    return (lv & 1) ? slab + (V - 1 - i) : slab + i;
-  };
-  // Edge range [*eb, *ee) of entry i of the frontier of level `lv`.
-  auto q_get = [&](uint32_t lv, uint32_t i, uint32_t* eb, uint32_t* ee) {
-    if constexpr (ER) {
-      if (i < QH) {
-        const uint2 r = sq2[(lv & 1) * QH + i];
-        *eb = r.x;
-        *ee = r.y;
-        return;
-      }
-    }
-    const uint32_t u = i < QH ? sq[(lv & 1) * QH + i] : *slab_at(lv, i);
-    *eb = __ldg(p.off + u);
-    *ee = __ldg(p.off + u + 1);
-  };
-  auto q_put = [&](uint32_t lv, uint32_t i, uint32_t v, uint32_t eb, uint32_t ee) {
-    if (i < QH) {
-      if constexpr (ER)
-        sq2[(lv & 1) * QH + i] = make_uint2(eb, ee);
-      else
-        sq[(lv & 1) * QH + i] = v;
-    } else {
-      *slab_at(lv, i) = v;
-    }
-  };
+  // queue halves after the bitmap
+  const uint32_t sbits = smem_addr(smem_dyn), scnt = smem_addr(s_cnt);
+  const CtaQueue<ER> q{sbits + (GB ? 0 : (words + 1) / 2 * 8),
+                       p.gqueue + (size_t)blockIdx.x * V, p.qh, V, p.off};
 
   for (;;) {
     if (threadIdx.x == 0) {
       s_src_idx = atomicAdd(p.work, 1u);
-      s_sum = 0;
-      s_reached = 0;
       s_cnt[0] = s_cnt[1] = s_cnt[2] = 0;
     }
-    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) bits[i] = 0;
+    for (uint32_t i = threadIdx.x; i < words; i += THREADS) bits[i] = 0;
     __syncthreads();
     const uint32_t si = s_src_idx;
     if (si >= p.num_sources) break;
@@ -158,86 +286,38 @@ __global__ void __launch_bounds__(THREADS, MINB) cta_bfs_kernel(CtaParams p) {
     if (threadIdx.x == 0) {
       bits[src >> 5] = 1u << (src & 31);
       if (row) row[src] = 0;
-      q_put(0, 0, src, __ldg(p.off + src), __ldg(p.off + src + 1));
+      q.put_source(src);
     }
-    uint32_t n_in = 1;
-    uint32_t level = 0, ecc = 0;
-    unsigned long long my_sum = 0;
-    uint32_t my_cnt = 0;
+    uint32_t n_in = 1, level = 0, reached = 0, slot = 0;  // slot: 4 * (level % 3)
+    unsigned long long sum = 0;
     __syncthreads();
     while (n_in) {
-      ecc = level;
-      const uint32_t nd = level + 1;
-      uint32_t* cnt = &s_cnt[level % 3];
-      if (threadIdx.x == 0) s_cnt[(level + 1) % 3] = 0;
-      // Threads sweep the frontier; each expands one vertex's out-edges.
-      for (uint32_t i = threadIdx.x; i < n_in; i += blockDim.x) {
-        uint32_t eb, ee;
-        q_get(level, i, &eb, &ee);
-        if constexpr (ER) {
-          // CTA_ER_BATCH edge records in flight before any visited check
-          // (road vertices have ~2 edges; more would cost registers, and so
-          // resident blocks, for little gain)
-          for (uint32_t e = eb; e < ee; e += CTA_ER_BATCH) {
-            uint4 r[CTA_ER_BATCH];
-#pragma unroll
-            for (int k = 0; k < CTA_ER_BATCH; ++k)
-              if (e + k < ee) r[k] = __ldg(p.erec + e + k);
-#pragma unroll
-            for (int k = 0; k < CTA_ER_BATCH; ++k) {
-              if (e + k >= ee) break;
-              const uint32_t v = r[k].x;
-              const uint32_t bit = 1u << (v & 31);
-              if constexpr (!GB) {
-                if (bits[v >> 5] & bit) continue;
-              }
-              const uint32_t old = atomicOr(&bits[v >> 5], bit);
-              if (old & bit) continue;
-              if (row) row[v] = nd;
-              my_sum += nd;
-              ++my_cnt;
-              q_put(level + 1, atomicAdd(cnt, 1u), v, r[k].y, r[k].z);
-            }
-          }
-        } else {
-          for (uint32_t e = eb; e < ee; ++e) {
-            const uint32_t v = __ldg(p.idx + e);
-            const uint32_t bit = 1u << (v & 31);
-            if constexpr (!GB) {
-              if (bits[v >> 5] & bit) continue;
-            }
-            const uint32_t old = atomicOr(&bits[v >> 5], bit);
-            if (old & bit) continue;
-            if (row) row[v] = nd;
-            my_sum += nd;
-            ++my_cnt;
-            q_put(level + 1, atomicAdd(cnt, 1u), v, 0, 0);
-          }
-        }
-      }
+      reached += n_in;
+      sum += (unsigned long long)level * n_in;
+      const uint32_t nslot = slot == 8 ? 0 : slot + 4;
+      if (threadIdx.x == 0) sts32(scnt + nslot, 0);
+      cta_expand<ER, THREADS, LPV, 4 / LPV>(
+          p, q, level, n_in, scnt + slot, row, [&](uint32_t v, uint32_t bit) {
+            return GB ? atomicOr(&bits[v >> 5], bit) : atoms_or(sbits + (v >> 5) * 4, bit);
+          });
       __syncthreads();
-      n_in = *cnt;
+      n_in = lds32(scnt + slot);
+      slot = nslot;
       ++level;
     }
     if (row) {
       // Unreached vertices: coalesced sweep of the row guided by the bitmap
       // (read from L2 in global mode: the bits were set by atomics).
-      for (uint32_t v = threadIdx.x; v < V; v += blockDim.x) {
-        const uint32_t w = GB ? __ldcg(bits + (v >> 5)) : bits[v >> 5];
-        if (!((w >> (v & 31)) & 1u)) row[v] = CTA_DIST_MAX;
-      }
+      if (reached < V)
+        for (uint32_t v = threadIdx.x; v < V; v += THREADS) {
+          const uint32_t w = GB ? __ldcg(bits + (v >> 5)) : bits[v >> 5];
+          if (!((w >> (v & 31)) & 1u)) row[v] = CTA_DIST_MAX;
+        }
     }
-    if (p.stats) {
-      if (my_cnt) {
-        atomicAdd(&s_sum, my_sum);
-        atomicAdd(&s_reached, my_cnt);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        p.stats[si].sum = s_sum;
-        p.stats[si].reached = s_reached + 1;
-        p.stats[si].ecc = ecc;
-      }
+    if (p.stats && threadIdx.x == 0) {
+      p.stats[si].sum = sum;
+      p.stats[si].reached = reached;
+      p.stats[si].ecc = level - 1;
     }
     __syncthreads();
   }
@@ -256,12 +336,9 @@ __global__ void __launch_bounds__(THREADS, MINB) cta_bfs_kernel(CtaParams p) {
 // per cluster) and the edge records work as in cta_bfs_kernel.
 template <int CL, bool ER>
 __global__ void __launch_bounds__(CTA_CLUSTER_THREADS, 1) cta_cluster_kernel(CtaParams p) {
-  constexpr int CTA_ER_BATCH = CTA_CLUSTER_ER_BATCH;
   extern __shared__ __align__(16) uint32_t smem_dyn[];
   __shared__ uint32_t s_src_idx;  // written into every block by rank 0
   __shared__ uint32_t s_cnt[3];
-  __shared__ unsigned long long s_sum;
-  __shared__ uint32_t s_reached;
   cg::cluster_group cluster = cg::this_cluster();
   const uint32_t rank = cluster.block_rank();
   const uint32_t V = p.V;
@@ -270,51 +347,35 @@ __global__ void __launch_bounds__(CTA_CLUSTER_THREADS, 1) cta_cluster_kernel(Cta
   const uint32_t w0 = min(words, rank * wpb);
   const uint32_t w1 = min(words, w0 + wpb);
   uint32_t* bits = smem_dyn;  // this block's slice: words [w0, w1)
-  const uint32_t QH = p.qh;
-  uint32_t* sq = smem_dyn + (wpb + 1) / 2 * 2;
-  uint2* sq2 = reinterpret_cast<uint2*>(sq);
-  uint32_t* slab = p.gqueue + (size_t)(blockIdx.x / CL) * V;
-  auto slab_at = [&](uint32_t lv, uint32_t i) -> uint32_t* {
-    return (lv & 1) ? slab + (V - 1 - i) : slab + i;
-  };
-  auto q_get = [&](uint32_t lv, uint32_t i, uint32_t* eb, uint32_t* ee) {
-    if constexpr (ER) {
-      if (i < QH) {
-        const uint2 r = sq2[(lv & 1) * QH + i];
-        *eb = r.x;
-        *ee = r.y;
-        return;
+  const uint32_t sbits = smem_addr(smem_dyn), scnt = smem_addr(s_cnt);
+  const CtaQueue<ER> q{sbits + (wpb + 1) / 2 * 8, p.gqueue + (size_t)(blockIdx.x / CL) * V,
+                       p.qh, V, p.off};
+  // Sets v's bit and returns the bitmap word as it was: in rank 0's own slice
+  // or in another block's, reached through distributed shared memory.
+  auto mark = [&](uint32_t v, uint32_t bit) -> uint32_t {
+    const uint32_t w = v >> 5;
+    uint32_t o = 0, base = 0;
+#pragma unroll
+    for (int r = 1; r < CL; ++r)
+      if (w >= r * wpb) {
+        o = r;
+        base = r * wpb;
       }
-    }
-    const uint32_t u = i < QH ? sq[(lv & 1) * QH + i] : *slab_at(lv, i);
-    *eb = __ldg(p.off + u);
-    *ee = __ldg(p.off + u + 1);
-  };
-  auto q_put = [&](uint32_t lv, uint32_t i, uint32_t v, uint32_t eb, uint32_t ee) {
-    if (i < QH) {
-      if constexpr (ER)
-        sq2[(lv & 1) * QH + i] = make_uint2(eb, ee);
-      else
-        sq[(lv & 1) * QH + i] = v;
-    } else {
-      *slab_at(lv, i) = v;
-    }
-  };
-  // Word w of the whole bitmap: in this block's slice (rank 0's own) or in
-  // the owning block's, reached through distributed shared memory.
-  auto word_ptr = [&](uint32_t w, bool* local) -> uint32_t* {
-    const uint32_t o = w / wpb;
-    uint32_t* at = bits + (w - o * wpb);
-    *local = o == rank;
-    return *local ? at : cluster.map_shared_rank(at, o);
+    uint32_t at, old;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(at)
+                 : "r"(sbits + (w - base) * 4), "r"(o));
+    asm volatile("atom.shared::cluster.or.b32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "r"(at), "r"(bit)
+                 : "memory");
+    return old;
   };
 
   for (;;) {
     if (rank == 0 && threadIdx.x == 0) {
       const uint32_t si = atomicAdd(p.work, 1u);
       for (int r = 0; r < CL; ++r) *cluster.map_shared_rank(&s_src_idx, r) = si;
-      s_sum = 0;
-      s_reached = 0;
       s_cnt[0] = s_cnt[1] = s_cnt[2] = 0;
     }
     for (uint32_t i = threadIdx.x; i < w1 - w0; i += blockDim.x) bits[i] = 0;
@@ -323,60 +384,31 @@ __global__ void __launch_bounds__(CTA_CLUSTER_THREADS, 1) cta_cluster_kernel(Cta
     if (si >= p.num_sources) break;  // the same value in every block
     const uint32_t src = p.sources[si];
     uint32_t* row = p.dist ? p.dist + (size_t)si * V : nullptr;
-    uint32_t ecc = 0;
     if (rank == 0) {
       if (threadIdx.x == 0) {
-        bool loc;
-        atomicOr(word_ptr(src >> 5, &loc), 1u << (src & 31));
+        mark(src, 1u << (src & 31));
         if (row) row[src] = 0;
-        q_put(0, 0, src, __ldg(p.off + src), __ldg(p.off + src + 1));
+        q.put_source(src);
       }
-      uint32_t n_in = 1;
-      uint32_t level = 0;
-      unsigned long long my_sum = 0;
-      uint32_t my_cnt = 0;
+      uint32_t n_in = 1, level = 0, reached = 0, slot = 0;  // slot: 4 * (level % 3)
+      unsigned long long sum = 0;
       __syncthreads();
       while (n_in) {
-        ecc = level;
-        const uint32_t nd = level + 1;
-        uint32_t* cnt = &s_cnt[level % 3];
-        if (threadIdx.x == 0) s_cnt[(level + 1) % 3] = 0;
-        for (uint32_t i = threadIdx.x; i < n_in; i += blockDim.x) {
-          uint32_t eb, ee;
-          q_get(level, i, &eb, &ee);
-          for (uint32_t e = eb; e < ee; e += (ER ? CTA_ER_BATCH : 1)) {
-            uint4 r[ER ? CTA_ER_BATCH : 1];
-            if constexpr (ER) {
-#pragma unroll
-              for (int k = 0; k < CTA_ER_BATCH; ++k)
-                if (e + k < ee) r[k] = __ldg(p.erec + e + k);
-            } else {
-              r[0] = make_uint4(__ldg(p.idx + e), 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int k = 0; k < (ER ? CTA_ER_BATCH : 1); ++k) {
-              if (e + k >= ee) break;
-              const uint32_t v = r[k].x;
-              const uint32_t bit = 1u << (v & 31);
-              bool loc;
-              uint32_t* wp = word_ptr(v >> 5, &loc);
-              if (loc && (*wp & bit)) continue;  // a remote pre-check costs the atomic's hop
-              const uint32_t old = atomicOr(wp, bit);
-              if (old & bit) continue;
-              if (row) row[v] = nd;
-              my_sum += nd;
-              ++my_cnt;
-              q_put(level + 1, atomicAdd(cnt, 1u), v, r[k].y, r[k].z);
-            }
-          }
-        }
+        reached += n_in;
+        sum += (unsigned long long)level * n_in;
+        const uint32_t nslot = slot == 8 ? 0 : slot + 4;
+        if (threadIdx.x == 0) sts32(scnt + nslot, 0);
+        cta_expand<ER, CTA_CLUSTER_THREADS, CTA_CLUSTER_LPV, 4 / CTA_CLUSTER_LPV>(
+            p, q, level, n_in, scnt + slot, row, mark);
         __syncthreads();
-        n_in = *cnt;
+        n_in = lds32(scnt + slot);
+        slot = nslot;
         ++level;
       }
-      if (p.stats && my_cnt) {
-        atomicAdd(&s_sum, my_sum);
-        atomicAdd(&s_reached, my_cnt);
+      if (p.stats && threadIdx.x == 0) {
+        p.stats[si].sum = sum;
+        p.stats[si].reached = reached;
+        p.stats[si].ecc = level - 1;
       }
     }
     cluster.sync();  // (2)
@@ -386,28 +418,23 @@ __global__ void __launch_bounds__(CTA_CLUSTER_THREADS, 1) cta_cluster_kernel(Cta
       for (uint32_t v = vb + threadIdx.x; v < ve; v += blockDim.x)
         if (!((bits[(v >> 5) - w0] >> (v & 31)) & 1u)) row[v] = CTA_DIST_MAX;
     }
-    if (rank == 0 && p.stats && threadIdx.x == 0) {
-      p.stats[si].sum = s_sum;
-      p.stats[si].reached = s_reached + 1;
-      p.stats[si].ecc = ecc;
-    }
     __syncthreads();  // the slice is read above and zeroed at the top
   }
 }
 
-// Edge records of a road-like graph: for every edge e = (u, v), {v, off[v],
-// off[v+1], 0}. One thread per vertex u.
+// Edge records of a road-like graph: for every edge e = (u, v), {v, off[v] <<
+// 4 | out-degree of v}. One thread per vertex u.
 __global__ void edge_records_kernel(uint32_t V, const uint32_t* __restrict__ off,
-                                    const uint32_t* __restrict__ idx, uint4* __restrict__ erec) {
+                                    const uint32_t* __restrict__ idx, uint2* __restrict__ erec) {
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < V; u += gridDim.x * blockDim.x) {
     for (uint32_t e = off[u]; e < off[u + 1]; ++e) {
       const uint32_t v = idx[e];
-      erec[e] = make_uint4(v, off[v], off[v + 1], 0u);
+      erec[e] = make_uint2(v, off[v] << 4 | (off[v + 1] - off[v]));
     }
   }
 }
 
-void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, uint4* erec,
+void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, uint2* erec,
                          cudaStream_t s) {
   edge_records_kernel<<<1024, 256, 0, s>>>(V, off, idx, erec);
 }
@@ -420,21 +447,20 @@ size_t cta_max_vertices(int device) {
   return ((size_t)optin - reserve) * 8;
 }
 
-template <bool GB, bool ER, int THREADS, int MINB>
-static int cta_occupancy(int block, size_t smem) {
-  auto fn = cta_bfs_kernel<GB, ER, THREADS, MINB>;
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, smem);
-  return occ;
+template <bool GB, bool ER>
+static void* cta_fn(int form) {
+  if (form == CTA_TPUT) return (void*)cta_bfs_kernel<GB, ER, CTA_TPUT>;
+  if constexpr (!GB) {
+    if (form == CTA_WIDE) return (void*)cta_bfs_kernel<GB, ER, CTA_WIDE>;
+    if (form == CTA_SMALL) return (void*)cta_bfs_kernel<GB, ER, CTA_SMALL>;
+  }
+  return (void*)cta_bfs_kernel<GB, ER, CTA_MID>;
 }
 
-template <bool GB, bool ER>
-static int cta_occupancy(int minb, int block, size_t smem) {
-  constexpr int LT = GB ? CTA_GB_THREADS : CTA_THREADS;
-  return minb >= CTA_MINB_THROUGHPUT
-             ? cta_occupancy<GB, ER, CTA_TPUT_THREADS, CTA_MINB_THROUGHPUT>(block, smem)
-             : cta_occupancy<GB, ER, LT, CTA_MINB_LATENCY>(block, smem);
+static void* cta_kernel(const CtaShape& sh) {
+  if (sh.global_bits)
+    return sh.edge_records ? cta_fn<true, true>(sh.form) : cta_fn<true, false>(sh.form);
+  return sh.edge_records ? cta_fn<false, true>(sh.form) : cta_fn<false, false>(sh.form);
 }
 
 template <int CL, bool ER>
@@ -489,7 +515,7 @@ static bool cta_cluster_shape(uint32_t V, int sms, int optin, bool edge_records,
   const int mode = env ? atoi(env) : -1;
   if (mode == 0) return false;
   const size_t words = ((size_t)V + 31) / 32;
-  const size_t entry = edge_records ? 2 * sizeof(uint32_t) : sizeof(uint32_t);
+  const size_t entry = sizeof(uint32_t);  // a vertex id or a packed edge range
   const size_t slack = 2048;
   for (int cl : {2, 4, 8}) {
     const size_t wpb = (words + cl - 1) / cl;
@@ -500,7 +526,6 @@ static bool cta_cluster_shape(uint32_t V, int sms, int optin, bool edge_records,
     sh.block = CTA_CLUSTER_THREADS;
     sh.edge_records = edge_records;
     sh.cluster = cl;
-    sh.minb = 1;
     sh.qh = (uint32_t)std::min<size_t>(CTA_SMEM_QUEUE, room / (2 * entry) / 32 * 32);
     sh.smem = slice + 2 * (size_t)sh.qh * entry;
     const int n = cluster_capacity(cl, edge_records, sh.smem, sh.block);
@@ -526,7 +551,7 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
   const size_t words = ((size_t)V + 31) / 32;
-  const size_t entry = edge_records ? 2 * sizeof(uint32_t) : sizeof(uint32_t);
+  const size_t entry = sizeof(uint32_t);  // a vertex id or a packed edge range
   const bool shared_bits = (size_t)V <= cta_max_vertices(device);
   if (!shared_bits && !allow_global) return false;
   if (!shared_bits && cta_cluster_shape(V, sms, optin, edge_records, num_sources, out))
@@ -534,29 +559,35 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   CtaShape sh{};
   sh.edge_records = edge_records;
   sh.global_bits = !shared_bits;
-  sh.minb = (shared_bits && num_sources > (size_t)sms * CTA_MINB_LATENCY) ? CTA_MINB_THROUGHPUT
-                                                                          : CTA_MINB_LATENCY;
-  sh.block = sh.minb >= CTA_MINB_THROUGHPUT ? CTA_TPUT_THREADS
-             : shared_bits                    ? CTA_THREADS
-                                              : CTA_GB_THREADS;
+  const size_t bitmap = shared_bits ? (words + 1) / 2 * 2 * sizeof(uint32_t) : 0;
+  const size_t slack = 2048;  // static shared variables + the driver's per-block reserve
+  const size_t fit = std::max<size_t>(1, (size_t)per_sm / (bitmap + slack));
+  const size_t per = std::min(fit, (num_sources + sms - 1) / std::max(sms, 1));
+  if (per > CTA_MID_BLOCKS) {
+    sh.form = CTA_TPUT;
+    sh.block = CtaForm<CTA_TPUT>::THREADS;
+    sh.minb = CtaForm<CTA_TPUT>::MINB;
+  } else if (per > 1 || !shared_bits) {
+    sh.form = CTA_MID;
+    sh.block = CtaForm<CTA_MID>::THREADS;
+    sh.minb = CtaForm<CTA_MID>::MINB;
+  } else {
+    sh.form = V >= CTA_WIDE_VERTICES ? CTA_WIDE : CTA_SMALL;
+    sh.block = V >= CTA_WIDE_VERTICES ? CtaForm<CTA_WIDE>::THREADS : CtaForm<CTA_SMALL>::THREADS;
+    sh.minb = 1;
+  }
   // The queue halves get the shared memory left once the bitmaps of minb
   // resident blocks have theirs, so the queue never costs a resident block.
   // A frontier beyond the halves continues in the global slab.
-  const size_t bitmap = shared_bits ? (words + 1) / 2 * 2 * sizeof(uint32_t) : 0;  // 8-byte end
-  const size_t slack = 2048;  // static shared variables + the driver's per-block reserve
-  const size_t fit = std::max<size_t>(1, (size_t)per_sm / (bitmap + slack));
   const size_t blocks = std::min<size_t>((size_t)sh.minb, fit);
   const size_t budget = std::min<size_t>((size_t)per_sm / blocks, (size_t)optin) - slack;
   const size_t room = budget > bitmap ? budget - bitmap : 0;
   sh.qh = (uint32_t)std::min<size_t>(CTA_SMEM_QUEUE, room / (2 * entry) / 32 * 32);
   sh.smem = bitmap + 2 * (size_t)sh.qh * entry;
-  int occ;
-  if (shared_bits)
-    occ = edge_records ? cta_occupancy<false, true>(sh.minb, sh.block, sh.smem)
-                       : cta_occupancy<false, false>(sh.minb, sh.block, sh.smem);
-  else
-    occ = edge_records ? cta_occupancy<true, true>(sh.minb, sh.block, sh.smem)
-                       : cta_occupancy<true, false>(sh.minb, sh.block, sh.smem);
+  void* fn = cta_kernel(sh);
+  int occ = 0;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, sh.block, sh.smem);
   if (occ < 1) return false;
   sh.grid = sms * occ;
   if (!shared_bits) {
@@ -566,16 +597,6 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   }
   *out = sh;
   return true;
-}
-
-template <bool GB, bool ER>
-static void launch_cta_t(const CtaParams& p, const CtaShape& sh, int grid, cudaStream_t s) {
-  constexpr int LT = GB ? CTA_GB_THREADS : CTA_THREADS;
-  if (sh.minb >= CTA_MINB_THROUGHPUT)
-    cta_bfs_kernel<GB, ER, CTA_TPUT_THREADS, CTA_MINB_THROUGHPUT>
-        <<<grid, sh.block, sh.smem, s>>>(p);
-  else
-    cta_bfs_kernel<GB, ER, LT, CTA_MINB_LATENCY><<<grid, sh.block, sh.smem, s>>>(p);
 }
 
 void launch_cta(const CtaParams& params, const CtaShape& sh, int grid, cudaStream_t s) {
@@ -600,17 +621,8 @@ void launch_cta(const CtaParams& params, const CtaShape& sh, int grid, cudaStrea
     cudaLaunchKernelExC(&cfg, cluster_kernel(sh.cluster, sh.edge_records), args);
     return;
   }
-  if (sh.global_bits) {
-    if (sh.edge_records)
-      launch_cta_t<true, true>(p, sh, grid, s);
-    else
-      launch_cta_t<true, false>(p, sh, grid, s);
-  } else {
-    if (sh.edge_records)
-      launch_cta_t<false, true>(p, sh, grid, s);
-    else
-      launch_cta_t<false, false>(p, sh, grid, s);
-  }
+  void* args[] = {&p};
+  cudaLaunchKernel(cta_kernel(sh), dim3(grid), dim3(sh.block), args, sh.smem, s);
 }
 
 // ---------------------------------------------------------------------------

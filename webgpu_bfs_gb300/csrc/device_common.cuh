@@ -209,14 +209,15 @@ struct CtaParams {
   SourceStats* stats;    // non-null: per-source reductions instead of rows
   uint32_t* gbits;       // global-bitmap mode: per resident block ceil(V/32) u32
   uint32_t qh;           // frontier entries per shared-memory queue half (set at launch)
-  const uint4* erec;     // per edge {target, target's edge begin, end, 0}, or null
+  const uint2* erec;     // per edge {target, target's edge begin << 4 | count}, or null
 };
 struct CtaShape {
   int grid = 0;           // resident blocks
   int block = 0;          // threads per block
   size_t smem = 0;        // dynamic shared memory: bitmap (shared mode) + queue halves
   uint32_t qh = 0;        // frontier entries per shared-memory queue half
-  int minb = 3;           // register budget: resident blocks per SM it is built for
+  int form = 0;           // block form (threads, lanes per vertex) of cta_kernel.cu
+  int minb = 1;           // resident blocks per SM the queue halves leave room for
   bool global_bits = false;
   bool edge_records = false;
   int cluster = 0;        // > 1: blocks per cluster sharing one source's bitmap
@@ -231,7 +232,7 @@ size_t cta_max_vertices(int device);
 bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_records,
                       size_t num_sources, CtaShape* out);
 void launch_cta(const CtaParams& p, const CtaShape& sh, int grid, cudaStream_t s);
-void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, uint4* erec,
+void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, uint2* erec,
                          cudaStream_t s);
 
 void launch_traversed_edges(uint32_t V, const uint32_t* off, const uint32_t* dist,

@@ -67,8 +67,8 @@ struct msbfs_graph {
   // Bottom-up work order: vertices with 0 < in-degree <= split, ascending ids.
   uint32_t n_order = 0;
   uint4* order = nullptr;  // {vertex, in-edge begin, in-edge end, 0}
-  // Road-like graphs: per edge {target, target's edge begin, end, 0}.
-  uint4* erec = nullptr;
+  // Road-like graphs: per edge {target, target's edge begin << 4 | count}.
+  uint2* erec = nullptr;
   std::vector<uint32_t> h_coff;  // host CSC offsets (V + 1): rebuilds the tables above
 };
 
@@ -953,10 +953,11 @@ int upload_graph(msbfs_engine* eng, size_t V, size_t E, const uint32_t* off, con
   int rc = build_bottom_up_tables(eng, g.get(), eng->split);
   if (rc) return rc;
   // Road-like graphs (the ones the router sends to the CTA path) get edge
-  // records, 16 bytes per edge, so a CTA-path level costs one dependent L2
-  // round trip instead of three.
-  if (is_road_like(g.get()) && E > 0) {
-    CK(cudaMalloc((void**)&g->erec, E * sizeof(uint4)));
+  // records, 8 bytes per edge, so a CTA-path level costs one dependent L2
+  // round trip instead of three. The packed edge range holds 28 bits of edge
+  // index and at most 15 out-edges (road-like: at most 8).
+  if (is_road_like(g.get()) && E > 0 && E < (size_t(1) << 28)) {
+    CK(cudaMalloc((void**)&g->erec, E * sizeof(uint2)));
     launch_edge_records((uint32_t)V, g->off, g->idx, g->erec, eng->stream);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(eng->stream));
