@@ -13,7 +13,8 @@
 //   Q[3][qcap]       u64 queue entries (seg << 32 | v): frontier vertices, one
 //                    entry per SEG out-edges so hub expansion is split (Q[0]
 //                    holds V + E/SEG0 entries: the sources' queue uses SEG0)
-//   stamp[V]         level at which v was last enqueued by a top-down step
+//   stamp[V]         when v was last enqueued by a top-down step: the pass's
+//                    epoch plus the level, so passes need no reset between them
 #pragma once
 
 #include <cstdint>
@@ -23,7 +24,7 @@ namespace msbfs {
 
 enum : uint32_t { DIR_PUSH = 0, DIR_PULL = 1 };
 enum : uint32_t { MODE_PUSH = 1, MODE_PULL = 2, MODE_HYBRID = 3 };
-enum : uint32_t { STATUS_LEVEL_CAP = 1u, STATUS_BAD_SOURCE = 2u, STATUS_CHECK = 4u };
+enum : uint32_t { STATUS_LEVEL_CAP = 1u, STATUS_BAD_SOURCE = 2u, STATUS_CHECK = 4u, STATUS_STUCK = 8u };
 
 // Per-level record written by the level controller (counters feed the
 // algorithmic-bytes model of the roofline; t is %globaltimer ns).
@@ -52,9 +53,8 @@ struct LevelCtl {
   uint32_t qcount[4];  // queue entries per slot (slot 3 unused)
   uint32_t qverts[4];  // vertices per slot
   unsigned long long qedges[4];  // sum of out-degrees per slot
-  unsigned long long explored;   // out-edges of all expanded frontiers
   unsigned long long pairs;      // discovered (s, v) pairs, sources included
-  uint32_t done_blocks;          // last-block-done counter of the level kernel
+  uint32_t done_blocks;          // last-block-done counter of a host-driven level
   uint32_t push_levels;
   uint32_t pull_levels;
   uint32_t check_site;           // bounds-checked build: first failed check site
@@ -64,6 +64,7 @@ struct LevelCtl {
   unsigned long long c_pairs;
   unsigned long long c_rows;
   unsigned long long t_start;    // min %globaltimer over the level's blocks
+  uint32_t build_queue;          // the next top-down level's queue is not built yet
   uint32_t use_bits;             // bottom-up step checks frontier bitmaps first
   uint32_t narrow;               // the pass's rows went to PassDesc::dist8 as bytes
   // Vertex-tile cursors of the running bottom-up step: the work list is cut
@@ -78,17 +79,13 @@ struct LevelCtl {
   uint32_t lanes[2][64];
 };
 
-// One slice of a high in-degree vertex's in-edge list, scanned by one warp
-// during bottom-up steps; the last slice to finish records the result.
-struct HeavyChunk {
-  uint32_t v;      // vertex
-  uint32_t j;      // slice index
-  uint32_t nch;    // slices of this vertex
-  uint32_t h;      // index of the vertex among heavy vertices
-};
+// Slices of the in-edge lists of vertices of in-degree >= heavy, scanned by
+// one warp each during bottom-up steps: {vertex, first in-edge, end, h}. h is
+// the vertex's index among those of several slices (its last slice to finish
+// records the result), SLICE_H for a vertex of one slice; SLICE_FIRST marks a
+// vertex's first slice.
+constexpr uint32_t SLICE_FIRST = 0x80000000u, SLICE_H = 0x7fffffffu;
 
-// Per-pass descriptor, read from device memory so one captured CUDA graph can
-// serve every pass and every call.
 // Per-source reductions of a traversal (served form): eccentricity (largest
 // finite distance), reached vertices (the source included) and the sum of
 // finite distances. Layout shared with msbfs_source_stats in msbfs.h.
@@ -98,6 +95,7 @@ struct SourceStats {
   uint32_t reached;
 };
 
+// Per-pass part of the kernel parameters.
 struct PassDesc {
   const uint32_t* sources;  // this pass's sources (device)
   uint32_t* dist;           // first row of this pass in the distance matrix
@@ -112,6 +110,12 @@ struct PassDesc {
   uint32_t reach_col;       // word column of this pass in that output
   uint32_t row_split;       // split materialisation: rows below go u32 to dist,
                             // rows from it on as bytes to dist8 (multiple of 32)
+};
+
+// Grid barrier of the traversal kernel (never reset between passes).
+struct GridSync {
+  uint32_t arrive;            // blocks that have arrived
+  alignas(128) uint32_t gen;  // barriers passed
 };
 
 struct LevelParams {
@@ -131,7 +135,9 @@ struct LevelParams {
   uint32_t* fbits[3];  // frontier membership bitmaps (V bits), rotated like F
   LevelCtl* ctl;
   LevelRec* log;      // LOG_CAP records
-  const PassDesc* desc;
+  PassDesc d;
+  GridSync* sync;
+  uint32_t epoch;     // stamp of level 0 of this pass
   uint32_t NP;        // planes allocated
   uint32_t qcap;      // entries per queue slot (slots 1, 2)
   uint32_t qcap0;     // entries of slot 0 (the sources' queue uses shorter entries)
@@ -140,13 +146,12 @@ struct LevelParams {
   uint32_t beta;      // pull -> push when n_f * beta < V
   uint32_t seg;       // out-edges per queue entry
   uint32_t seg0;      // out-edges per entry of the sources' queue (level 0)
-  uint32_t heavy;     // in-degree from which a whole warp scans one vertex
   uint32_t max_levels;
-  uint32_t split;     // in-degree above which in-edges are sliced across warps
-  uint32_t n_hchunks;
-  const HeavyChunk* hchunks;
-  uint32_t* hcand;    // [n_heavy][W] candidate words of sliced vertices
-  uint32_t* hcount;   // [n_heavy] slices finished this level
+  uint32_t n_slices;
+  const uint4* slices;
+  const uint32_t* hslices;  // slices of each vertex of several
+  uint32_t* hcand;    // [vertices of several slices][W] candidate words
+  uint32_t* hcount;   // [the same] slices finished this level
   // Bit ci: the vertex of slice ci may still need lanes. Set at pass start,
   // cleared for good once the slice finds none needed (a vertex's needed
   // lanes only shrink: visited lanes grow, live lanes die).
@@ -154,17 +159,24 @@ struct LevelParams {
   uint32_t hlive_words;
   uint32_t bits_div;  // bitmap check when the frontier holds < V / bits_div vertices
   uint32_t n_order;
-  const uint4* order;  // {v, in-edge begin, end, 0} for 0 < in-degree <= split (work order)
+  const uint4* order;  // {v, in-edge begin, end, 0} for 0 < in-degree < heavy (work order)
 };
 
-// Launch helpers implemented in level_kernels.cu / cta_kernel.cu.
+constexpr int MAT_BLOCK = 256;
+constexpr int MAT_TILE_WORDS = MAT_BLOCK * 4;
+constexpr int MAT_NPMAX = 8;
+
+// Launch helpers implemented in level_launch.cu / cta_kernel.cu.
 struct LevelKernelInfo {
-  void* init;         // kernel symbols for graph nodes
+  void* traverse;     // a pass's whole traversal, cooperative
+  int traverse_grid;  // its resident grid
+  void* init;         // the same level by level, driven by the host
   void* level[2][2];  // [direction: DIR_PUSH, DIR_PULL][with profiling counters]
   int level_grids[2]; // resident grid per direction
   void* materialize;
   void* reduce;       // per-source reductions in place of materialize
   void* cleanup;
+  void* queue;        // a top-down level's queue after a bottom-up one (host-driven loop)
   int level_block;
   int mat_block;
   int mat_grid;
@@ -179,7 +191,10 @@ size_t materialize_smem_bytes(uint32_t W, uint32_t NP);
 // (vertex tile, word group) items of a materialisation over V vertices at
 // W words per vertex: an upper bound on what a pass of fewer sources uses.
 size_t materialize_items(uint32_t V, uint32_t W);
-void launch_init(const LevelParams& p, cudaStream_t s);
+// A whole traversal (source init, levels, frontier cleanup) in one cooperative
+// launch of k.traverse_grid blocks.
+cudaError_t launch_traverse(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
+void launch_init(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
 // Launches the level kernel of direction `dir` (DIR_PUSH / DIR_PULL), or
 // both (pull, then push) when dir is DIR_BOTH; `count` picks the form that
 // keeps the profiling counters.
@@ -195,7 +210,8 @@ void launch_level(const LevelParams& p, const LevelKernelInfo& k, uint32_t dir, 
 enum : uint32_t { MAT_BYTES = 0, MAT_WIDE = 1, MAT_ALL = 2 };
 void launch_materialize(const LevelParams& p, const LevelKernelInfo& k, bool reduce,
                         cudaStream_t s, uint32_t phase = MAT_ALL);
-void launch_cleanup(const LevelParams& p, cudaStream_t s);
+void launch_queue(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
+void launch_cleanup(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
 
 struct CtaParams {
   uint32_t V;

@@ -5,12 +5,12 @@
 // a mutex) with a CUDA runtime underneath instead of wgpu:
 //  * graphs are uploaded once and stay resident (CSR + CSC, aliased when the
 //    graph is symmetric, like PushPullGraphBuffers in buffer.rs:108-221);
-//  * a level-synchronous pass is ONE cudaGraphLaunch: memset control block,
-//    source init, a WHILE conditional node around the level kernel (its last
-//    block sets the condition, so no host round trip per level or per batch
-//    of levels, replacing multi_word_bp.rs:730-814's speculative 4..64-hop
-//    submits and indirect_sparse_push.rs:1462-1578's macro batches), the
-//    distance materialisation and the frontier cleanup;
+//  * a level-synchronous pass is one cooperative launch that runs the source
+//    init and every level (the last block of a level decides the next one, so
+//    no host round trip per level or per batch of levels, replacing
+//    multi_word_bp.rs:730-814's speculative 4..64-hop submits and
+//    indirect_sparse_push.rs:1462-1578's macro batches), and the distance
+//    materialisation;
 //  * the CTA-per-source path is one persistent launch per call.
 #include <cuda_runtime.h>
 
@@ -59,12 +59,14 @@ struct msbfs_graph {
   uint32_t* idx = nullptr;
   uint32_t* coff = nullptr;  // CSC (== CSR when symmetric)
   uint32_t* cidx = nullptr;
-  // In-edge lists longer than `split` are cut into slices for bottom-up steps.
-  uint32_t split = 0;
-  uint32_t n_heavy = 0;
-  uint32_t n_hchunks = 0;
-  HeavyChunk* hchunks = nullptr;
-  // Bottom-up work order: vertices with 0 < in-degree <= split, ascending ids.
+  // Bottom-up steps: in-edge lists of `heavy` and more are scanned by whole
+  // warps, in slices of at most `split`.
+  uint32_t split = 0, heavy = 0;  // as asked for (the tables may use shorter slices)
+  uint32_t n_heavy = 0;   // vertices of several slices
+  uint32_t n_slices = 0;
+  uint4* slices = nullptr;
+  uint32_t* hslices = nullptr;
+  // Bottom-up work order: vertices with 0 < in-degree < heavy, ascending ids.
   uint32_t n_order = 0;
   uint4* order = nullptr;  // {vertex, in-edge begin, in-edge end, 0}
   // Road-like graphs: per edge {target, target's edge begin << 4 | count}.
@@ -82,22 +84,14 @@ struct Workspace {
   LevelParams p{};
   LevelKernelInfo k{};
   LevelCtl* d_ctl = nullptr;
-  PassDesc* d_desc = nullptr;
   LevelRec* d_log = nullptr;
   std::vector<void*> allocs;
   // Set when a pass stopped part-way (an error after work was queued): its
   // buffers may hold that pass's bits, so the next call builds a fresh
   // workspace instead of reusing this one.
   bool dirty = false;
-  // One instantiated pass per ending: [0] materialise, [1] reduce, [2] the
-  // byte rows of a split materialisation only (built on first use).
-  cudaGraph_t graph[3] = {nullptr, nullptr, nullptr};
-  cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
+  uint32_t next_epoch = 1;  // stamps of later passes start here (0: never enqueued)
   ~Workspace() {
-    for (int i = 0; i < 3; ++i) {
-      if (exec[i]) cudaGraphExecDestroy(exec[i]);
-      if (graph[i]) cudaGraphDestroy(graph[i]);
-    }
     for (void* a : allocs) cudaFree(a);
   }
 };
@@ -142,7 +136,8 @@ struct msbfs_engine {
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr, ev_pass = nullptr, ev_copies = nullptr;
   std::mutex mu;
   std::string last_error;
-  uint32_t max_words = 16;
+  uint32_t max_words = 0;   // words per vertex of a pass at most (0: widest_pass)
+  size_t total_mem = 0;     // device memory
   uint32_t alpha = 14;
   uint32_t beta = 24;
   uint32_t seg = MSBFS_PUSH_SEG;  // out-edges per top-down queue entry
@@ -259,113 +254,8 @@ int dev_alloc(msbfs_engine* eng, Workspace* w, void** ptr, size_t bytes) {
   return MSBFS_OK;
 }
 
-// The pass ends in materialize_kernel (variant 0), reduce_kernel (1,
-// per-source reductions) or, for a split materialisation, the byte-row
-// phase alone (2: the host then launches the u32 phase and the cleanup).
-enum : int { PASS_ROWS = 0, PASS_STATS = 1, PASS_BYTES = 2 };
-int build_graph_exec(msbfs_engine* eng, Workspace* w, int variant) {
-  const bool reduce = variant == PASS_STATS;
-  cudaGraph_t g = nullptr;
-  CK(cudaGraphCreate(&g, 0));
-  w->graph[variant] = g;
-  cudaGraphNode_t n_mctl, n_mst, n_init, n_cond, n_lvl, n_mat, n_clean;
-  cudaMemsetParams m1{};
-  m1.dst = w->d_ctl;
-  m1.value = 0;
-  m1.elementSize = 1;
-  m1.width = sizeof(LevelCtl);
-  m1.height = 1;
-  m1.pitch = sizeof(LevelCtl);
-  CK(cudaGraphAddMemsetNode(&n_mctl, g, nullptr, 0, &m1));
-  cudaMemsetParams m2{};
-  m2.dst = w->p.stamp;
-  m2.value = 0xFFFFFFFFu;
-  m2.elementSize = 4;
-  m2.width = w->p.V;
-  m2.height = 1;
-  m2.pitch = (size_t)w->p.V * 4;
-  CK(cudaGraphAddMemsetNode(&n_mst, g, nullptr, 0, &m2));
-  cudaGraphNode_t n_mfb;
-  cudaMemsetParams m3{};
-  m3.dst = w->p.fbits[0];
-  m3.value = 0;
-  m3.elementSize = 4;
-  m3.width = 3 * (((size_t)w->p.V + 31) / 32);
-  m3.height = 1;
-  m3.pitch = m3.width * 4;
-  CK(cudaGraphAddMemsetNode(&n_mfb, g, nullptr, 0, &m3));
-  cudaGraphNode_t n_mhl;
-  cudaMemsetParams m4{};
-  m4.dst = w->p.hlive;
-  m4.value = 0xFFFFFFFFu;
-  m4.elementSize = 4;
-  m4.width = std::max(w->p.hlive_words, 1u);
-  m4.height = 1;
-  m4.pitch = m4.width * 4;
-  CK(cudaGraphAddMemsetNode(&n_mhl, g, nullptr, 0, &m4));
-
-  void* args_p[] = {&w->p};
-  cudaKernelNodeParams ki{};
-  ki.func = w->k.init;
-  ki.gridDim = dim3(1);
-  ki.blockDim = dim3(256);
-  ki.sharedMemBytes = 0;
-  ki.kernelParams = args_p;
-  cudaGraphNode_t deps_init[4] = {n_mctl, n_mst, n_mfb, n_mhl};
-  CK(cudaGraphAddKernelNode(&n_init, g, deps_init, 4, &ki));
-
-  cudaGraphConditionalHandle h;
-  CK(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-  cudaGraphNodeParams cp{};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = h;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  CK(cudaGraphAddNode(&n_cond, g, &n_init, nullptr, 1, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-
-  // Loop body: the bottom-up kernel, then the top-down kernel; the one whose
-  // direction the control block does not name returns at once (a mode
-  // that never changes direction gets only its own).
-  void* args_l[] = {&w->p, &h};
-  n_lvl = nullptr;
-  for (uint32_t dir : {(uint32_t)DIR_PULL, (uint32_t)DIR_PUSH}) {
-    if ((dir == DIR_PULL && w->mode == MODE_PUSH) || (dir == DIR_PUSH && w->mode == MODE_PULL))
-      continue;
-    cudaKernelNodeParams kl{};
-    kl.func = w->k.level[dir][w->count];
-    kl.gridDim = dim3(w->k.level_grids[dir]);
-    kl.blockDim = dim3(w->k.level_block);
-    kl.sharedMemBytes = 0;
-    kl.kernelParams = args_l;
-    cudaGraphNode_t prev = n_lvl;
-    CK(cudaGraphAddKernelNode(&n_lvl, body, prev ? &prev : nullptr, prev ? 1 : 0, &kl));
-  }
-
-  uint32_t phase = variant == PASS_BYTES ? MAT_BYTES : MAT_ALL;
-  void* args_m[] = {&w->p, &phase};
-  cudaKernelNodeParams km{};
-  km.func = reduce ? w->k.reduce : w->k.materialize;
-  km.gridDim = dim3(reduce ? w->k.red_grid : w->k.mat_grid);
-  km.blockDim = dim3(reduce ? w->k.red_block : w->k.mat_block);
-  km.sharedMemBytes = reduce ? 0u : (unsigned)w->k.mat_smem;
-  km.kernelParams = reduce ? args_p : args_m;
-  CK(cudaGraphAddKernelNode(&n_mat, g, &n_cond, 1, &km));
-
-  if (variant != PASS_BYTES) {
-    cudaKernelNodeParams kc{};
-    kc.func = w->k.cleanup;
-    kc.gridDim = dim3(256);
-    kc.blockDim = dim3(256);
-    kc.sharedMemBytes = 0;
-    kc.kernelParams = args_p;
-    CK(cudaGraphAddKernelNode(&n_clean, g, &n_cond, 1, &kc));
-  }
-  (void)n_lvl;
-  (void)n_mat;
-  (void)n_clean;
-  CK(cudaGraphInstantiate(&w->exec[variant], g, 0));
-  return MSBFS_OK;
+uint32_t level_planes(const msbfs_graph* g) {
+  return std::min<uint32_t>(bit_length_u64(g->V > 1 ? g->V - 1 : 1), 8);
 }
 
 int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t mode,
@@ -387,8 +277,7 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   w->graph_id = g->id;
   w->W = W;
   w->mode = mode;
-  const uint32_t dist_bits = bit_length_u64(g->V > 1 ? g->V - 1 : 1);
-  const uint32_t NP = std::min<uint32_t>(dist_bits, 8);
+  const uint32_t NP = level_planes(g);
   if (!level_kernel_info(W, NP, eng->num_sms, &w->k))
     return set_err(eng, MSBFS_ERR_INVALID_ARGUMENT, "unsupported words per vertex");
   // Work is claimed dynamically, so a smaller grid is only slower, never wrong.
@@ -403,6 +292,11 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
     w->k.mat_grid = (int)std::max<size_t>(1, std::min(want, items));
   }
   w->k.red_grid = std::max(1, (int)((uint64_t)w->k.red_grid * eng->sm_share / 100));
+  // Blocks that a small graph cannot feed only make the grid barriers of its
+  // levels longer: a block per 1,024 lane loads (visited pieces and edges).
+  const uint64_t loads = (uint64_t)g->V * std::max(1u, W / 4) + g->E;
+  w->k.traverse_grid = (int)std::min<uint64_t>(w->k.traverse_grid, std::max<uint64_t>(32, loads / 1024));
+  w->k.traverse_grid = std::max(1, (int)((uint64_t)w->k.traverse_grid * eng->sm_share / 100));
   LevelParams& p = w->p;
   p.V = (uint32_t)g->V;
   p.W = W;
@@ -423,13 +317,12 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   p.beta = eng->beta;
   p.seg = eng->seg;
   p.seg0 = std::min<uint32_t>(MSBFS_PUSH_SEG0, eng->seg);
-  p.heavy = eng->heavy;
   p.bits_div = eng->bits_div;
   p.max_levels = (uint32_t)std::min<uint64_t>(g->V + 2, 0xFFFFFFF0ull);
   if (eng->level_cap) p.max_levels = std::min(p.max_levels, eng->level_cap);
-  p.split = g->split;
-  p.n_hchunks = g->n_hchunks;
-  p.hchunks = g->hchunks;
+  p.n_slices = g->n_slices;
+  p.slices = g->slices;
+  p.hslices = g->hslices;
   p.n_order = g->n_order;
   p.order = g->order;
   int rc;
@@ -456,9 +349,8 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(LevelCtl)))) return rc;
   w->d_ctl = (LevelCtl*)ptr;
   p.ctl = w->d_ctl;
-  if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(PassDesc)))) return rc;
-  w->d_desc = (PassDesc*)ptr;
-  p.desc = w->d_desc;
+  if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(GridSync)))) return rc;
+  p.sync = (GridSync*)ptr;
   if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(LevelRec) * LOG_CAP))) return rc;
   w->d_log = (LevelRec*)ptr;
   p.log = w->d_log;
@@ -466,25 +358,28 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   p.hcand = (uint32_t*)ptr;
   if ((rc = dev_alloc(eng, w.get(), &ptr, (size_t)g->n_heavy * 4))) return rc;
   p.hcount = (uint32_t*)ptr;
-  p.hlive_words = (g->n_hchunks + 31) / 32;
+  p.hlive_words = (g->n_slices + 31) / 32;
   if ((rc = dev_alloc(eng, w.get(), &ptr, (size_t)std::max(p.hlive_words, 1u) * 4))) return rc;
   p.hlive = (uint32_t*)ptr;
-  if (!eng->host_loop) {
-    rc = build_graph_exec(eng, w.get(), PASS_ROWS);
-    if (rc) {
-      // Conditional graph nodes unavailable: fall back to the host-driven loop.
-      eng->host_loop = true;
-      cudaGetLastError();
-    }
-  }
+  if (p.hlive_words)
+    CK(cudaMemsetAsync(p.hlive, 0xFF, p.hlive_words * sizeof(uint32_t), eng->stream));
   *out = w.get();
   eng->ws[key] = std::move(w);
   return MSBFS_OK;
 }
 
-// Host-driven fallback loop: launches level kernels in speculative batches of
-// 8 and reads the control block between batches (extra launches after the
-// last level return immediately).
+// Reserves the stamps of one pass: level L of the pass stamps epoch + L.
+int next_epoch(msbfs_engine* eng, Workspace* w) {
+  const uint64_t span = (uint64_t)w->p.max_levels + 2;
+  if (w->next_epoch + span > 0xFFFFFFFFull) {
+    CK(cudaMemsetAsync(w->p.stamp, 0, w->p.V * sizeof(uint32_t), eng->stream));
+    w->next_epoch = 1;
+  }
+  w->p.epoch = w->next_epoch;
+  w->next_epoch += (uint32_t)span;
+  return MSBFS_OK;
+}
+
 int ensure_events(msbfs_engine* eng, size_t n) {
   while (eng->lvl_events.size() < n) {
     cudaEvent_t e;
@@ -500,11 +395,7 @@ int ensure_events(msbfs_engine* eng, size_t n) {
 int run_pass_profiled(msbfs_engine* eng, Workspace* w, bool reduce, std::vector<float>* ms) {
   int rc;
   CK(cudaMemsetAsync(w->d_ctl, 0, sizeof(LevelCtl), eng->stream));
-  CK(cudaMemsetAsync(w->p.stamp, 0xFF, w->p.V * sizeof(uint32_t), eng->stream));
-  CK(cudaMemsetAsync(w->p.fbits[0], 0, 3 * ((w->p.V + 31) / 32) * sizeof(uint32_t), eng->stream));
-  if (w->p.hlive_words)
-    CK(cudaMemsetAsync(w->p.hlive, 0xFF, w->p.hlive_words * sizeof(uint32_t), eng->stream));
-  launch_init(w->p, eng->stream);
+  launch_init(w->p, w->k, eng->stream);
   LevelCtl probe{};
   CK(cudaMemcpyAsync(&probe, w->d_ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost, eng->stream));
   CK(cudaStreamSynchronize(eng->stream));
@@ -512,6 +403,7 @@ int run_pass_profiled(msbfs_engine* eng, Workspace* w, bool reduce, std::vector<
   for (uint32_t L = 0;; ++L) {
     if ((rc = ensure_events(eng, 2))) return rc;
     CK(cudaEventRecord(eng->lvl_events[0], eng->stream));
+    if (probe.build_queue) launch_queue(w->p, w->k, eng->stream);
     launch_level(w->p, w->k, probe.dir, w->count, eng->stream);
     CK(cudaEventRecord(eng->lvl_events[1], eng->stream));
     CK(cudaGetLastError());
@@ -529,7 +421,7 @@ int run_pass_profiled(msbfs_engine* eng, Workspace* w, bool reduce, std::vector<
   CK(cudaEventRecord(eng->lvl_events[0], eng->stream));
   launch_materialize(w->p, w->k, reduce, eng->stream);
   CK(cudaEventRecord(eng->lvl_events[1], eng->stream));
-  launch_cleanup(w->p, eng->stream);
+  launch_cleanup(w->p, w->k, eng->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(eng->stream));
   float t = 0.f;
@@ -538,13 +430,12 @@ int run_pass_profiled(msbfs_engine* eng, Workspace* w, bool reduce, std::vector<
   return MSBFS_OK;
 }
 
+// Host-driven loop: launches level kernels in speculative batches of 8 and
+// reads the control block between batches (extra launches after the last
+// level return immediately).
 int run_pass_host_loop(msbfs_engine* eng, Workspace* w, bool reduce) {
   CK(cudaMemsetAsync(w->d_ctl, 0, sizeof(LevelCtl), eng->stream));
-  CK(cudaMemsetAsync(w->p.stamp, 0xFF, w->p.V * sizeof(uint32_t), eng->stream));
-  CK(cudaMemsetAsync(w->p.fbits[0], 0, 3 * ((w->p.V + 31) / 32) * sizeof(uint32_t), eng->stream));
-  if (w->p.hlive_words)
-    CK(cudaMemsetAsync(w->p.hlive, 0xFF, w->p.hlive_words * sizeof(uint32_t), eng->stream));
-  launch_init(w->p, eng->stream);
+  launch_init(w->p, w->k, eng->stream);
   LevelCtl probe{};
   for (uint64_t launched = 0;;) {
     const uint32_t dirs = w->mode == MODE_PUSH ? DIR_PUSH : w->mode == MODE_PULL ? DIR_PULL
@@ -561,13 +452,27 @@ int run_pass_host_loop(msbfs_engine* eng, Workspace* w, bool reduce) {
     }
   }
   launch_materialize(w->p, w->k, reduce, eng->stream);
-  launch_cleanup(w->p, eng->stream);
+  launch_cleanup(w->p, w->k, eng->stream);
   CK(cudaGetLastError());
   return MSBFS_OK;
 }
 
-uint32_t choose_words(msbfs_engine* eng, size_t S) {
-  size_t lanes = std::min<size_t>(S, (size_t)eng->max_words * 32);
+// Words per vertex of the widest pass when the caller sets none. A pass costs
+// far less than twice one of half its width (the levels' latency and fixed
+// parts are shared, and a gathered row of 128 bytes costs little more than
+// one of 64). ms of a call at up to 16 / 32 / 64 words: Erdos-Renyi 100,000 x
+// 16, S=700 0.525 / 0.421 / -, S=2,048 1.125 / 0.893 / 0.705; R-MAT 20, S=513
+// 2.00 / 2.05 / -, S=2,048 5.99 / 4.92 / 4.38. Passes above 16 words keep
+// their traversal state within an eighth of the device memory.
+uint32_t widest_pass(const msbfs_engine* eng, const msbfs_graph* g) {
+  if (eng->max_words) return eng->max_words;
+  uint32_t W = 64;
+  while (W > 16 && (uint64_t)g->V * W * 4 * (5 + level_planes(g)) > eng->total_mem / 8) W >>= 1;
+  return W;
+}
+
+uint32_t choose_words(const msbfs_engine* eng, const msbfs_graph* g, size_t S) {
+  size_t lanes = std::min<size_t>(S, (size_t)widest_pass(eng, g) * 32);
   uint32_t need = (uint32_t)((lanes + 31) / 32);
   uint32_t W = 1;
   while (W < need) W <<= 1;
@@ -681,26 +586,16 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
   const uint32_t mode = path == MSBFS_PATH_PUSH   ? MODE_PUSH
                         : path == MSBFS_PATH_PULL ? MODE_PULL
                                                   : MODE_HYBRID;
-  const uint32_t W = choose_words(eng, S);
+  const uint32_t W = choose_words(eng, g, S);
   const size_t PW = (size_t)W * 32;
   const size_t passes = (S + PW - 1) / PW;
   Workspace* w = nullptr;
   if ((rc = get_workspace(eng, g, W, mode, &w))) return rc;
   const bool reduce = stats_dev != nullptr;
-  if (reduce && !eng->host_loop && w->exec[0] && !w->exec[1] &&
-      build_graph_exec(eng, w, PASS_STATS) != MSBFS_OK) {
-    eng->host_loop = true;
-    cudaGetLastError();
-  }
-  // Split materialisation (graph loop only): the pass's graph ends after
-  // the byte rows; the u32 rows and the cleanup follow as plain launches
-  // while the host widens the bytes.
-  bool split = split_frac > 0.0 && dist8_dev && dist_dev && !reduce && !reach_dev &&
-               eng->profiling == 0 && !eng->host_loop && w->exec[PASS_ROWS];
-  if (split && !w->exec[PASS_BYTES] && build_graph_exec(eng, w, PASS_BYTES) != MSBFS_OK) {
-    cudaGetLastError();
-    split = false;
-  }
+  // Split materialisation (one-launch traversal only): the u32 rows follow
+  // the byte rows in a second launch, while the host widens the bytes.
+  const bool one_launch = !eng->host_loop && eng->profiling == 0;
+  const bool split = split_frac > 0.0 && dist8_dev && dist_dev && !reduce && !reach_dev && one_launch;
   eng->last_split = split;
   eng->split_rows.assign(passes, 0);
   while (split && eng->split_events.size() < passes) {
@@ -748,23 +643,22 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
     d.reach_col = (uint32_t)(ps * W);
     d.row_split = split ? (uint32_t)(split_frac * (double)np) / 32u * 32u : 0u;
     eng->split_rows[ps] = d.row_split;
-    // Pageable source: the copy is staged before the call returns, so the
-    // stack descriptor can go out of scope.
-    CK(cudaMemcpyAsync(w->d_desc, &d, sizeof d, cudaMemcpyHostToDevice, eng->stream));
+    w->p.d = d;
+    if ((rc = next_epoch(eng, w))) return rc;
     if (eng->profiling >= 2) {
       if ((rc = run_pass_profiled(eng, w, reduce, &eng->pass_event_ms[ps]))) return rc;
-    } else if (split) {
-      CK(cudaGraphLaunch(w->exec[PASS_BYTES], eng->stream));
-      CK(cudaMemcpyAsync(&eng->h_ctl[ps], w->d_ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost,
-                         eng->stream));
-      CK(cudaEventRecord(eng->split_events[ps], eng->stream));
-      launch_materialize(w->p, w->k, false, eng->stream, MAT_WIDE);
-      launch_cleanup(w->p, eng->stream);
-      CK(cudaGetLastError());
-    } else if (w->exec[reduce] && !eng->host_loop) {
-      CK(cudaGraphLaunch(w->exec[reduce], eng->stream));
-    } else {
+    } else if (!one_launch) {
       if ((rc = run_pass_host_loop(eng, w, reduce))) return rc;
+    } else {
+      CK(launch_traverse(w->p, w->k, eng->stream));
+      if (split) {
+        launch_materialize(w->p, w->k, false, eng->stream, MAT_BYTES);
+        CK(cudaMemcpyAsync(&eng->h_ctl[ps], w->d_ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost,
+                           eng->stream));
+        CK(cudaEventRecord(eng->split_events[ps], eng->stream));
+      }
+      launch_materialize(w->p, w->k, reduce, eng->stream, split ? MAT_WIDE : MAT_ALL);
+      CK(cudaGetLastError());
     }
     CK(cudaMemcpyAsync(&eng->h_ctl[ps], w->d_ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost,
                        eng->stream));
@@ -844,77 +738,105 @@ int finish_call(msbfs_engine* eng, msbfs_stats* stats) {
   if (status & STATUS_CHECK)
     return set_err(eng, MSBFS_ERR_CUDA,
                    "bounds check failed at site " + std::to_string(check_site));
+  if (status & STATUS_STUCK) {
+    CK(cudaStreamSynchronize(eng->stream));
+    eng->ws.clear();  // the pass left its traversal state as it was
+    return set_err(eng, MSBFS_ERR_TIMEOUT, "a level's grid barrier ran out of time");
+  }
   if (status & STATUS_LEVEL_CAP) return set_err(eng, MSBFS_ERR_TIMEOUT, "level cap reached");
   if (status & STATUS_BAD_SOURCE) return set_err(eng, MSBFS_ERR_SOURCE_OOB, "source out of range");
   return MSBFS_OK;
 }
 
-// Slice table of in-edge lists longer than `split` and the bottom-up work
+// Slice table of the vertices of in-degree >= heavy and the bottom-up work
 // list of the other vertices with in-edges, from the graph's host CSC
-// offsets. Rebuilt when the autotuner changes the slice length; the caller
-// drops the workspaces that point at the old tables first.
-int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split) {
+// offsets. Rebuilt when the autotuner changes the slice length or the
+// in-degree; the caller drops the workspaces that point at the old tables
+// first.
+int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, uint32_t heavy) {
   const size_t V = g->V;
   const std::vector<uint32_t>& coff = g->h_coff;
-  cudaFree(g->hchunks);
+  cudaFree(g->slices);
+  cudaFree(g->hslices);
   cudaFree(g->order);
-  g->hchunks = nullptr;
+  g->slices = nullptr;
+  g->hslices = nullptr;
   g->order = nullptr;
   g->split = split;
+  g->heavy = heavy;
   g->n_heavy = 0;
-  std::vector<HeavyChunk> chunks;
-  for (size_t v = 0; v < V; ++v) {
-    const uint32_t indeg = coff[v + 1] - coff[v];
-    if (indeg <= split) continue;
-    const uint32_t nch = (indeg + split - 1) / split;
-    for (uint32_t j = 0; j < nch; ++j) chunks.push_back(HeavyChunk{(uint32_t)v, j, nch, g->n_heavy});
-    g->n_heavy++;
+  // A slice is one warp's serial work. With fewer than two full slices of
+  // edges per resident warp, shorter ones: a level of a small graph lasts as
+  // long as its longest slice (directed R-MAT 18, S=333: bottom-up levels of
+  // 220 us behind warps that scanned up to 16 vertices of <= 512 in-edges).
+  uint32_t len = split;
+  const uint64_t warps = (uint64_t)eng->num_sms * 64;
+  while (len > 64 && (uint64_t)len * 2 * warps > g->E) len /= 2;
+  // Heavy vertices by in-degree, descending (a counting sort; those beyond
+  // its range keep their order in front).
+  constexpr uint32_t TOP = 1u << 16;
+  std::vector<uint32_t> at(TOP + 1, 0), by_degree;
+  auto degree_rank = [&](size_t v) { return TOP - 1 - std::min(coff[v + 1] - coff[v], TOP - 1); };
+  heavy = std::max(heavy, 1u);
+  for (size_t v = 0; v < V; ++v)
+    if (coff[v + 1] - coff[v] >= heavy) at[degree_rank(v) + 1]++;
+  for (uint32_t i = 0; i < TOP; ++i) at[i + 1] += at[i];
+  by_degree.resize(at[TOP]);
+  for (size_t v = 0; v < V; ++v)
+    if (coff[v + 1] - coff[v] >= heavy) by_degree[at[degree_rank(v)]++] = (uint32_t)v;
+  std::vector<uint32_t> per_vertex;  // slices of each vertex of several
+  std::vector<uint32_t> h(by_degree.size());
+  size_t many = 0;  // the vertices of several slices come first
+  for (size_t i = 0; i < by_degree.size(); ++i) {
+    const uint32_t v = by_degree[i], d = coff[v + 1] - coff[v];
+    h[i] = d > len ? g->n_heavy++ : SLICE_H;
+    if (d > len) {
+      per_vertex.push_back((d + len - 1) / len);
+      many = i + 1;
+    }
   }
-  // Longest lists first so their slices start early in every bottom-up step.
-  std::stable_sort(chunks.begin(), chunks.end(), [](const HeavyChunk& a, const HeavyChunk& b) {
-    return a.nch > b.nch;
-  });
-  g->n_hchunks = (uint32_t)chunks.size();
-  CK(cudaMalloc((void**)&g->hchunks, std::max<size_t>(chunks.size(), 1) * sizeof(HeavyChunk)));
-  if (!chunks.empty())
-    CK(cudaMemcpy(g->hchunks, chunks.data(), chunks.size() * sizeof(HeavyChunk),
-                  cudaMemcpyHostToDevice));
-  // Bottom-up work list: the vertices with 0 < in-degree <= split, ascending
-  // ids (neighbouring vertices share cache lines of the visited and frontier
-  // rows). MSBFS_ORDER_WINDOW > 1 sorts by in-degree, descending, within
-  // windows of that many entries, so the groups of a warp scan in-edge lists
-  // of similar length; on R-MAT scale 22, S=512 the lost locality outweighs
-  // the balance (window 256: +8%, window 1024: +10% bottom-up time), so the
-  // default keeps plain id order.
-#ifndef MSBFS_ORDER_WINDOW
-#define MSBFS_ORDER_WINDOW 0
-#endif
-  std::vector<uint32_t> order;
-  order.reserve(V);
-  for (size_t v = 0; v < V; ++v) {
-    const uint32_t d = coff[v + 1] - coff[v];
-    if (d > 0 && d <= split) order.push_back((uint32_t)v);
+  // First slices first: by the time a vertex's later slices run, the lanes
+  // its first ones found are published, and they can stop at once.
+  std::vector<uint4> slices;
+  for (uint32_t j = 0;; ++j) {
+    const size_t before = slices.size();
+    for (size_t i = 0; i < (j ? many : by_degree.size()); ++i) {
+      const uint32_t v = by_degree[i], d = coff[v + 1] - coff[v];
+      const uint64_t first = (uint64_t)j * len;
+      if (first >= d) {
+        if (d < TOP - 1) break;  // shorter lists follow
+        continue;
+      }
+      const uint32_t sb = coff[v] + (uint32_t)first;
+      const uint32_t se = d - first > len ? sb + len : coff[v + 1];
+      slices.push_back(make_uint4(v, sb, se, h[i] | (j ? 0u : SLICE_FIRST)));
+    }
+    if (slices.size() == before) break;
   }
-  const size_t win = MSBFS_ORDER_WINDOW;
-  if (win > 1) {
-    auto deg_desc = [&](uint32_t a, uint32_t b) {
-      return coff[a + 1] - coff[a] > coff[b + 1] - coff[b];
-    };
-    for (size_t i = 0; i < order.size(); i += win)
-      std::stable_sort(order.begin() + i, order.begin() + std::min(order.size(), i + win),
-                       deg_desc);
-  }
-  g->n_order = (uint32_t)order.size();
+  g->n_slices = (uint32_t)slices.size();
+  // Bottom-up work list: the other vertices with in-edges, ascending ids
+  // (neighbouring vertices share cache lines of the visited and frontier
+  // rows; sorting them by in-degree within windows of 256 or 1,024 entries,
+  // for groups of similar length, cost 8 and 10% on R-MAT scale 22, S=512).
   // Each entry carries the vertex and its in-edge range, so a bottom-up
   // step starts a vertex's scan one dependent load earlier.
-  std::vector<uint4> ent(order.size());
-  for (size_t i = 0; i < order.size(); ++i) {
-    const uint32_t v = order[i];
-    ent[i] = make_uint4(v, coff[v], coff[v + 1], 0u);
+  std::vector<uint4> order;
+  order.reserve(V);
+  for (size_t v = 0; v < V; ++v) {
+    const uint32_t b = coff[v], e = coff[v + 1];
+    if (e > b && e - b < heavy) order.push_back(make_uint4((uint32_t)v, b, e, 0u));
   }
-  CK(cudaMalloc((void**)&g->order, std::max<size_t>(ent.size(), 1) * sizeof(uint4)));
-  if (!ent.empty())
-    CK(cudaMemcpy(g->order, ent.data(), ent.size() * sizeof(uint4), cudaMemcpyHostToDevice));
+  g->n_order = (uint32_t)order.size();
+  auto upload = [&](const void* src, size_t bytes, void** dst) -> int {
+    CK(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
+    if (bytes) CK(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
+    return MSBFS_OK;
+  };
+  int rc;
+  if ((rc = upload(slices.data(), slices.size() * sizeof(uint4), (void**)&g->slices)) ||
+      (rc = upload(per_vertex.data(), per_vertex.size() * sizeof(uint32_t), (void**)&g->hslices)) ||
+      (rc = upload(order.data(), order.size() * sizeof(uint4), (void**)&g->order)))
+    return rc;
   return MSBFS_OK;
 }
 
@@ -950,7 +872,7 @@ int upload_graph(msbfs_engine* eng, size_t V, size_t E, const uint32_t* off, con
     if (E) CK(cudaMemcpy(g->cidx, t.idx.data(), E * 4, cudaMemcpyHostToDevice));
   }
   g->h_coff = std::move(t.off);
-  int rc = build_bottom_up_tables(eng, g.get(), eng->split);
+  int rc = build_bottom_up_tables(eng, g.get(), eng->split, eng->heavy);
   if (rc) return rc;
   // Road-like graphs (the ones the router sends to the CTA path) get edge
   // records, 8 bytes per edge, so a CTA-path level costs one dependent L2
@@ -987,7 +909,8 @@ void free_graph(msbfs_graph* g) {
   }
   cudaFree(g->off);
   cudaFree(g->idx);
-  cudaFree(g->hchunks);
+  cudaFree(g->slices);
+  cudaFree(g->hslices);
   cudaFree(g->order);
   cudaFree(g->erec);
   delete g;
@@ -1198,8 +1121,12 @@ int msbfs_engine_create(int device, int method, msbfs_engine** out) {
       cudaMalloc((void**)&e->d_counter, sizeof(unsigned long long)) != cudaSuccess)
     return MSBFS_ERR_CUDA;
   e->stream = e->own_stream;
+  size_t free_mem = 0;
+  cudaMemGetInfo(&free_mem, &e->total_mem);
   const char* hl = getenv("MSBFS_HOST_LOOP");
-  e->host_loop = hl && hl[0] == '1';
+  int coop = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+  e->host_loop = !coop || (hl && hl[0] == '1');
   const char* zc = getenv("MSBFS_ZERO_COPY");
   e->zero_copy = !(zc && zc[0] == '0');
   const char* nr = getenv("MSBFS_NARROW");
@@ -1267,7 +1194,7 @@ int msbfs_engine_set_tuning(msbfs_engine* e, uint32_t max_words, uint32_t alpha,
   if (beta) e->beta = beta;
   cudaSetDevice(e->device);
   cudaStreamSynchronize(e->stream);
-  e->ws.clear();  // thresholds are baked into the captured graphs
+  e->ws.clear();  // thresholds are baked into the workspaces
   return MSBFS_OK;
 }
 
@@ -1279,7 +1206,7 @@ int msbfs_engine_set_sm_share(msbfs_engine* e, uint32_t percent) {
   e->sm_share = percent;
   cudaSetDevice(e->device);
   cudaStreamSynchronize(e->stream);
-  e->ws.clear();  // grid sizes are baked into the captured graphs
+  e->ws.clear();  // grid sizes are baked into the workspaces
   return MSBFS_OK;
 }
 
@@ -1289,7 +1216,7 @@ int msbfs_engine_set_level_cap(msbfs_engine* e, uint32_t max_levels) {
   e->level_cap = max_levels;
   cudaSetDevice(e->device);
   cudaStreamSynchronize(e->stream);
-  e->ws.clear();  // the cap is baked into the captured graphs
+  e->ws.clear();  // the cap is baked into the workspaces
   return MSBFS_OK;
 }
 
@@ -1298,7 +1225,7 @@ int msbfs_engine_set_profiling(msbfs_engine* e, int level) {
   std::lock_guard<std::mutex> lk(e->mu);
   auto counting = [](int l) { return l == 1 || l == 2; };
   if (counting(e->profiling) != counting(level)) {
-    // The captured graphs hold the counting or the production level kernels.
+    // The workspaces hold the counting or the production level kernels.
     cudaSetDevice(e->device);
     cudaStreamSynchronize(e->stream);
     e->ws.clear();
@@ -1525,8 +1452,8 @@ struct LevelSettings {
   }
 };
 
-// The thresholds are baked into an engine's captured graphs, so its
-// workspaces are dropped; a new slice length rebuilds the graph's bottom-up
+// The thresholds are baked into an engine's workspaces, so they
+// are dropped; a new slice length rebuilds the graph's bottom-up
 // tables (done only when no other engine runs on the graph).
 int apply_settings(msbfs_engine* eng, msbfs_graph* g, const LevelSettings& s) {
   CK(cudaStreamSynchronize(eng->stream));
@@ -1537,7 +1464,8 @@ int apply_settings(msbfs_engine* eng, msbfs_graph* g, const LevelSettings& s) {
   eng->beta = s.beta;
   eng->bits_div = s.bits_div;
   eng->heavy = s.heavy;
-  if (s.split != g->split) return build_bottom_up_tables(eng, g, s.split);
+  if (s.split != g->split || s.heavy != g->heavy)
+    return build_bottom_up_tables(eng, g, s.split, s.heavy);
   return MSBFS_OK;
 }
 
@@ -1577,7 +1505,7 @@ extern "C" int msbfs_engine_autotune(msbfs_engine* e, msbfs_graph* g, const uint
       msbfs::graph_class(g->V, g->E, g->max_deg) + "/s" + std::to_string(bucket);
   msbfs_tuning t{};
   std::strncpy(t.class_name, key.c_str(), sizeof t.class_name - 1);
-  LevelSettings best{e->max_words, e->alpha, e->beta, g->split, e->bits_div, e->heavy};
+  LevelSettings best{widest_pass(e, g), e->alpha, e->beta, g->split, e->bits_div, g->heavy};
   auto report = [&](const LevelSettings& s) {
     // The words a pass of this call uses (a cap above the sources' need
     // makes no difference).
@@ -1605,7 +1533,10 @@ extern "C" int msbfs_engine_autotune(msbfs_engine* e, msbfs_graph* g, const uint
     double ms = 0;
     while (in >> k >> s.words >> s.alpha >> s.beta >> s.split >> s.bits_div >> s.heavy >> ms) {
       if (k != key) continue;
-      if (shared) s.split = g->split;
+      if (shared) {
+        s.split = g->split;
+        s.heavy = g->heavy;
+      }
       if ((rc = apply_settings(e, g, s))) return rc;
       t.from_cache = 1;
       t.ms = ms;
@@ -1628,7 +1559,7 @@ extern "C" int msbfs_engine_autotune(msbfs_engine* e, msbfs_graph* g, const uint
   // One setting at a time, each from the best found so far; a change is
   // kept only when it is at least 2% faster (timing noise).
   for (int i = 0; i < 6; ++i) {
-    if (i == 3 && shared) continue;
+    if ((i == 3 || i == 5) && shared) continue;
     const LevelSettings base = best;
     for (uint32_t c : cands[i]) {
       LevelSettings s = base;

@@ -1,10 +1,10 @@
 // Level-synchronous bit-parallel multi-source BFS kernels for sm_103a.
 //
 // One pass traverses up to 32*W sources at once: lane s of word s/32 of a
-// vertex's W-word row belongs to source s. A level is one launch of
-// level_kernel<W, DIR>, a bottom-up (pull) or a top-down (push) step, as
-// decided on the device by the previous level; the loop itself is a
-// CUDA-graph WHILE node whose condition the last block of each level sets.
+// vertex's W-word row belongs to source s. A level is a bottom-up (pull) or a
+// top-down (push) step, as decided on the device by the previous level; all
+// levels of a pass run in one cooperative launch of traverse_kernel<W>, one
+// grid barrier apart.
 //
 // Semantics follow the reference's WGSL kernels:
 //   bottom-up step  crates/shaders/src/multi_word_bp_pull_512.wgsl:69-138
@@ -22,7 +22,7 @@
 // warp per heavy vertex, warp-aggregated atomics, block-staged queue
 // compaction, bit-sliced level planes materialised into coalesced rows) is
 // this file's own.
-#include <cooperative_groups.h>
+#pragma once
 
 #include "device_common.cuh"
 
@@ -37,14 +37,15 @@ constexpr int BQ_CAP = 2048;  // discovered vertices staged per block
 #define MSBFS_PULL_CH 4
 #endif
 #ifndef MSBFS_LEVEL_MIN_BLOCKS
-// 8 resident blocks of 256 threads (all 64 warps of an SM, 32 registers):
-// the bottom-up gathers are latency-bound, and the extra warps outweigh the
-// spilled registers (R-MAT scale 22, S=512: dense levels 2.29 -> 1.92 ms
-// against 6 blocks at 40 registers; 4 and 5 blocks were slower still).
-#define MSBFS_LEVEL_MIN_BLOCKS (2048 / MSBFS_LEVEL_BLOCK)
+// 6 resident blocks of 256 threads (48 warps an SM, 40 registers). The
+// bottom-up gathers are latency-bound: fewer warps leave them waiting, more
+// spill, and every block takes part in the grid barriers. us of a traversal
+// at 8 / 6 / 5 / 4 blocks: R-MAT 22 S=512 5,358 / 5,312 / 5,482 / 5,740,
+// R-MAT 21 S=64 1,080 / 1,022 / 1,048 / 1,163, R-MAT 17 S=129 347 / 277 /
+// 265 / 261.
+#define MSBFS_LEVEL_MIN_BLOCKS (1536 / MSBFS_LEVEL_BLOCK)
 #endif
 constexpr int CH = MSBFS_PULL_CH;  // in-neighbours gathered per chunk
-constexpr int MAT_BLOCK = 256;
 constexpr uint32_t FULL = 0xffffffffu;
 constexpr uint32_t DIST_MAX = 0xffffffffu;
 
@@ -55,7 +56,7 @@ constexpr uint32_t DIST_MAX = 0xffffffffu;
 // into MSBFS_ERR_CUDA naming the site. The default build compiles the
 // checks out.
 #ifdef MSBFS_BOUNDS_CHECK
-__device__ __noinline__ void check_fail(LevelCtl* c, uint32_t site) {
+static __device__ __noinline__ void check_fail(LevelCtl* c, uint32_t site) {
   atomicOr(&c->status, STATUS_CHECK);
   atomicCAS(&c->check_site, 0u, site);
 }
@@ -72,7 +73,7 @@ __device__ __noinline__ void check_fail(LevelCtl* c, uint32_t site) {
 // Check sites (reported by the host as "bounds check failed at site N").
 enum : uint32_t {
   CK_TILE_LOOP = 1, CK_ORDER_ENTRY = 3, CK_GATHER_ID = 4, CK_SLICE = 5,
-  CK_PUSH_ENTRY = 6, CK_PUSH_TARGET = 7, CK_CLEAR_ENTRY = 8, CK_QUEUE_CAP = 9
+  CK_PUSH_ENTRY = 6, CK_PUSH_TARGET = 7, CK_QUEUE_CAP = 9
 };
 
 template <int W>
@@ -102,53 +103,23 @@ __device__ __forceinline__ Words<VEC> ld_words(const uint32_t* p) {
   return r;
 }
 
-// Read-only path: frontier words of the level being expanded and the graph.
+// Frontier words of the level being expanded: cached in L1, but not on the
+// read-only path, which may not be used for words that this launch writes
+// (the traversal runs all its levels in one launch, and its grid barrier
+// orders ordinary loads only).
 template <int VEC>
-__device__ __forceinline__ Words<VEC> ldg_words(const uint32_t* p) {
+__device__ __forceinline__ Words<VEC> ldca_words(const uint32_t* p) {
   Words<VEC> r;
   if constexpr (VEC == 4) {
-    uint4 t = __ldg(reinterpret_cast<const uint4*>(p));
+    uint4 t = __ldca(reinterpret_cast<const uint4*>(p));
     r.w[0] = t.x; r.w[1] = t.y; r.w[2] = t.z; r.w[3] = t.w;
   } else if constexpr (VEC == 2) {
-    uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
+    uint2 t = __ldca(reinterpret_cast<const uint2*>(p));
     r.w[0] = t.x; r.w[1] = t.y;
   } else {
-    r.w[0] = __ldg(p);
+    r.w[0] = __ldca(p);
   }
   return r;
-}
-
-// Frontier-row gathers of the bottom-up step (random rows, L1 hit rate
-// 14-21% on R-MAT 22). MSBFS_GATHER_LOAD picks the cache path: 0 the
-// read-only path, 1 the same without allocating in L1, 2 L2 only. R-MAT
-// scale 22, S=512, step ms: 7.54 / 8.03 / 7.63 -- the hubs' rows that L1
-// keeps are worth its allocation traffic.
-#ifndef MSBFS_GATHER_LOAD
-#define MSBFS_GATHER_LOAD 0
-#endif
-template <int VEC>
-__device__ __forceinline__ Words<VEC> gather_words(const uint32_t* p) {
-  if constexpr (MSBFS_GATHER_LOAD == 1 && VEC == 4) {
-    Words<VEC> r;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3])
-                 : "l"(p));
-    return r;
-  } else if constexpr (MSBFS_GATHER_LOAD == 2) {
-    Words<VEC> r;
-    if constexpr (VEC == 4) {
-      uint4 t = __ldcg(reinterpret_cast<const uint4*>(p));
-      r.w[0] = t.x; r.w[1] = t.y; r.w[2] = t.z; r.w[3] = t.w;
-    } else if constexpr (VEC == 2) {
-      uint2 t = __ldcg(reinterpret_cast<const uint2*>(p));
-      r.w[0] = t.x; r.w[1] = t.y;
-    } else {
-      r.w[0] = __ldcg(p);
-    }
-    return r;
-  } else {
-    return ldg_words<VEC>(p);
-  }
 }
 
 // L2-coherent read of words other blocks update with atomics this level.
@@ -190,17 +161,23 @@ __device__ __forceinline__ uint32_t nseg_of(uint32_t deg, uint32_t seg) {
   return deg ? (deg + seg - 1) / seg : 1u;
 }
 
+// A vertex of this many queue entries has them written by the whole block.
+constexpr uint32_t BIG_ITEM = 16;
+constexpr uint32_t BIG_CAP = 64;  // such vertices per flush; the rest are written one by one
+
 struct BlockQueue {
   uint32_t items[BQ_CAP];
   uint32_t count;
   uint32_t base;
   uint32_t warp_sum[LEVEL_BLOCK / 32];
   unsigned long long warp_edges[LEVEL_BLOCK / 32];
+  uint32_t n_big;
+  uint3 big[BIG_CAP];  // {vertex, first position, entries}
 };
 
 // Enqueue straight into the global queue (sources, and blocks whose staging
 // area is full). Entry i of vertex v covers out-edges [i*seg, (i+1)*seg).
-__device__ void enqueue_global(const LevelParams& p, uint32_t slot, uint32_t v, uint32_t seg) {
+static __device__ void enqueue_global(const LevelParams& p, uint32_t slot, uint32_t v, uint32_t seg) {
   const uint32_t deg = p.out_off[v + 1] - p.out_off[v];
   const uint32_t n = nseg_of(deg, seg);
   const uint32_t base = atomicAdd(&p.ctl->qcount[slot], n);
@@ -222,7 +199,7 @@ __device__ __forceinline__ void bq_push(const LevelParams& p, BlockQueue& bq, ui
 
 // Compacts the block's staged vertices into the global queue with one
 // atomicAdd per block: per-item segment counts, block-wide exclusive scan.
-__device__ void flush_block_queue(const LevelParams& p, BlockQueue& bq, uint32_t slot) {
+static __device__ void flush_block_queue(const LevelParams& p, BlockQueue& bq, uint32_t slot) {
   __syncthreads();
   const uint32_t n = min(bq.count, (uint32_t)BQ_CAP);
   if (n == 0) return;  // uniform: read after the barrier
@@ -258,6 +235,7 @@ __device__ void flush_block_queue(const LevelParams& p, BlockQueue& bq, uint32_t
       run += t;
       etot += bq.warp_edges[w];
     }
+    bq.n_big = 0;
     bq.base = atomicAdd(&p.ctl->qcount[slot], run);
     atomicAdd(&p.ctl->qverts[slot], n);
     atomicAdd(&p.ctl->qedges[slot], etot);
@@ -269,9 +247,23 @@ __device__ void flush_block_queue(const LevelParams& p, BlockQueue& bq, uint32_t
     const uint32_t v = bq.items[i];
     const uint32_t deg = p.out_off[v + 1] - p.out_off[v];
     const uint32_t ns = nseg_of(deg, p.seg);
+    const uint32_t big = ns >= BIG_ITEM ? atomicAdd(&bq.n_big, 1u) : BIG_CAP;
+    if (big < BIG_CAP) {
+      bq.big[big] = make_uint3(v, pos, ns);
+      pos += ns;
+      continue;
+    }
     for (uint32_t s = 0; s < ns; ++s, ++pos)
       if (BCHECK(pos < (slot == 0 ? p.qcap0 : p.qcap), CK_QUEUE_CAP))
         Q[pos] = ((unsigned long long)s << 32) | v;
+  }
+  __syncthreads();
+  const uint32_t n_big = min(bq.n_big, BIG_CAP);
+  for (uint32_t k = 0; k < n_big; ++k) {
+    const uint3 it = bq.big[k];
+    for (uint32_t s = tid; s < it.z; s += LEVEL_BLOCK)
+      if (BCHECK(it.y + s < (slot == 0 ? p.qcap0 : p.qcap), CK_QUEUE_CAP))
+        Q[it.y + s] = ((unsigned long long)s << 32) | it.x;
   }
 }
 
@@ -302,8 +294,8 @@ __device__ __forceinline__ void record_level(const LevelParams& p, uint32_t v, u
     // Deeper than the planes can encode: mark the lanes and write the rows.
     // With per-source reductions instead of rows, the deep lanes are folded
     // into the reductions here.
-    uint32_t* dist = p.desc->dist;  // null when reductions or reachability are wanted
-    SourceStats* st = p.desc->stats;
+    uint32_t* dist = p.d.dist;  // null when reductions or reachability are wanted
+    SourceStats* st = p.d.stats;
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
       uint32_t bits = newly.w[j];
@@ -355,19 +347,22 @@ __device__ __forceinline__ Words<VEC> alive_lanes(const uint32_t* s_alive, uint3
   return m;
 }
 
-// Visited/frontier/level/queue writes for a vertex owned by the calling group
-// (all LPV lanes call it with their own VEC words).
+// Visited/frontier/level writes for a vertex owned by the calling group (all
+// LPV lanes call it with their own VEC words).
 // The visited words are read again here rather than held in registers
 // through the gather loop (the group owns the vertex: nothing else writes
-// them during the level).
+// them during the level). The new frontier is recorded as membership bits
+// only: the next bottom-up step needs no queue, and one for a top-down step
+// is built from the bits (build_queue).
 template <int W, int VEC>
-__device__ __forceinline__ void pull_commit(const LevelParams& p, BlockQueue& bq, uint32_t* s_lanes,
-                                            uint32_t L, uint32_t v, uint32_t k0, uint32_t lig,
+__device__ __forceinline__ void pull_commit(const LevelParams& p, uint32_t* s_lanes, uint32_t L,
+                                            uint32_t v, uint32_t k0, uint32_t lig,
                                             const Words<VEC>& newly, LevelCounters& cnt) {
 #pragma unroll
   for (int q = 0; q < VEC; ++q) {
     cnt.pairs += __popc(newly.w[q]);
-    if (newly.w[q]) atomicOr(s_lanes + k0 + q, newly.w[q]);
+    if (newly.w[q] & ~*(volatile uint32_t*)(s_lanes + k0 + q))
+      atomicOr(s_lanes + k0 + q, newly.w[q]);
   }
   // A lane whose words gained nothing leaves them as they are: its visited
   // words are unchanged, its frontier words of level L+1 are already zero
@@ -385,7 +380,6 @@ __device__ __forceinline__ void pull_commit(const LevelParams& p, BlockQueue& bq
   if (lig == 0) {
     cnt.newv += 1;
     atomicOr(p.fbits[(L + 1) % 3] + (v >> 5), 1u << (v & 31));
-    bq_push(p, bq, (L + 1) % 3, v);
   }
 }
 
@@ -393,17 +387,16 @@ __device__ __forceinline__ void pull_commit(const LevelParams& p, BlockQueue& bq
 // 16-byte row loads; with a dense one the extra dependent load costs more
 // than it saves, so the controller turns the check off (`fb` null).
 __device__ __forceinline__ bool in_frontier(const uint32_t* fb, uint32_t u) {
-  return !fb || ((__ldg(fb + (u >> 5)) >> (u & 31)) & 1u);
+  return !fb || ((__ldca(fb + (u >> 5)) >> (u & 31)) & 1u);
 }
 
-// Vertex tiles a warp claims per cursor bump: small batches even out the end
-// of a level (R-MAT scale 22, S=512, 8 blocks per SM, slices of 512: a step
-// takes 8.59 ms with 2 tiles, 8.52 with 1, 8.83 with 4; at 6 blocks and
-// slices of 256, 4 tiles had been 8% and 8 tiles 6% below 16).
+// Vertex tiles a warp claims per cursor bump (small batches even out the end
+// of a level).
 #ifndef MSBFS_TILE_BATCH
 #define MSBFS_TILE_BATCH 2
 #endif
 constexpr uint32_t TILE_BATCH = MSBFS_TILE_BATCH;
+constexpr uint32_t TURN_TILES = 8;  // tiles per warp up to which none are claimed
 
 // In-neighbour id as gathered: FULL when absent or, with a frontier bitmap,
 // outside the frontier (so its row is not loaded). The lane holding an id
@@ -415,178 +408,200 @@ __device__ __forceinline__ uint32_t gather_id(const LevelParams& p, const uint32
 }
 
 // Bottom-up step over all vertices, in two parts.
-// (1) Sliced vertices (in-degree > split): each warp takes one slice of one
-//     vertex's in-edges, ORs the in-neighbours' frontier rows (every group of
-//     the warp takes CH of them per round), publishes the partial candidate
-//     words with atomicOr, and the last slice to arrive commits the vertex.
+// (1) Vertices of in-degree >= heavy, in slices of at most `split` in-edges:
+//     a warp takes one slice, ORs the in-neighbours' frontier rows (every
+//     group of the warp takes CH of them per round) and stops once they cover
+//     every lane still to be discovered. A vertex of one slice is committed
+//     at once; the slices of a longer list publish their partial candidate
+//     words with atomicOr, and the last one to arrive commits the vertex.
 // (2) Every other vertex: a group of LPV lanes owns it, each lane holding VEC
 //     of its W words; in-neighbours are gathered CH at a time (CH independent
-//     16-byte loads in flight per lane) and the scan stops once the candidate
-//     words cover every lane still to be discovered. Vertices with in-degree
-//     >= heavy are scanned by the whole warp.
+//     16-byte loads in flight per lane), with the same early stop.
 template <int W>
-__device__ void pull_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lanes,
-                           const uint32_t* s_alive, uint32_t L, LevelCounters& cnt) {
+__device__ __forceinline__ void pull_phase(const LevelParams& p, uint32_t* s_lanes,
+                                           const uint32_t* s_alive, uint32_t L,
+                                           LevelCounters& cnt) {
   using G = Geo<W>;
   constexpr int VEC = G::VEC, LPV = G::LPV, GPW = G::GPW;
+  constexpr int NI = LPV >= CH ? 1 : CH;  // in-neighbour ids held per lane
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t lig = lane % LPV;
   const uint32_t gbase = lane - lig;
   const uint32_t gid = lane / LPV;
   const uint32_t gmask = (LPV == 32) ? FULL : (((1u << LPV) - 1u) << gbase);
   const uint32_t k0 = lig * VEC;
-  const uint32_t* __restrict__ Fin = p.F[L % 3];
-  const uint32_t* __restrict__ fb =
-      *(volatile uint32_t*)&p.ctl->use_bits ? p.fbits[L % 3] : nullptr;
-  const uint32_t* __restrict__ in_off = p.in_off;
+  const uint32_t* Fin = p.F[L % 3];
+  const uint32_t* fb = __ldcg(&p.ctl->use_bits) ? p.fbits[L % 3] : nullptr;
   const uint32_t* __restrict__ in_idx = p.in_idx;
   const uint32_t warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
 
-  // ---- (1) sliced high in-degree vertices. A warp takes its slices 32 at a
-  // time and first tests their bits in p.hlive, so slices whose vertex needs
-  // no lane any more (cleared below, for the rest of the pass) cost one bit
-  // test instead of a chain of dependent loads.
-  for (uint32_t cb = warp_g; cb < p.n_hchunks; cb += 32 * nwarps) {
+  // ---- (1) slices. A warp takes its slices 32 at a time and first tests
+  // their bits in p.hlive, so slices whose vertex needs no lane any more
+  // (cleared below, for the rest of the pass) cost one bit test instead of a
+  // chain of dependent loads.
+  for (uint32_t cb = warp_g; cb < p.n_slices; cb += 32 * nwarps) {
     const uint32_t mine = cb + lane * nwarps;
-    const bool live = mine < p.n_hchunks && ((p.hlive[mine >> 5] >> (mine & 31)) & 1u);
+    const bool live = mine < p.n_slices && ((p.hlive[mine >> 5] >> (mine & 31)) & 1u);
     uint32_t todo = __ballot_sync(FULL, live);
-   while (todo) {
-    const uint32_t ci = cb + (__ffs(todo) - 1) * nwarps;
-    todo &= todo - 1;
-    const HeavyChunk hk = p.hchunks[ci];
-    const uint32_t v = hk.v;
-    if (!BCHECK(v < p.V && hk.j < hk.nch, CK_SLICE)) continue;
-    const uint32_t vb = __ldg(in_off + v);
-    const uint32_t beg = vb + hk.j * p.split;
-    const uint32_t end = min(__ldg(in_off + v + 1), beg + p.split);
-    const Words<VEC> visw = ld_words<VEC>(p.vis + (size_t)v * W + k0);
-    Words<VEC> needed, hc, shared_c;
-    bool sat = true;
-    uint32_t* hrow = p.hcand + (size_t)hk.h * W + k0;
-    shared_c = ldcg_words<VEC>(hrow);
-    const Words<VEC> lmask = alive_lanes<VEC>(s_alive, k0);
+    while (todo) {
+      const uint32_t ci = cb + (__ffs(todo) - 1) * nwarps;
+      todo &= todo - 1;
+      const uint4 sl = __ldg(p.slices + ci);
+      const uint32_t v = sl.x, beg = sl.y, end = sl.z, h = sl.w & SLICE_H;
+      if (!BCHECK(v < p.V && beg <= end && end <= p.E, CK_SLICE)) continue;
+      const bool whole = h == SLICE_H;  // the vertex's only slice
+      uint32_t* hrow = p.hcand + (whole ? 0 : (size_t)h * W) + k0;
+      Words<VEC> needed = ld_words<VEC>(p.vis + (size_t)v * W + k0), hc;
+      const Words<VEC> lmask = alive_lanes<VEC>(s_alive, k0);
+      bool sat = !whole;
+      if (!whole) hc = ldcg_words<VEC>(hrow);
 #pragma unroll
-    for (int q = 0; q < VEC; ++q) {
-      needed.w[q] = ~visw.w[q] & lmask.w[q];
-      hc.w[q] = 0;
-      sat &= (shared_c.w[q] & needed.w[q]) == needed.w[q];
-    }
-    // Every slice of v sees the same `needed` (only the committing slice
-    // writes v's visited row, after all slices arrived).
-    if (!__any_sync(FULL, any_bits<VEC>(needed))) {
-      if (lane == 0) atomicAnd(&p.hlive[ci >> 5], ~(1u << (ci & 31)));
-      continue;
-    }
-    if (hk.j == 0 && lane == 0) cnt.active += 1;
-    if (!__all_sync(FULL, sat)) {
-      // Each round the warp gathers GPW*CH in-neighbours; the ids of the next
-      // round are fetched while this round's frontier rows are in flight, so
-      // a round costs one memory latency, not two.
-      constexpr int NI = LPV >= CH ? 1 : CH;  // ids held per lane
-      uint32_t ids[NI];
-#pragma unroll
-      for (int j = 0; j < NI; ++j) {
-        const uint32_t e = beg + gid * CH + (LPV >= CH ? lig : j);
-        ids[j] = ((LPV < CH || lig < CH) && e < end) ? __ldg(in_idx + e) : FULL;
+      for (int q = 0; q < VEC; ++q) {
+        needed.w[q] = ~needed.w[q] & lmask.w[q];
+        if (!whole) sat &= (hc.w[q] & needed.w[q]) == needed.w[q];
+        hc.w[q] = 0;
       }
-      for (uint32_t base = beg; base < end; base += GPW * CH) {
-        const uint32_t e0 = base + gid * CH;
-        if (lig == 0 && e0 < end) cnt.edges += min((uint32_t)CH, end - e0);
-        uint32_t u[CH];
-        if constexpr (LPV >= CH) {
-          const uint32_t mine = gather_id(p, fb, ids[0]);
-#pragma unroll
-          for (int j = 0; j < CH; ++j) u[j] = __shfl_sync(FULL, mine, gbase + j);
-        } else {
-#pragma unroll
-          for (int j = 0; j < CH; ++j) u[j] = gather_id(p, fb, ids[j]);
-        }
+      // Every slice of v sees the same `needed` (only the committing slice
+      // writes v's visited row, after all slices arrived).
+      if (!__any_sync(FULL, any_bits<VEC>(needed))) {
+        if (lane == 0) atomicAnd(&p.hlive[ci >> 5], ~(1u << (ci & 31)));
+        continue;
+      }
+      if ((sl.w & SLICE_FIRST) && lane == 0) cnt.active += 1;
+      if (!__all_sync(FULL, sat)) {
+        // Each round the warp gathers GPW*CH in-neighbours; the ids of the next
+        // round are fetched while this round's frontier rows are in flight, so
+        // a round costs one memory latency, not two. Whether the rows cover
+        // the needed lanes is looked at after rounds 1, 2 and every 4th (the
+        // look is 3 shuffles a word).
+        uint32_t ids[NI];
 #pragma unroll
         for (int j = 0; j < NI; ++j) {
-          const uint32_t e = e0 + GPW * CH + (LPV >= CH ? lig : j);
+          const uint32_t e = beg + gid * CH + (LPV >= CH ? lig : j);
           ids[j] = ((LPV < CH || lig < CH) && e < end) ? __ldg(in_idx + e) : FULL;
         }
+        uint32_t round = 0;
+        for (uint32_t base = beg; base < end; base += GPW * CH, ++round) {
+          const uint32_t e0 = base + gid * CH;
+          if (lig == 0 && e0 < end) cnt.edges += min((uint32_t)CH, end - e0);
+          uint32_t u[CH];
+          if constexpr (LPV >= CH) {
+            const uint32_t mine_id = gather_id(p, fb, ids[0]);
 #pragma unroll
-        for (int j = 0; j < CH; ++j) {
-          if (u[j] != FULL) {
-            cnt.rows += 1;
-            Words<VEC> f = gather_words<VEC>(Fin + (size_t)u[j] * W + k0);
+            for (int j = 0; j < CH; ++j) u[j] = __shfl_sync(FULL, mine_id, gbase + j);
+          } else {
 #pragma unroll
-            for (int q = 0; q < VEC; ++q) hc.w[q] |= f.w[q];
+            for (int j = 0; j < CH; ++j) u[j] = gather_id(p, fb, ids[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < NI; ++j) {
+            const uint32_t e = e0 + GPW * CH + (LPV >= CH ? lig : j);
+            ids[j] = ((LPV < CH || lig < CH) && e < end) ? __ldg(in_idx + e) : FULL;
+          }
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            if (u[j] != FULL) {
+              cnt.rows += 1;
+              Words<VEC> f = ldca_words<VEC>(Fin + (size_t)u[j] * W + k0);
+#pragma unroll
+              for (int q = 0; q < VEC; ++q) hc.w[q] |= f.w[q];
+            }
+          }
+          if (round < 2 || (round & 3) == 3) {
+            bool s2 = true;
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) {
+              uint32_t c = hc.w[q];
+#pragma unroll
+              for (int o = LPV; o < 32; o <<= 1) c |= __shfl_xor_sync(FULL, c, o);
+              hc.w[q] = c;
+              s2 &= (c & needed.w[q]) == needed.w[q];
+            }
+            if (__all_sync(FULL, s2)) break;
           }
         }
-        bool s2 = true;
 #pragma unroll
         for (int q = 0; q < VEC; ++q) {
-          uint32_t c = hc.w[q];
 #pragma unroll
-          for (int o = LPV; o < 32; o <<= 1) c |= __shfl_xor_sync(FULL, c, o);
-          hc.w[q] = c;
-          s2 &= (c & needed.w[q]) == needed.w[q];
+          for (int o = LPV; o < 32; o <<= 1) hc.w[q] |= __shfl_xor_sync(FULL, hc.w[q], o);
+          hc.w[q] &= needed.w[q];
         }
-        if (__all_sync(FULL, s2)) break;
+        if (!whole && gid == 0) {
+#pragma unroll
+          for (int q = 0; q < VEC; ++q)
+            if (hc.w[q]) atomicOr(hrow + q, hc.w[q]);
+        }
+      }
+      if (!whole) {
+        __threadfence();
+        uint32_t last = 0;
+        if (lane == 0) last = (atomicAdd(p.hcount + h, 1u) == __ldg(p.hslices + h) - 1) ? 1u : 0u;
+        last = __shfl_sync(FULL, last, 0);
+        if (!last) continue;
+        __threadfence();
+        hc = ldcg_words<VEC>(hrow);
+        __syncwarp();
+        if (gid == 0) {
+          Words<VEC> zero;
+#pragma unroll
+          for (int q = 0; q < VEC; ++q) {
+            hc.w[q] &= needed.w[q];
+            zero.w[q] = 0;
+          }
+          st_words<VEC>(hrow, zero);
+        }
+        if (lane == 0) p.hcount[h] = 0;
       }
       if (gid == 0) {
-#pragma unroll
-        for (int q = 0; q < VEC; ++q)
-          if (hc.w[q] & needed.w[q]) atomicOr(hrow + q, hc.w[q] & needed.w[q]);
+        const bool any_new = (__ballot_sync(gmask, any_bits<VEC>(hc)) & gmask) != 0;
+        if (any_new) pull_commit<W, VEC>(p, s_lanes, L, v, k0, lig, hc, cnt);
       }
     }
-    __threadfence();
-    uint32_t last = 0;
-    if (lane == 0) last = (atomicAdd(p.hcount + hk.h, 1u) == hk.nch - 1) ? 1u : 0u;
-    last = __shfl_sync(FULL, last, 0);
-    if (last) {
-      __threadfence();
-      if (gid == 0) {
-        const Words<VEC> fin = ldcg_words<VEC>(hrow);
-        Words<VEC> newly, zero;
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-          newly.w[q] = fin.w[q] & needed.w[q];
-          zero.w[q] = 0;
-        }
-        st_words<VEC>(hrow, zero);
-        const bool any_new = (__ballot_sync(gmask, any_bits<VEC>(newly)) & gmask) != 0;
-        if (any_new) pull_commit<W, VEC>(p, bq, s_lanes, L, v, k0, lig, newly, cnt);
-        if (lane == 0) p.hcount[hk.h] = 0;
-      }
-    }
-   }
   }
 
   // ---- (2) all other vertices with in-edges, in the graph's work order
   // (ascending ids: neighbouring vertices share cache lines of the visited
-  // and frontier rows), so vertices without in-edges cost nothing. Tiles are
-  // claimed dynamically: work concentrates at some ids (R-MAT puts its hubs
-  // first) and a static split would leave most warps idle behind a few.
+  // and frontier rows), so vertices without in-edges cost nothing. Their
+  // lists are short, so tiles are dealt out in turn; where a warp gets more
+  // than a few, the second half is claimed as warps get done, from
+  // WORK_STRIPES cursors. All tiles by claims / all in turn / half and half,
+  // us: R-MAT 22 S=512 level 2 1,388 / 1,516 / 1,422, level 5 (few vertices
+  // left) 163 / 127 / 138; R-MAT 20 S=1 level 4 41 / 27 / 27 (a claim is an
+  // atomic round trip).
   const uint32_t ntiles = (p.n_order + GPW - 1) / GPW;
-  const uint32_t per_stripe = (ntiles + WORK_STRIPES - 1) / WORK_STRIPES;
-  uint32_t stripe = warp_g % WORK_STRIPES, exhausted = 0;
-  uint32_t tile = 0, tile_end = 0;
+  const uint32_t turn = ntiles > TURN_TILES * nwarps ? ntiles / 2 : ntiles;
+  const uint32_t per_stripe = (ntiles - turn + WORK_STRIPES - 1) / WORK_STRIPES;
+  uint32_t stripe = warp_g % WORK_STRIPES;
+  uint32_t tile = warp_g, tile_end = turn, step = nwarps;
   [[maybe_unused]] uint32_t guard = 0;
   for (;;) {
     LOOP_GUARD(guard, ntiles + 2 * WORK_STRIPES + 2, CK_TILE_LOOP)
-    if (tile == tile_end) {
-      // Claim from the warp's stripe; move to the next once it runs dry.
-      while (exhausted < WORK_STRIPES) {
-        const uint32_t sb = stripe * per_stripe, se = min(sb + per_stripe, ntiles);
-        uint32_t t0 = 0;
-        if (lane == 0) t0 = sb < se ? sb + atomicAdd(&p.ctl->work[stripe][0], TILE_BATCH) : se;
+    if (tile >= tile_end) {
+      // Claim from the warp's stripe; once it runs dry, from the next one
+      // that a look at all cursors at once (a lane each) finds tiles in.
+      uint32_t left = turn < ntiles;
+      while (left) {
+        const uint32_t sb = turn + stripe * per_stripe, se = min(sb + per_stripe, ntiles);
+        uint32_t t0 = se;
+        if (lane == 0 && sb < se) t0 = sb + atomicAdd(&p.ctl->work[stripe][0], TILE_BATCH);
         t0 = __shfl_sync(FULL, t0, 0);
         if (t0 < se) {
           tile = t0;
           tile_end = min(t0 + TILE_BATCH, se);
+          step = 1;
           break;
         }
-        ++exhausted;
-        stripe = (stripe + 1) % WORK_STRIPES;
+        const uint32_t cs = (stripe + 1 + lane) % WORK_STRIPES;  // lanes 0..15: nearest first
+        const uint32_t cb = turn + cs * per_stripe, ce = min(cb + per_stripe, ntiles);
+        left = __ballot_sync(FULL, lane < WORK_STRIPES && cb < ce &&
+                                       cb + __ldcg(&p.ctl->work[cs][0]) < ce);
+        if (left) stripe = (stripe + __ffs(left)) % WORK_STRIPES;
       }
-      if (tile == tile_end) break;  // every stripe is done
+      if (tile >= tile_end) break;  // every stripe is done
     }
     const uint32_t oi = tile * GPW + gid;
-    ++tile;
+    tile += step;
     uint32_t v = 0, beg = 0, end = 0;
     if (oi < p.n_order) {
       const uint4 ent = __ldg(p.order + oi);
@@ -606,13 +621,11 @@ __device__ void pull_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lan
       for (int j = 0; j < VEC; ++j) needed.w[j] = ~visw.w[j] & lmask.w[j];
     }
     const bool need = (__ballot_sync(FULL, any_bits<VEC>(needed)) & gmask) != 0;
-    const bool heavy = need && (end - beg) >= p.heavy;
     if (lig == 0 && need) cnt.active += 1;
 
-    if (need && !heavy) {
+    if (need) {
       // The next chunk's in-neighbour ids are fetched while the current
       // chunk's frontier rows are in flight.
-      constexpr int NI = LPV >= CH ? 1 : CH;  // ids held per lane
       uint32_t ids[NI];
       bool lane_sat = !any_bits<VEC>(needed);
 #pragma unroll
@@ -642,7 +655,7 @@ __device__ void pull_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lan
         for (int j = 0; j < CH; ++j) {
           if (!lane_sat && u[j] != FULL) {
             cnt.rows += 1;
-            f[j] = gather_words<VEC>(Fin + (size_t)u[j] * W + k0);
+            f[j] = ldca_words<VEC>(Fin + (size_t)u[j] * W + k0);
           } else {
 #pragma unroll
             for (int q = 0; q < VEC; ++q) f[j].w[q] = 0;
@@ -662,70 +675,11 @@ __device__ void pull_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lan
       }
     }
 
-    uint32_t hmask = __ballot_sync(FULL, heavy && lig == 0);
-    while (hmask) {
-      const uint32_t hl = __ffs(hmask) - 1;
-      hmask &= hmask - 1;
-      const uint32_t hbeg = __shfl_sync(FULL, beg, hl);
-      const uint32_t hend = __shfl_sync(FULL, end, hl);
-      Words<VEC> hneed, hc;
-#pragma unroll
-      for (int q = 0; q < VEC; ++q) {
-        hneed.w[q] = __shfl_sync(FULL, needed.w[q], hl + lig);
-        hc.w[q] = 0;
-      }
-      constexpr int NI = LPV >= CH ? 1 : CH;  // ids held per lane (next round)
-      uint32_t ids[NI];
-#pragma unroll
-      for (int j = 0; j < NI; ++j) {
-        const uint32_t e = hbeg + gid * CH + (LPV >= CH ? lig : j);
-        ids[j] = ((LPV < CH || lig < CH) && e < hend) ? __ldg(in_idx + e) : FULL;
-      }
-      for (uint32_t base = hbeg; base < hend; base += GPW * CH) {
-        const uint32_t e0 = base + gid * CH;
-        if (lig == 0 && e0 < hend) cnt.edges += min((uint32_t)CH, hend - e0);
-        uint32_t u[CH];
-        if constexpr (LPV >= CH) {
-          const uint32_t mine = gather_id(p, fb, ids[0]);
-#pragma unroll
-          for (int j = 0; j < CH; ++j) u[j] = __shfl_sync(FULL, mine, gbase + j);
-        } else {
-#pragma unroll
-          for (int j = 0; j < CH; ++j) u[j] = gather_id(p, fb, ids[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < NI; ++j) {
-          const uint32_t e = e0 + GPW * CH + (LPV >= CH ? lig : j);
-          ids[j] = ((LPV < CH || lig < CH) && e < hend) ? __ldg(in_idx + e) : FULL;
-        }
-#pragma unroll
-        for (int j = 0; j < CH; ++j) {
-          if (u[j] != FULL) {
-            cnt.rows += 1;
-            Words<VEC> f = gather_words<VEC>(Fin + (size_t)u[j] * W + k0);
-#pragma unroll
-            for (int q = 0; q < VEC; ++q) hc.w[q] |= f.w[q];
-          }
-        }
-        bool sat = true;
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-          uint32_t c = hc.w[q];
-#pragma unroll
-          for (int o = LPV; o < 32; o <<= 1) c |= __shfl_xor_sync(FULL, c, o);
-          hc.w[q] = c;
-          sat &= (c & hneed.w[q]) == hneed.w[q];
-        }
-        if (__all_sync(FULL, sat)) break;
-      }
-      if (gbase == hl) cand = hc;
-    }
-
     Words<VEC> newly;
 #pragma unroll
     for (int q = 0; q < VEC; ++q) newly.w[q] = cand.w[q] & needed.w[q];
     const bool any_new = (__ballot_sync(FULL, any_bits<VEC>(newly)) & gmask) != 0;
-    if (any_new) pull_commit<W, VEC>(p, bq, s_lanes, L, v, k0, lig, newly, cnt);
+    if (any_new) pull_commit<W, VEC>(p, s_lanes, L, v, k0, lig, newly, cnt);
   }
 }
 
@@ -735,7 +689,7 @@ __device__ void pull_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lan
 // frontier vertices share a hub) are merged into one atomicOr by the first
 // of them, which then owns the follow-up writes for that word.
 template <int W>
-__device__ void push_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lanes, uint32_t L,
+__device__ __forceinline__ void push_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lanes, uint32_t L,
                            LevelCounters& cnt) {
   using G = Geo<W>;
   constexpr int VEC = G::VEC, LPV = G::LPV, GPW = G::GPW;
@@ -749,22 +703,32 @@ __device__ void push_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lan
   // The sources' queue (level 0) uses shorter entries: a few hundred
   // sources would otherwise leave most groups idle behind long edge walks.
   const uint32_t seg = L == 0 ? p.seg0 : p.seg;
-  const uint32_t* __restrict__ Fin = p.F[si];
-  uint32_t* __restrict__ Fout = p.F[so];
-  const unsigned long long* __restrict__ Qi = p.Q[si];
-  const uint32_t nin = *(volatile uint32_t*)&p.ctl->qcount[si];
+  const uint32_t* Fin = p.F[si];
+  uint32_t* Fout = p.F[so];
+  const unsigned long long* Qi = p.Q[si];
+  const uint32_t nin = __ldcg(&p.ctl->qcount[si]);
   const uint32_t group_g = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * GPW + lane / LPV;
   const uint32_t ngroups = ((gridDim.x * blockDim.x) >> 5) * GPW;
+  // With fewer entries than groups, `parts` groups share an entry's edges: a
+  // group walks its edges one after the other, a dependent chain of several
+  // microseconds each (R-MAT 20, one source: level 1, 25 entries of up to 64
+  // edges, 357 us with a group per entry).
+  uint32_t pshift = 0;
+  while (nin && (2u << pshift) <= seg && ((unsigned long long)nin << (pshift + 1)) <= ngroups)
+    ++pshift;
+  const uint32_t part_len = (seg + (1u << pshift) - 1) >> pshift;
+  const uint32_t nparts = nin << pshift;  // pshift > 0 only while this is <= ngroups
 
-  for (uint32_t i = group_g; i < nin; i += ngroups) {
-    const unsigned long long ent = Qi[i];
+  for (uint32_t i = group_g; i < nparts; i += ngroups) {
+    const unsigned long long ent = __ldcg(Qi + (i >> pshift));
     const uint32_t u = (uint32_t)ent;
     const uint32_t sg = (uint32_t)(ent >> 32);
     if (!BCHECK(u < p.V, CK_PUSH_ENTRY)) continue;
-    const Words<VEC> f = ldg_words<VEC>(Fin + (size_t)u * W + k0);
+    const Words<VEC> f = ldca_words<VEC>(Fin + (size_t)u * W + k0);
     const uint32_t ob = __ldg(p.out_off + u), oe = __ldg(p.out_off + u + 1);
-    const uint32_t eb = ob + sg * seg;
-    const uint32_t ee = min(oe, eb + seg);
+    const uint32_t pe = (i & ((1u << pshift) - 1)) * part_len;
+    const uint32_t eb = min(oe, ob + sg * seg + pe);
+    const uint32_t ee = min(oe, eb + min(part_len, seg - pe));
     if (lig == 0) cnt.edges += ee - eb;
     // The next edge's target and its visited words are fetched while this
     // edge is processed. A stale visited word only widens `needed`; the
@@ -807,7 +771,8 @@ __device__ void push_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lan
         }
       }
       if (__ballot_sync(gmask, found) != 0 && lane == gbase) {
-        if (__ldcg(p.stamp + v) != d && atomicExch(p.stamp + v, d) != d) {
+        const uint32_t st = p.epoch + d;
+        if (__ldcg(p.stamp + v) != st && atomicExch(p.stamp + v, st) != st) {
           atomicOr(p.fbits[so] + (v >> 5), 1u << (v & 31));
           bq_push(p, bq, so, v);
           cnt.newv += 1;
@@ -817,52 +782,56 @@ __device__ void push_phase(const LevelParams& p, BlockQueue& bq, uint32_t* s_lan
   }
 }
 
-// Device-side level controller, run by the last block of each level.
-__device__ void controller(const LevelParams& p, cudaGraphConditionalHandle h, uint32_t L,
-                           uint32_t dir) {
-  volatile LevelCtl* c = p.ctl;
-  const uint32_t so = (L + 1) % 3;
-  const uint32_t n_next = c->qverts[so];
-  const unsigned long long m_next = c->qedges[so];
-  if (L < LOG_CAP) {
-    LevelRec r;
-    r.level = L;
-    r.dir = dir;
-    r.frontier_vertices = c->qverts[L % 3];
-    r.frontier_entries = c->qcount[L % 3];
-    r.active = c->c_active;
-    r.edges = c->c_edges;
-    r.new_vertices = c->c_newv;
-    r.new_pairs = c->c_pairs;
-    r.rows = c->c_rows / (p.W >= 4 ? p.W / 4 : 1);  // counted per 16-byte piece
-    r.t_start = c->t_start;
-    r.t_end = globaltimer();
-    p.log[L] = r;
+// Whether bottom-up steps test the frontier bitmap before they load a row.
+__device__ __forceinline__ uint32_t frontier_is_sparse(const LevelParams& p, uint32_t nverts) {
+  return (p.bits_div && (unsigned long long)nverts * p.bits_div < p.V) ? 1u : 0u;
+}
+
+// Device-side level controller, run by one warp of the last block to finish a
+// level. `log`: also write the level's record.
+static __device__ void controller(const LevelParams& p, uint32_t L, uint32_t dir, bool log) {
+  LevelCtl* c = p.ctl;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t so = (L + 1) % 3, sc = (L + 2) % 3;
+  const uint32_t n_next = __ldcg(&c->qverts[so]);
+  const unsigned long long m_next = __ldcg(&c->qedges[so]);
+  if (log && lane == 0) {
+    if (L < LOG_CAP) {
+      LevelRec r;
+      r.level = L;
+      r.dir = dir;
+      r.frontier_vertices = __ldcg(&c->qverts[L % 3]);
+      r.frontier_entries = __ldcg(&c->qcount[L % 3]);
+      r.active = __ldcg(&c->c_active);
+      r.edges = __ldcg(&c->c_edges);
+      r.new_vertices = __ldcg(&c->c_newv);
+      r.new_pairs = __ldcg(&c->c_pairs);
+      r.rows = __ldcg(&c->c_rows) / (p.W >= 4 ? p.W / 4 : 1);  // counted per 16-byte piece
+      r.t_start = __ldcg(&c->t_start);
+      r.t_end = globaltimer();
+      p.log[L] = r;
+    }
+    c->c_active = 0;
+    c->c_edges = 0;
+    c->c_newv = 0;
+    c->c_pairs = 0;
+    c->c_rows = 0;
+    c->t_start = ~0ull;
   }
-  c->c_active = 0;
-  c->c_edges = 0;
-  c->c_newv = 0;
-  c->c_pairs = 0;
-  c->c_rows = 0;
-  c->t_start = ~0ull;
-  if (dir == DIR_PUSH)
-    c->push_levels = c->push_levels + 1;
-  else
-    c->pull_levels = c->pull_levels + 1;
-  bool stop = false;
-  if (n_next == 0) {
-    stop = true;
-  } else if (L + 1 >= p.max_levels) {
-    c->status = c->status | STATUS_LEVEL_CAP;
-    stop = true;
+  if (lane == 0) {
+    if (dir == DIR_PUSH)
+      c->push_levels += 1;
+    else
+      c->pull_levels += 1;
   }
-  if (stop) {
-    c->terminated = 1;
-    if (h) cudaGraphSetConditional(h, 0);
+  const bool capped = n_next != 0 && L + 1 >= p.max_levels;
+  if (n_next == 0 || capped) {
+    if (lane == 0) {
+      if (capped) atomicOr(&c->status, STATUS_LEVEL_CAP);
+      c->terminated = 1;
+    }
     return;
   }
-  const unsigned long long explored = c->explored + c->qedges[L % 3];
-  c->explored = explored;
   uint32_t nd = dir;
   if (p.mode == MODE_PUSH) {
     nd = DIR_PUSH;
@@ -877,136 +846,81 @@ __device__ void controller(const LevelParams& p, cudaGraphConditionalHandle h, u
     // Back to top-down once the frontier holds fewer than V / beta vertices.
     if ((unsigned long long)n_next * p.beta < p.V) nd = DIR_PUSH;
   }
-  for (uint32_t k = 0; k < p.W; ++k) c->lanes[L & 1][k] = 0;  // becomes level L+2's collector
-  const uint32_t sc = (L + 2) % 3;  // slot of level L-1, becomes level L+2
-  c->qcount[sc] = 0;
-  c->qverts[sc] = 0;
-  c->qedges[sc] = 0;
-  c->dir = nd;
-  c->level = L + 1;
-  c->done_blocks = 0;
-  for (uint32_t k = 0; k < WORK_STRIPES; ++k) c->work[k][0] = 0;
-  c->use_bits = (p.bits_div && (unsigned long long)n_next * p.bits_div < p.V) ? 1u : 0u;
-  __threadfence();
-  if (h) cudaGraphSetConditional(h, 1);
+  for (uint32_t k = lane; k < p.W; k += 32) c->lanes[L & 1][k] = 0;  // becomes level L+2's collector
+  if (lane < WORK_STRIPES) c->work[lane][0] = 0;
+  if (lane == 0) {
+    // slot of level L-1, becomes level L+2
+    c->qcount[sc] = 0;
+    c->qverts[sc] = 0;
+    c->qedges[sc] = 0;
+    c->dir = nd;
+    if (dir == DIR_PULL && nd == DIR_PUSH) {
+      c->build_queue = 1;
+      c->qverts[so] = 0;  // counted again with the queue
+    }
+    c->level = L + 1;
+    c->use_bits = frontier_is_sparse(p, n_next);
+  }
 }
 
-// Zeroes the frontier words of the n entries of queue slot `sl` (entries
-// with a non-zero segment repeat a vertex, so only segment 0 clears).
+// Zeroes the frontier rows of slot `sl` and its membership bitmap: a warp
+// loads up to 32 bitmap words, fewer when they would leave warps idle, and
+// clears the 32 rows of each word with members in coalesced stores.
 template <int W>
-__device__ __forceinline__ void clear_frontier_rows(const LevelParams& p, uint32_t sl, uint32_t n,
-                                                    size_t t0, size_t nthreads) {
-  const unsigned long long* Q = p.Q[sl];
-  uint32_t* F = p.F[sl];
-  const size_t total = (size_t)n * W;
-  for (size_t i = t0; i < total; i += nthreads) {
-    const unsigned long long ent = Q[i / W];
-    if ((ent >> 32) == 0 && BCHECK((uint32_t)ent < p.V, CK_CLEAR_ENTRY))
-      F[(size_t)(uint32_t)ent * W + i % W] = 0;
+__device__ __forceinline__ void clear_frontier(const LevelParams& p, uint32_t sl) {
+  constexpr int VEC = Geo<W>::VEC, LPV = Geo<W>::LPV, GPW = Geo<W>::GPW;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t words = (p.V + 31) / 32;
+  const uint32_t per = min((words + nwarps - 1) / nwarps, 32u);
+  uint32_t* bits = p.fbits[sl];
+  Words<VEC> zero;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) zero.w[j] = 0;
+  for (uint32_t wb = warp_g * per; wb < words; wb += nwarps * per) {
+    const uint32_t x = lane < per && wb + lane < words ? __ldcg(bits + wb + lane) : 0u;
+    uint32_t todo = __ballot_sync(FULL, x != 0);
+    if (x) bits[wb + lane] = 0;
+    while (todo) {
+      const uint32_t l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t m = __shfl_sync(FULL, x, l);
+      uint32_t* row = p.F[sl] + (size_t)(wb + l) * 32 * W + (lane % LPV) * VEC;
+#pragma unroll
+      for (uint32_t b = lane / LPV; b < 32; b += GPW)
+        if ((m >> b) & 1u) st_words<VEC>(row + (size_t)b * W, zero);
+    }
   }
 }
 
-// One level of the traversal, bottom-up (DIR_PULL) or top-down (DIR_PUSH):
-// the two directions are separate kernels, each with its own register
-// budget, and both sit in the level loop's body -- the pull kernel first --
-// so the one whose direction the control block does not name returns at
-// once. When a pull level's controller turns the traversal top-down, the
-// push kernel of the same body iteration runs the next level. COUNT keeps
-// the per-level work counters of the profiling log (the production form
-// compiles them out; the discovered-pair count is always kept).
-#ifndef MSBFS_PUSH_MIN_BLOCKS
-#define MSBFS_PUSH_MIN_BLOCKS MSBFS_LEVEL_MIN_BLOCKS
-#endif
-template <int W, uint32_t DIR, bool COUNT>
-__global__ void __launch_bounds__(LEVEL_BLOCK, DIR == DIR_PULL ? MSBFS_LEVEL_MIN_BLOCKS
-                                                               : MSBFS_PUSH_MIN_BLOCKS)
-    level_kernel(LevelParams p, cudaGraphConditionalHandle h) {
-  __shared__ BlockQueue bq;
-  __shared__ unsigned long long s_red[5][LEVEL_BLOCK / 32];
-  __shared__ uint32_t s_lanes[W];
-  __shared__ uint32_t s_alive[W];
-  __shared__ uint32_t s_last;
-  volatile LevelCtl* c = p.ctl;
-  // Speculative launches of the host-driven loop, and the kernel of the
-  // other direction in the loop body, return here.
-  if (c->terminated || c->dir != DIR) return;
-  const uint32_t L = c->level;
-  if (threadIdx.x == 0) {
-    bq.count = 0;
-    atomicMin(&p.ctl->t_start, globaltimer());
-  }
-  if constexpr (DIR == DIR_PULL) {
-    const uint32_t P = p.desc->num_sources;
-    for (uint32_t k = threadIdx.x; k < W; k += blockDim.x)
-      s_alive[k] = lane_word_mask(P, k) & c->lanes[L & 1][k];
-  }
-  for (uint32_t k = threadIdx.x; k < W; k += blockDim.x) s_lanes[k] = 0;
+// Fills the queue of slot `sl` from its membership bitmap, for a top-down step
+// after a bottom-up one (which keeps no queue).
+template <int W>
+__device__ __forceinline__ void build_queue(const LevelParams& p, BlockQueue& bq, uint32_t sl) {
+  if (threadIdx.x == 0) bq.count = 0;
   __syncthreads();
-
-  // Clear the frontier words of level L-1 (not read or written this level).
-  {
-    const uint32_t sc = (L + 2) % 3;
-    clear_frontier_rows<W>(p, sc, c->qcount[sc], blockIdx.x * (size_t)blockDim.x + threadIdx.x,
-                           (size_t)gridDim.x * blockDim.x);
-    uint32_t* fc = p.fbits[sc];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (p.V + 31) / 32;
-         i += gridDim.x * blockDim.x)
-      fc[i] = 0;
-  }
-
-  LevelCounters cnt;
-  if constexpr (DIR == DIR_PULL)
-    pull_phase<W>(p, bq, s_lanes, s_alive, L, cnt);
-  else
-    push_phase<W>(p, bq, s_lanes, L, cnt);
-  flush_block_queue(p, bq, (L + 1) % 3);  // starts with a block barrier
-  for (uint32_t k = threadIdx.x; k < W; k += blockDim.x)
-    if (s_lanes[k]) atomicOr(&p.ctl->lanes[(L + 1) & 1][k], s_lanes[k]);
-
-  unsigned long long vals[5] = {cnt.active, cnt.edges, cnt.newv, cnt.pairs, cnt.rows};
-  if constexpr (!COUNT) vals[0] = vals[1] = vals[2] = vals[4] = 0;
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    if (!COUNT && i != 3) continue;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) vals[i] += __shfl_xor_sync(FULL, vals[i], o);
-    if ((threadIdx.x & 31) == 0) s_red[i][threadIdx.x >> 5] = vals[i];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long tot[5] = {0, 0, 0, 0, 0};
-    for (int i = 0; i < 5; ++i) {
-      if (!COUNT && i != 3) continue;
-      for (int w = 0; w < LEVEL_BLOCK / 32; ++w) tot[i] += s_red[i][w];
-    }
-    if (tot[0]) atomicAdd(&p.ctl->c_active, tot[0]);
-    if (tot[1]) atomicAdd(&p.ctl->c_edges, tot[1]);
-    if (tot[2]) atomicAdd(&p.ctl->c_newv, tot[2]);
-    if (tot[4]) atomicAdd(&p.ctl->c_rows, tot[4]);
-    if (tot[3]) {
-      atomicAdd(&p.ctl->c_pairs, tot[3]);
-      atomicAdd(&p.ctl->pairs, tot[3]);
-    }
-    __threadfence();
-    const uint32_t prev = atomicAdd(&p.ctl->done_blocks, 1u);
-    s_last = (prev == gridDim.x - 1);
-    if (s_last) {
-      __threadfence();
-      controller(p, h, L, DIR);
+  const uint32_t words = (p.V + 31) / 32;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) {
+    uint32_t x = __ldcg(p.fbits[sl] + i);
+    while (x) {
+      const uint32_t b = __ffs(x) - 1;
+      x &= x - 1;
+      bq_push(p, bq, sl, i * 32 + b);
     }
   }
+  flush_block_queue(p, bq, sl);
 }
 
 // Level-0 frontier: lane i of word i/32 at vertex sources[i]. Duplicate
 // sources share a vertex and are merged by atomicOr; the vertex is enqueued
-// once (stamp 0).
+// once (the stamp). Run by one block on a zeroed control block.
 template <int W>
-__global__ void init_kernel(LevelParams p) {
-  const PassDesc* dsc = p.desc;
-  const uint32_t P = dsc->num_sources;
-  unsigned long long ok = 0;
+__device__ __forceinline__ void init_sources(const LevelParams& p) {
+  const uint32_t P = p.d.num_sources;
+  uint32_t ok = 0;
   for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
-    const uint32_t s = dsc->sources[i];
+    const uint32_t s = p.d.sources[i];
     if (s >= p.V) {
       atomicOr(&p.ctl->status, STATUS_BAD_SOURCE);
       continue;
@@ -1017,14 +931,233 @@ __global__ void init_kernel(LevelParams p) {
     atomicOr(p.F[0] + w, bit);
     atomicOr(&p.ctl->lanes[0][i >> 5], bit);
     atomicOr(p.fbits[0] + (s >> 5), 1u << (s & 31));
-    if (atomicExch(p.stamp + s, 0u) != 0u) enqueue_global(p, 0, s, p.seg0);
+    if (atomicExch(p.stamp + s, p.epoch) != p.epoch) enqueue_global(p, 0, s, p.seg0);
     ++ok;
   }
-  if (ok) atomicAdd(&p.ctl->pairs, ok);
+  if (ok) atomicAdd(&p.ctl->pairs, (unsigned long long)ok);
   if (threadIdx.x == 0) {
     p.ctl->dir = (p.mode == MODE_PULL) ? DIR_PULL : DIR_PUSH;
+    p.ctl->use_bits = frontier_is_sparse(p, P);
     p.ctl->t_start = ~0ull;
   }
+}
+
+template <int W>
+__global__ void init_kernel(const __grid_constant__ LevelParams p) {
+  init_sources<W>(p);
+}
+
+#ifndef MSBFS_PUSH_MIN_BLOCKS
+#define MSBFS_PUSH_MIN_BLOCKS MSBFS_LEVEL_MIN_BLOCKS
+#endif
+
+// Per-block working storage of a level.
+template <int W>
+struct LevelShared {
+  BlockQueue bq;
+  unsigned long long red[5][LEVEL_BLOCK / 32];
+  uint32_t lanes[W];
+  uint32_t alive[W];
+  uint32_t flag;
+};
+
+// One level, this block's share: clears the frontier rows and bitmap of level
+// L-1 (not read or written this level), runs the bottom-up or top-down step,
+// appends the block's discoveries to the next queue and adds its counts to
+// the control block. Starts and ends with the block's threads in step.
+template <int W, uint32_t DIR, bool COUNT>
+__device__ __forceinline__ void run_level(const LevelParams& p, LevelShared<W>& sh, uint32_t L) {
+  LevelCtl* c = p.ctl;
+  if (threadIdx.x == 0) sh.bq.count = 0;
+  if constexpr (DIR == DIR_PULL) {
+    const uint32_t P = p.d.num_sources;
+    for (uint32_t k = threadIdx.x; k < W; k += blockDim.x)
+      sh.alive[k] = lane_word_mask(P, k) & __ldcg(&c->lanes[L & 1][k]);
+  }
+  for (uint32_t k = threadIdx.x; k < W; k += blockDim.x) sh.lanes[k] = 0;
+  clear_frontier<W>(p, (L + 2) % 3);
+  __syncthreads();
+
+  LevelCounters cnt;
+  if constexpr (DIR == DIR_PULL) {
+    pull_phase<W>(p, sh.lanes, sh.alive, L, cnt);
+    __syncthreads();
+  } else {
+    push_phase<W>(p, sh.bq, sh.lanes, L, cnt);
+    flush_block_queue(p, sh.bq, (L + 1) % 3);  // starts with a block barrier
+  }
+  for (uint32_t k = threadIdx.x; k < W; k += blockDim.x)
+    if (sh.lanes[k]) atomicOr(&c->lanes[(L + 1) & 1][k], sh.lanes[k]);
+
+  // Bottom-up steps count the new frontier's vertices here, top-down ones
+  // with the queue.
+  constexpr bool NEWV = COUNT || DIR == DIR_PULL;
+  unsigned long long vals[5] = {cnt.active, cnt.edges, cnt.newv, cnt.pairs, cnt.rows};
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    if (!COUNT && i != 3 && !(i == 2 && NEWV)) continue;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vals[i] += __shfl_xor_sync(FULL, vals[i], o);
+    if ((threadIdx.x & 31) == 0) sh.red[i][threadIdx.x >> 5] = vals[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < 5) {
+    const uint32_t i = threadIdx.x;
+    unsigned long long tot = 0;
+    if (COUNT || i == 3 || (i == 2 && NEWV))
+      for (int w = 0; w < LEVEL_BLOCK / 32; ++w) tot += sh.red[i][w];
+    if (tot) {
+      if (i == 3) atomicAdd(&c->pairs, tot);
+      if (i == 2 && DIR == DIR_PULL) atomicAdd(&c->qverts[(L + 1) % 3], (uint32_t)tot);
+      if constexpr (COUNT)
+        atomicAdd(i == 0   ? &c->c_active
+                  : i == 1 ? &c->c_edges
+                  : i == 2 ? &c->c_newv
+                  : i == 3 ? &c->c_pairs
+                           : &c->c_rows,
+                  tot);
+    }
+  }
+}
+
+// One level as a launch of its own, for the host-driven loop (profiling,
+// devices without cooperative launches): the two directions are separate
+// kernels and the one whose direction the control block does not name
+// returns at once. COUNT keeps the per-level work counters of the profiling
+// log (the production form compiles them out; the discovered-pair count is
+// always kept).
+template <int W, uint32_t DIR, bool COUNT>
+__global__ void __launch_bounds__(LEVEL_BLOCK, DIR == DIR_PULL ? MSBFS_LEVEL_MIN_BLOCKS
+                                                               : MSBFS_PUSH_MIN_BLOCKS)
+    level_kernel(const __grid_constant__ LevelParams p) {
+  __shared__ LevelShared<W> sh;
+  volatile LevelCtl* c = p.ctl;
+  // Speculative launches past the last level, and the other direction's.
+  if (c->terminated || c->dir != DIR || (DIR == DIR_PUSH && c->build_queue)) return;
+  const uint32_t L = c->level;
+  if (COUNT && threadIdx.x == 0) atomicMin(&p.ctl->t_start, globaltimer());
+  run_level<W, DIR, COUNT>(p, sh, L);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    sh.flag = atomicAdd(&p.ctl->done_blocks, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (sh.flag && threadIdx.x < 32) {
+    __threadfence();
+    controller(p, L, DIR, true);
+    if (threadIdx.x == 0) p.ctl->done_blocks = 0;
+  }
+}
+
+// The queue a top-down level needs after a bottom-up one, in the host-driven
+// loop; returns at once when the control block asks for none.
+template <int W>
+__global__ void __launch_bounds__(LEVEL_BLOCK) queue_kernel(const __grid_constant__ LevelParams p) {
+  __shared__ BlockQueue bq;
+  volatile LevelCtl* c = p.ctl;
+  if (c->terminated || !c->build_queue) return;
+  build_queue<W>(p, bq, c->level % 3);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&p.ctl->done_blocks, 1u) == gridDim.x - 1) {
+      p.ctl->done_blocks = 0;
+      p.ctl->build_queue = 0;
+    }
+  }
+}
+
+// Grid barrier of the traversal kernel between levels, with the controller
+// run by the last block to arrive. Only valid in a cooperative launch (every
+// block resident). The wait is bounded: a block that gives up flags
+// STATUS_STUCK and returns false.
+constexpr uint32_t BARRIER_SPINS = 1u << 26;  // tens of seconds
+template <int W, typename Last>
+__device__ __forceinline__ bool level_barrier(const LevelParams& p, LevelShared<W>& sh,
+                                              Last&& last_block) {
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    GridSync* g = p.sync;
+    uint32_t gen = 0, last = 0;
+    if (threadIdx.x == 0) {
+      gen = __ldcg(&g->gen);  // cannot advance before this block arrives
+      __threadfence();
+      last = atomicAdd(&g->arrive, 1u) == gridDim.x - 1;
+    }
+    last = __shfl_sync(FULL, last, 0);
+    bool ok = true;
+    if (last) {
+      __threadfence();
+      last_block();
+      __syncwarp();
+      if (threadIdx.x == 0) {
+        g->arrive = 0;
+        __threadfence();
+        asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(&g->gen), "r"(gen + 1) : "memory");
+      }
+    } else if (threadIdx.x == 0) {
+      uint32_t now = gen, spins = 0;
+      do {
+        asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(&g->gen) : "memory");
+      } while (now == gen && ++spins < BARRIER_SPINS);
+      if (now == gen) {
+        atomicOr(&p.ctl->status, STATUS_STUCK);
+        ok = false;
+      }
+    }
+    if (threadIdx.x == 0) {
+      __threadfence();
+      sh.flag = ok;
+    }
+  }
+  __syncthreads();
+  return sh.flag;
+}
+
+// A whole pass's traversal in one cooperative launch: source init, then level
+// after level with one grid barrier each, then the frontier state's cleanup.
+// A level costs its work plus one barrier. As a graph of kernel launches (a
+// WHILE node around the two level kernels) an empty top-down level took 24 us
+// and an empty bottom-up one 53, against a few here, which was most of the time
+// of traversals of small graphs. Bound of a large level: as pull_phase.
+template <int W>
+__global__ void __launch_bounds__(LEVEL_BLOCK, MSBFS_LEVEL_MIN_BLOCKS)
+    traverse_kernel(const __grid_constant__ LevelParams p) {
+  __shared__ LevelShared<W> sh;
+  LevelCtl* c = p.ctl;
+  if (blockIdx.x == 0) {
+    for (uint32_t i = threadIdx.x; i < sizeof(LevelCtl) / 4; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(c)[i] = 0;
+    __syncthreads();
+    init_sources<W>(p);
+  }
+  uint32_t L = 0;
+  if (!level_barrier<W>(p, sh, [] {})) return;
+  for (;;) {
+    const uint32_t dir = __ldcg(&c->dir);
+    if (__ldcg(&c->build_queue)) {
+      build_queue<W>(p, sh.bq, L % 3);
+      if (!level_barrier<W>(p, sh, [&] {
+            if (threadIdx.x == 0) c->build_queue = 0;
+          }))
+        return;
+    }
+    if (dir == DIR_PULL)
+      run_level<W, DIR_PULL, false>(p, sh, L);
+    else
+      run_level<W, DIR_PUSH, false>(p, sh, L);
+    if (!level_barrier<W>(p, sh, [&] { controller(p, L, dir, false); })) return;
+    if (__ldcg(&c->terminated)) break;
+    ++L;
+  }
+  // Leave the frontier state as the next pass expects it: rows of the last
+  // expanded level and, when the level cap stopped a traversal that was
+  // still going, of the one after it; both bitmaps; the live slices.
+  for (uint32_t k = 0; k < 2; ++k) clear_frontier<W>(p, (L + k) % 3);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.hlive_words;
+       i += gridDim.x * blockDim.x)
+    p.hlive[i] = FULL;
 }
 
 __device__ __forceinline__ uint32_t bit_length(uint32_t x) { return x ? 32 - __clz(x) : 0; }
@@ -1039,8 +1172,6 @@ __device__ __forceinline__ uint32_t bit_length(uint32_t x) { return x ? 32 - __c
 // lane loaded one 4-byte word per vertex (64-byte stride) and relied on the
 // warps sharing a tile to meet in L1, ran 3.9 to 5.6 ms on R-MAT scale 22,
 // S=512 depending on how closely those warps kept in step.
-constexpr int MAT_TILE_WORDS = MAT_BLOCK * 4;
-constexpr int MAT_NPMAX = 8;
 constexpr int MAT_COLS = 16;  // (word, 64-vertex segment) columns per tile
 #ifndef MSBFS_MAT_MIN_BLOCKS
 #define MSBFS_MAT_MIN_BLOCKS 5
@@ -1300,8 +1431,6 @@ constexpr int RED_BLOCK = 256;
 #define MSBFS_RED_MIN_BLOCKS 3
 #endif
 constexpr int RED_MIN_BLOCKS = MSBFS_RED_MIN_BLOCKS;
-constexpr uint32_t RED_CHUNK = 2048;  // vertices per reduction work item
-
 template <int VEC>
 __device__ __forceinline__ bool any_word(const Words<VEC>& x) {
   uint32_t a = 0;
@@ -1311,10 +1440,11 @@ __device__ __forceinline__ bool any_word(const Words<VEC>& x) {
 }
 
 // Per-source reductions (distance sum, reached count, eccentricity) straight
-// from the visited words and level planes, with no S*V matrix. A warp item is
-// one group of G = min(4, W) words of RED_CHUNK consecutive vertices; lane l
-// loads the group of vertex vb + l as one vector (the next tile's visited
-// group is fetched while this one is reduced). For each word c of the group
+// from the visited words and level planes, with no S*V matrix. A block takes
+// one group of G = min(4, W) words of a share of the vertices, its warps
+// tiles of 32 of them in turn; lane l loads the group of vertex vb + l as
+// one vector (the next tile's visited group is fetched while this one is
+// reduced). For each word c of the group
 // the warp transposes the visited word and each level plane (32x32 bits), so
 // lane j holds source 32c+j's bits over the 32 vertices: the reached count is
 // a popcount, the distance sum a popcount per plane, the eccentricity the
@@ -1324,12 +1454,11 @@ __device__ __forceinline__ bool any_word(const Words<VEC>& x) {
 // buffers). Lanes flagged in ovf (deeper than the planes encode) were folded
 // in by the level kernel.
 template <int W>
-__global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(LevelParams p) {
+__global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(const __grid_constant__ LevelParams p) {
   constexpr int G = W >= 4 ? 4 : W;
-  const PassDesc* dsc = p.desc;
-  SourceStats* st = dsc->stats;
+  SourceStats* st = p.d.stats;
   if (!st) return;
-  const uint32_t P = dsc->num_sources;
+  const uint32_t P = p.d.num_sources;
   const uint32_t Wu = (P + 31) / 32;
   const uint32_t ngroups = (Wu + G - 1) / G;
   const uint32_t dmax = p.ctl->level;
@@ -1337,16 +1466,27 @@ __global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(Level
   const bool use_ovf = dmax >= (1u << p.NP);
   const uint32_t lane = threadIdx.x & 31;
   const size_t VW = (size_t)p.V * W;
-  const size_t nitems = (size_t)((p.V + RED_CHUNK - 1) / RED_CHUNK) * ngroups;
-  const size_t warp_g = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
-  const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  // Blocks per word group: each reduces one share of the vertices and adds
+  // its totals once (a share per warp left most warps idle on graphs of a
+  // million vertices: R-MAT 20, one source, 78 us against 22 here).
+  const uint32_t shares = max(gridDim.x / ngroups, 1u);
+  const uint32_t per_share = ((p.V + shares - 1) / shares + 31) / 32 * 32;
+  __shared__ unsigned long long s_sum[G * 32];
+  __shared__ uint32_t s_cnt[G * 32], s_ecc[G * 32];
   Words<G> zero;
 #pragma unroll
   for (int j = 0; j < G; ++j) zero.w[j] = 0;
-  for (size_t it = warp_g; it < nitems; it += nwarps) {
-    const uint32_t g = (uint32_t)(it % ngroups);
-    const uint32_t v0 = (uint32_t)(it / ngroups) * RED_CHUNK;
-    const uint32_t v_end = min(v0 + RED_CHUNK, p.V);
+  for (uint32_t it = blockIdx.x; it < shares * ngroups; it += gridDim.x) {
+    const uint32_t g = it % ngroups;
+    const size_t begin = (size_t)(it / ngroups) * per_share;
+    if (begin >= p.V) continue;  // the same for the whole block
+    const uint32_t v_end = (uint32_t)min(begin + per_share, (size_t)p.V);
+    const uint32_t v0 = (uint32_t)begin + (threadIdx.x & ~31u);
+    for (uint32_t i = threadIdx.x; i < G * 32; i += RED_BLOCK) {
+      s_sum[i] = 0;
+      s_cnt[i] = s_ecc[i] = 0;
+    }
+    __syncthreads();
     unsigned long long sum[G];
     uint32_t cnt[G], ecc[G];
 #pragma unroll
@@ -1356,12 +1496,12 @@ __global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(Level
     }
     Words<G> xn = zero;
     if (v0 + lane < v_end) xn = ld_words<G>(p.vis + (size_t)(v0 + lane) * W + (size_t)g * G);
-    for (uint32_t vb = v0; vb < v_end; vb += 32) {
+    for (uint32_t vb = v0; vb < v_end; vb += RED_BLOCK) {
       const uint32_t v = vb + lane;
       const size_t a = (size_t)v * W + (size_t)g * G;
       const Words<G> x = xn;
       xn = zero;
-      if (v + 32 < v_end) xn = ld_words<G>(p.vis + a + 32 * (size_t)W);
+      if (v + RED_BLOCK < v_end) xn = ld_words<G>(p.vis + a + RED_BLOCK * (size_t)W);
       const bool any = any_word(x);
       if (__ballot_sync(FULL, any) == 0) continue;  // warp-uniform
       Words<G> o = zero, pl[MAT_NPMAX];
@@ -1401,13 +1541,21 @@ __global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(Level
     }
 #pragma unroll
     for (int i = 0; i < G; ++i) {
-      const uint32_t s = 32 * (g * G + i) + lane;
-      if (cnt[i] && s < P) {
-        atomicAdd(&st[s].sum, sum[i]);
-        atomicMax(&st[s].ecc, ecc[i]);
-        atomicAdd(&st[s].reached, cnt[i]);
+      if (!cnt[i]) continue;
+      atomicAdd(&s_sum[32 * i + lane], sum[i]);
+      atomicMax(&s_ecc[32 * i + lane], ecc[i]);
+      atomicAdd(&s_cnt[32 * i + lane], cnt[i]);
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < G * 32; i += RED_BLOCK) {
+      const uint32_t s = 32 * g * G + i;
+      if (s_cnt[i] && s < P) {
+        atomicAdd(&st[s].sum, s_sum[i]);
+        atomicMax(&st[s].ecc, s_ecc[i]);
+        atomicAdd(&st[s].reached, s_cnt[i]);
       }
     }
+    __syncthreads();
   }
 }
 
@@ -1479,10 +1627,10 @@ __device__ __forceinline__ void stage_tile(const LevelParams& p, uint32_t* sh, s
 // per-source reductions run reduce_kernel instead.
 template <int W>
 __global__ void __launch_bounds__(MAT_BLOCK, MAT_MIN_BLOCKS)
-    materialize_kernel(LevelParams p, uint32_t phase) {
+    materialize_kernel(const __grid_constant__ LevelParams p, uint32_t phase) {
   using G = MatGeo<W>;
   extern __shared__ uint32_t mat_sh[];  // [1 + NP][TW][RS]: visited words, then planes
-  const PassDesc* dsc = p.desc;
+  const PassDesc* dsc = &p.d;
   if (dsc->stats) return;
   const uint32_t P = dsc->num_sources;
   const uint32_t Wu = (P + 31) / 32;
@@ -1558,54 +1706,25 @@ __global__ void __launch_bounds__(MAT_BLOCK, MAT_MIN_BLOCKS)
   }
 }
 
-size_t materialize_items(uint32_t V, uint32_t W) {
-  const uint32_t tw = W <= 16 ? W : 16;
-  const uint32_t tv = MAT_TILE_WORDS / tw;
-  return (size_t)((V + tv - 1) / tv) * ((W + tw - 1) / tw);
-}
-
-size_t materialize_smem_bytes(uint32_t W, uint32_t NP) {
-  const uint32_t tw = W <= 16 ? W : 16;
-  const uint32_t tv = MAT_TILE_WORDS / tw;
-  const uint32_t np = NP < (uint32_t)MAT_NPMAX ? NP : (uint32_t)MAT_NPMAX;
-  return (size_t)(1 + np) * tw * (tv + 2) * sizeof(uint32_t);
-}
-
-// Zeroes the frontier rows left after the loop has stopped: those of the
-// last expanded level L and, when the level cap stopped a traversal that was
-// still going, those of level L + 1 (empty after a normal stop).
+// Leaves the frontier state of a host-driven pass as the next pass expects
+// it, like the end of traverse_kernel.
 template <int W>
-__global__ void cleanup_kernel(LevelParams p) {
+__global__ void cleanup_kernel(const __grid_constant__ LevelParams p) {
   const uint32_t L = p.ctl->level;
-  for (uint32_t k = 0; k < 2; ++k)
-    clear_frontier_rows<W>(p, (L + k) % 3, p.ctl->qcount[(L + k) % 3],
-                           blockIdx.x * (size_t)blockDim.x + threadIdx.x,
-                           (size_t)gridDim.x * blockDim.x);
-}
-
-// Traversed edges of a distance matrix (crates/cli/src/bench.rs:478-491).
-__global__ void traversed_edges_kernel(uint32_t V, const uint32_t* __restrict__ off,
-                                       const uint32_t* __restrict__ dist, uint32_t S,
-                                       unsigned long long* out) {
-  unsigned long long acc = 0;
-  const size_t total = (size_t)S * V;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-       i += (size_t)gridDim.x * blockDim.x) {
-    if (dist[i] != DIST_MAX) {
-      const uint32_t v = (uint32_t)(i % V);
-      acc += __ldg(off + v + 1) - __ldg(off + v);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
+  for (uint32_t k = 0; k < 2; ++k) clear_frontier<W>(p, (L + k) % 3);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.hlive_words;
+       i += gridDim.x * blockDim.x)
+    p.hlive[i] = FULL;
 }
 
 // ------------------------------------------------------------------ host side
 
+// Kernel symbols and launch shapes at W words per vertex (instantiated in the
+// level_w*.cu files, so the widths compile in parallel).
 template <int W>
-static void fill_info(int num_sms, uint32_t NP, LevelKernelInfo* k) {
+void fill_level_info(int num_sms, uint32_t NP, LevelKernelInfo* k) {
   k->init = (void*)init_kernel<W>;
+  k->traverse = (void*)traverse_kernel<W>;
   k->level[DIR_PUSH][0] = (void*)level_kernel<W, DIR_PUSH, false>;
   k->level[DIR_PUSH][1] = (void*)level_kernel<W, DIR_PUSH, true>;
   k->level[DIR_PULL][0] = (void*)level_kernel<W, DIR_PULL, false>;
@@ -1613,131 +1732,23 @@ static void fill_info(int num_sms, uint32_t NP, LevelKernelInfo* k) {
   k->materialize = (void*)materialize_kernel<W>;
   k->reduce = (void*)reduce_kernel<W>;
   k->cleanup = (void*)cleanup_kernel<W>;
+  k->queue = (void*)queue_kernel<W>;
+  auto resident = [&](const void* fn, int block, size_t smem) {
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, smem);
+    return num_sms * (occ < 1 ? 1 : occ);
+  };
   k->level_block = LEVEL_BLOCK;
+  k->traverse_grid = resident(k->traverse, LEVEL_BLOCK, 0);
   // The counting form runs at the production form's grid (it is only run
   // for its counters; the roofline's durations come from the production form).
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, level_kernel<W, DIR_PULL, false>,
-                                                LEVEL_BLOCK, 0);
-  k->level_grids[DIR_PULL] = num_sms * (occ < 1 ? 1 : occ);
-  occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, level_kernel<W, DIR_PUSH, false>,
-                                                LEVEL_BLOCK, 0);
-  k->level_grids[DIR_PUSH] = num_sms * (occ < 1 ? 1 : occ);
+  for (uint32_t d : {(uint32_t)DIR_PUSH, (uint32_t)DIR_PULL})
+    k->level_grids[d] = resident(k->level[d][0], LEVEL_BLOCK, 0);
   k->mat_block = MAT_BLOCK;
   k->mat_smem = materialize_smem_bytes(W, NP);
-  int mocc = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mocc, materialize_kernel<W>, MAT_BLOCK,
-                                                k->mat_smem);
-  if (mocc < 1) mocc = 1;
-  k->mat_grid = num_sms * mocc;
+  k->mat_grid = resident(k->materialize, MAT_BLOCK, k->mat_smem);
   k->red_block = RED_BLOCK;
-  int rocc = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rocc, reduce_kernel<W>, RED_BLOCK, 0);
-  if (rocc < 1) rocc = 1;
-  k->red_grid = num_sms * rocc;
-}
-
-bool level_kernel_info(uint32_t W, uint32_t NP, int num_sms, LevelKernelInfo* out) {
-  switch (W) {
-    case 1: fill_info<1>(num_sms, NP, out); return true;
-    case 2: fill_info<2>(num_sms, NP, out); return true;
-    case 4: fill_info<4>(num_sms, NP, out); return true;
-    case 8: fill_info<8>(num_sms, NP, out); return true;
-    case 16: fill_info<16>(num_sms, NP, out); return true;
-    case 32: fill_info<32>(num_sms, NP, out); return true;
-    case 64: fill_info<64>(num_sms, NP, out); return true;
-    default: return false;
-  }
-}
-
-template <int W>
-static void launch_init_t(const LevelParams& p, cudaStream_t s) {
-  init_kernel<W><<<1, 256, 0, s>>>(p);
-}
-void launch_init(const LevelParams& p, cudaStream_t s) {
-  switch (p.W) {
-    case 1: launch_init_t<1>(p, s); break;
-    case 2: launch_init_t<2>(p, s); break;
-    case 4: launch_init_t<4>(p, s); break;
-    case 8: launch_init_t<8>(p, s); break;
-    case 16: launch_init_t<16>(p, s); break;
-    case 32: launch_init_t<32>(p, s); break;
-    case 64: launch_init_t<64>(p, s); break;
-  }
-}
-
-template <int W, bool COUNT>
-static void launch_level_t(const LevelParams& p, const LevelKernelInfo& k, uint32_t dir,
-                           cudaStream_t s) {
-  const cudaGraphConditionalHandle none = 0;
-  if (dir != DIR_PUSH)
-    level_kernel<W, DIR_PULL, COUNT><<<k.level_grids[DIR_PULL], k.level_block, 0, s>>>(p, none);
-  if (dir != DIR_PULL)
-    level_kernel<W, DIR_PUSH, COUNT><<<k.level_grids[DIR_PUSH], k.level_block, 0, s>>>(p, none);
-}
-template <int W>
-static void launch_level_w(const LevelParams& p, const LevelKernelInfo& k, uint32_t dir,
-                           bool count, cudaStream_t s) {
-  if (count)
-    launch_level_t<W, true>(p, k, dir, s);
-  else
-    launch_level_t<W, false>(p, k, dir, s);
-}
-void launch_level(const LevelParams& p, const LevelKernelInfo& k, uint32_t dir, bool count,
-                  cudaStream_t s) {
-  switch (p.W) {
-    case 1: launch_level_w<1>(p, k, dir, count, s); break;
-    case 2: launch_level_w<2>(p, k, dir, count, s); break;
-    case 4: launch_level_w<4>(p, k, dir, count, s); break;
-    case 8: launch_level_w<8>(p, k, dir, count, s); break;
-    case 16: launch_level_w<16>(p, k, dir, count, s); break;
-    case 32: launch_level_w<32>(p, k, dir, count, s); break;
-    case 64: launch_level_w<64>(p, k, dir, count, s); break;
-  }
-}
-
-template <int W>
-static void launch_mat_t(const LevelParams& p, const LevelKernelInfo& k, bool reduce,
-                         cudaStream_t s, uint32_t phase) {
-  if (reduce)
-    reduce_kernel<W><<<k.red_grid, k.red_block, 0, s>>>(p);
-  else
-    materialize_kernel<W><<<k.mat_grid, k.mat_block, k.mat_smem, s>>>(p, phase);
-}
-void launch_materialize(const LevelParams& p, const LevelKernelInfo& k, bool reduce,
-                        cudaStream_t s, uint32_t phase) {
-  switch (p.W) {
-    case 1: launch_mat_t<1>(p, k, reduce, s, phase); break;
-    case 2: launch_mat_t<2>(p, k, reduce, s, phase); break;
-    case 4: launch_mat_t<4>(p, k, reduce, s, phase); break;
-    case 8: launch_mat_t<8>(p, k, reduce, s, phase); break;
-    case 16: launch_mat_t<16>(p, k, reduce, s, phase); break;
-    case 32: launch_mat_t<32>(p, k, reduce, s, phase); break;
-    case 64: launch_mat_t<64>(p, k, reduce, s, phase); break;
-  }
-}
-
-template <int W>
-static void launch_cleanup_t(const LevelParams& p, cudaStream_t s) {
-  cleanup_kernel<W><<<256, 256, 0, s>>>(p);
-}
-void launch_cleanup(const LevelParams& p, cudaStream_t s) {
-  switch (p.W) {
-    case 1: launch_cleanup_t<1>(p, s); break;
-    case 2: launch_cleanup_t<2>(p, s); break;
-    case 4: launch_cleanup_t<4>(p, s); break;
-    case 8: launch_cleanup_t<8>(p, s); break;
-    case 16: launch_cleanup_t<16>(p, s); break;
-    case 32: launch_cleanup_t<32>(p, s); break;
-    case 64: launch_cleanup_t<64>(p, s); break;
-  }
-}
-
-void launch_traversed_edges(uint32_t V, const uint32_t* off, const uint32_t* dist,
-                            uint32_t num_sources, unsigned long long* out, cudaStream_t s) {
-  cudaMemsetAsync(out, 0, sizeof(unsigned long long), s);
-  traversed_edges_kernel<<<1024, 256, 0, s>>>(V, off, dist, num_sources, out);
+  k->red_grid = resident(k->reduce, RED_BLOCK, 0);
 }
 
 }  // namespace msbfs
