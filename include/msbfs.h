@@ -329,8 +329,8 @@ typedef struct msbfs_server_config {
   uint32_t general_sm_percent;     /* grid share of the other slots (0 -> 100) */
   uint32_t reserved;               /* must be 0                                */
 } msbfs_server_config;
-/* Totals since creation: traversals launched and kernel launches (level
- * loop launches counted from each traversal's level count). */
+/* Totals since creation: traversals launched and kernel launches (two per
+ * pass of the level path, one per CTA-path call). */
 int msbfs_server_counters(msbfs_server *server, uint64_t *traversals,
                           uint64_t *kernel_launches);
 typedef struct msbfs_request_info {

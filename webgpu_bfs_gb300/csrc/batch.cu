@@ -36,6 +36,7 @@
 
 #include "../../include/msbfs.h"
 #include "host_graph.h"
+#include "host_pool.h"
 
 namespace msbfs {
 
@@ -405,6 +406,8 @@ struct msbfs_batch {
   msbfs_engine* eng = nullptr;  // plain per-graph comparison path
   std::vector<msbfs_graph*> eng_graphs;
   double last_ms = 0;
+  std::mutex result_mu;  // one result copy at a time on the pool
+  HostPool pool;
   ~msbfs_batch() {
     for (msbfs_graph* g : eng_graphs) msbfs_graph_destroy(g);
     if (eng) msbfs_engine_destroy(eng);
@@ -718,7 +721,15 @@ int msbfs_batch_result(msbfs_batch* b, size_t i, uint32_t* out) {
   if (!b || i >= b->graphs.size() || !out) return MSBFS_ERR_INVALID_ARGUMENT;
   BCK(cudaSetDevice(b->device));
   const BatchGraph& g = b->graphs[i];
-  BCK(cudaMemcpyAsync(out, g.dist, (size_t)g.S * g.V * 4, cudaMemcpyDeviceToHost, b->stream));
+  const size_t bytes = (size_t)g.S * g.V * 4;
+  std::lock_guard<std::mutex> lk(b->result_mu);
+  cudaPointerAttributes attr{};
+  if (cudaPointerGetAttributes(&attr, out) != cudaSuccess) cudaGetLastError();
+  if (attr.type == cudaMemoryTypeUnregistered) {
+    prefault(b->pool, out, bytes);
+    b->pool.wait();
+  }
+  BCK(cudaMemcpyAsync(out, g.dist, bytes, cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaStreamSynchronize(b->stream));
   return MSBFS_OK;
 }

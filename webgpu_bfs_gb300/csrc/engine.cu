@@ -32,6 +32,7 @@
 #include "../../include/msbfs.h"
 #include "device_common.cuh"
 #include "host_graph.h"
+#include "host_pool.h"
 
 using namespace msbfs;
 
@@ -185,6 +186,7 @@ struct msbfs_engine {
   uint8_t* h_dist8 = nullptr;  // page-locked landing buffer of the byte rows
   size_t h_dist8_cap = 0;
   std::vector<cudaEvent_t> chunk_events;  // one per landed chunk of byte rows
+  HostPool pool;              // host-side output work of the running call
   // Page-locked output: share of a pass's rows written as u32 over the link
   // (MSBFS_SPLIT_ROWS; R-MAT 22, S=512: 1.0 50.5 ms per call, 0.8 47.0,
   // 0.7 45.8, 0.6 44.0, 0.5 ~45).
@@ -917,8 +919,8 @@ void free_graph(msbfs_graph* g) {
 }
 
 // Copies n byte distances from the device to the host through a ring of
-// page-locked chunk slots (one event per slot on the copy stream) while
-// every hardware thread widens each chunk, once it has landed, into u32
+// page-locked chunk slots (one event per slot on the copy stream) while the
+// engine's host threads widen each chunk, once it has landed, into u32
 // (0xFF -> 0xFFFFFFFF) at `out`: the host link carries a quarter of the
 // bytes, and the host's cores, which write memory faster than the link
 // delivers it, do the widening. The calling thread issues the copies; a
@@ -927,7 +929,10 @@ void free_graph(msbfs_graph* g) {
 // the slot's event.
 int widen_to_host(msbfs_engine* eng, const uint8_t* src, uint32_t* out, size_t n) {
   if (n == 0) return MSBFS_OK;
-  constexpr size_t CHUNK = 32u << 20, SLOTS = 16;
+  constexpr size_t SLOTS = 16, CHUNK_MAX = 32u << 20;
+  // Chunks of an eighth of the rows (1 MB at least), so that small calls
+  // overlap their copies with the widening too.
+  const size_t CHUNK = std::min(CHUNK_MAX, std::max<size_t>(1u << 20, (n / 8 + 4095) / 4096 * 4096));
   const size_t stage = std::min(n, CHUNK * SLOTS);
   if (stage > eng->h_dist8_cap) {
     if (eng->h_dist8) cudaFreeHost(eng->h_dist8);
@@ -942,47 +947,47 @@ int widen_to_host(msbfs_engine* eng, const uint8_t* src, uint32_t* out, size_t n
     eng->chunk_events.push_back(e);
   }
   const size_t nchunks = (n + CHUNK - 1) / CHUNK;
-  const unsigned T = std::max(1u, std::thread::hardware_concurrency());
+  // A worker per 256 KB (us into fresh memory with 4 / 16 workers: 1 MB of
+  // distances, R-MAT 14 S=64, 289 / 381; 17 MB, R-MAT 17 S=129, 2,114 / 1,616).
+  const unsigned T =
+      (unsigned)std::min<size_t>(HostPool::max_workers(), std::max<size_t>(n >> 18, 1));
   std::mutex mu;
   std::condition_variable cv;
   size_t issued = 0, widened = 0;  // chunks issued / widened by every worker (in order)
   unsigned slot_done[SLOTS] = {};
   bool failed = false;
   const uint8_t* ring = eng->h_dist8;
-  std::vector<std::thread> workers;
-  for (unsigned k = 0; k < T; ++k) {
-    workers.emplace_back([&, k] {
-      cudaSetDevice(eng->device);
-      for (size_t c = 0; c < nchunks; ++c) {
-        {
-          std::unique_lock<std::mutex> lk(mu);
-          cv.wait(lk, [&] { return issued > c || failed; });
-          if (failed) return;
-        }
-        const size_t slot = c % SLOTS;
-        if (cudaEventSynchronize(eng->chunk_events[slot]) != cudaSuccess) {
-          std::lock_guard<std::mutex> lk(mu);
-          failed = true;
-          cv.notify_all();
-          return;
-        }
-        const size_t b = c * CHUNK, len = std::min(CHUNK, n - b);
-        const size_t lo = len * k / T, hi = len * (k + 1) / T;
-        const uint8_t* in = ring + slot * CHUNK;
-        uint32_t* o = out + b;
-        for (size_t i = lo; i < hi; ++i) {
-          const uint32_t d = in[i];
-          o[i] = d == 0xFFu ? 0xFFFFFFFFu : d;
-        }
-        std::lock_guard<std::mutex> lk(mu);
-        if (++slot_done[slot] == T) {
-          slot_done[slot] = 0;
-          ++widened;
-          cv.notify_all();
-        }
+  eng->pool.start(T, [&](unsigned k) {
+    cudaSetDevice(eng->device);
+    for (size_t c = 0; c < nchunks; ++c) {
+      {
+        std::unique_lock<std::mutex> lk(mu);
+        cv.wait(lk, [&] { return issued > c || failed; });
+        if (failed) return;
       }
-    });
-  }
+      const size_t slot = c % SLOTS;
+      if (cudaEventSynchronize(eng->chunk_events[slot]) != cudaSuccess) {
+        std::lock_guard<std::mutex> lk(mu);
+        failed = true;
+        cv.notify_all();
+        return;
+      }
+      const size_t b = c * CHUNK, len = std::min(CHUNK, n - b);
+      const size_t lo = len * k / T, hi = len * (k + 1) / T;
+      const uint8_t* in = ring + slot * CHUNK;
+      uint32_t* o = out + b;
+      for (size_t i = lo; i < hi; ++i) {
+        const uint32_t d = in[i];
+        o[i] = d == 0xFFu ? 0xFFFFFFFFu : d;
+      }
+      std::lock_guard<std::mutex> lk(mu);
+      if (++slot_done[slot] == T) {
+        slot_done[slot] = 0;
+        ++widened;
+        cv.notify_all();
+      }
+    }
+  });
   cudaError_t err = cudaSuccess;
   for (size_t c = 0; c < nchunks && err == cudaSuccess; ++c) {
     const size_t slot = c % SLOTS, b = c * CHUNK, len = std::min(CHUNK, n - b);
@@ -1001,13 +1006,30 @@ int widen_to_host(msbfs_engine* eng, const uint8_t* src, uint32_t* out, size_t n
       failed = true;
     cv.notify_all();
   }
-  for (std::thread& t : workers) t.join();
+  eng->pool.wait();
   if (failed || err != cudaSuccess) {
     cudaGetLastError();
     return set_err(eng, MSBFS_ERR_CUDA, "byte-row copy failed");
   }
   return MSBFS_OK;
 }
+
+// Whether p is ordinary host memory (not page-locked, managed or device).
+bool is_pageable(const void* p) {
+  cudaPointerAttributes attr{};
+  if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return attr.type == cudaMemoryTypeUnregistered;
+}
+
+// Waits for the engine's host workers when the scope ends, on every path: the
+// caller may free the buffer they work on once the call has returned.
+struct PoolScope {
+  HostPool& pool;
+  ~PoolScope() { pool.wait(); }
+};
 
 // Blocking run into caller-owned host memory.
 int run_host(msbfs_engine* eng, int method, const msbfs_graph* g, const uint32_t* sources,
@@ -1025,6 +1047,7 @@ int run_host(msbfs_engine* eng, int method, const msbfs_graph* g, const uint32_t
   // the host link serves ~9x slower than a staged copy, so it keeps staging.
   const bool cta = method_path(resolve_method(g, method, S)) == MSBFS_PATH_CTA;
   const size_t V = g->V;
+  const PoolScope scope{eng->pool};
   uint32_t* zc = nullptr;  // device address of page-locked `out`
   if (eng->zero_copy && !cta) {
     cudaPointerAttributes attr{};
@@ -1043,6 +1066,14 @@ int run_host(msbfs_engine* eng, int method, const msbfs_graph* g, const uint32_t
   // link while the host widens the rest, which travel as bytes. Without room
   // for the byte rows the call keeps u32 rows throughout.
   const bool use_bytes = eng->narrow && !cta && (!zc || eng->split_frac < 1.0);
+  // u32 rows copied into pageable memory: fresh pages are made present while
+  // the traversal runs (byte rows' widening faults them in by itself). Road
+  // 339x338 into fresh memory: S=256 (117 MB) 5.27 -> 4.43 ms, S=16 (7 MB)
+  // 0.68 -> 0.70.
+  constexpr size_t PREFAULT_FROM = size_t(32) << 20;
+  const size_t out_bytes = S * V * sizeof(uint32_t);
+  if (!use_bytes && !zc && out_bytes >= PREFAULT_FROM && is_pageable(out))
+    prefault(eng->pool, out, out_bytes);
   if (use_bytes && grow(eng, &eng->d_dist8, &eng->d_dist8_cap, S * V) == MSBFS_OK) {
     uint32_t* wide = zc;
     if (!wide) {

@@ -213,8 +213,7 @@ void scheduler(msbfs_server* s) {
         msbfs_stats st{};
         rc = msbfs_engine_synchronize(sl.eng, &st);
         s->traversals++;
-        s->kernel_launches +=
-            st.path == MSBFS_PATH_CTA ? 1 : (uint64_t)(st.levels + 3) * st.passes;
+        s->kernel_launches += st.path == MSBFS_PATH_CTA ? 1 : 2 * (uint64_t)st.passes;
       }
       const size_t eb = elem_bytes(sl.mode, s->V);
       for (const Part& p : sl.parts) {
