@@ -103,3 +103,37 @@ def test_batched_vertex_tiles_match_oracle(native, oracle, tmp_path, div):
                 assert_same(b.result(i), want, g, s, f"vertex tiles W<={words} div={div} {i}")
         finally:
             b.close()
+
+
+@pytest.mark.parametrize("chunk", [1, 3])
+def test_batched_single_source_items_match_oracle(native, oracle, tmp_path, chunk):
+    """Single-source items forced for every class: lists around the length
+    from which whole warps take them (128) and around their pieces (1,024),
+    more pieces in one level than a block sets aside, frontiers beyond the
+    shared-memory queue halves (2,048), single vertices and deep paths."""
+    def fan(n, hubs):  # every hub linked to the n others
+        e = [(h, hubs + i) for h in range(hubs) for i in range(n)]
+        return native.CsrGraph.from_edge_list(n + hubs, e + [(v, u) for u, v in e])
+    items = []
+    for n in (127, 128, 129, 1023, 1024, 1025, 2049, 5000):
+        items.append((native.star_graph(n + 1), np.array([0, 1, n], np.uint32)))
+    items.append((fan(1100, 600), np.array([0, 700, 1699], np.uint32)))  # 1,200 pieces at once
+    items.append((native.generate_graph500_rmat(13, 16, 2),
+                  np.arange(0, 8192, 1500, dtype=np.uint32)))
+    items.append((native.single_vertex(), np.array([0], np.uint32)))
+    items.append((native.disconnected_cliques([3, 200, 1, 40]), np.array([0, 5, 203], np.uint32)))
+    items.append((native.path_graph(900), np.array([0, 450], np.uint32)))
+    b = native.BatchedBfs(items)
+    try:
+        classes = sorted({b.config(i)["class"] for i in range(len(items))})
+        cache = tmp_path / "single.txt"
+        cache.write_text("".join(f"{c} 1 8 16 {chunk} 0 1.0\n" for c in classes))
+        b.autotune(samples_per_class=1, cache_path=str(cache))
+        for _ in range(2):
+            b.run()
+            for i, (g, s) in enumerate(items):
+                assert b.config(i)["alg"] == "source_per_bfs"
+                want = oracle.ms_bfs_fifo(g.num_vertices, g.row_offsets, g.col_indices, s)
+                assert_same(b.result(i), want, g, s, f"single-source items {i}")
+    finally:
+        b.close()

@@ -495,3 +495,24 @@ def test_cta_block_forms(native, gpu_engine, oracle, graph):
     src = np.arange(0, 600, 7, dtype=np.uint32)
     got = gpu_engine.run_ms_bfs_with_method(native.GpuBfsMethod.WorkgroupPersistentBfs, hub, src)
     assert_same(got, oracle.ms_bfs_fifo(600, hub.row_offsets, hub.col_indices, src), hub, src, "star")
+
+
+def test_level_records_of_both_forms_agree(native):
+    """The counting and the production level kernels, driven by the host,
+    record the same directions and discovered pairs for every level, and with
+    the sources these are all pairs reached."""
+    g = native.generate_graph500_rmat(12, 8, 3)
+    src = native.sample_sources(g, 70, 1, min_degree=1)
+    eng = native.GpuBfsEngine(native.GpuBfsMethod.PushPullAdaptive)
+    try:
+        logs = []
+        for level in (1, 2, 3):
+            eng.set_profiling(level)
+            eng.run_ms_bfs(g, src)
+            recs = [(r["level"], r["dir"], r["new_pairs"]) for r in eng.level_log() if r["dir"] < 2]
+            assert sum(r[2] for r in recs) + src.size == eng.last_stats["reached_pairs"]
+            logs.append(recs)
+        assert logs[0] == logs[1] == logs[2]
+        assert {r[1] for r in logs[0]} == {0, 1}
+    finally:
+        eng.close()

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "../../include/msbfs.h"
+#include "cta_expand.cuh"
 #include "host_graph.h"
 #include "host_pool.h"
 
@@ -271,50 +272,92 @@ __device__ void bp_item(const BatchGraph& g, uint32_t s0, uint32_t P, uint32_t* 
   __syncthreads();
 }
 
-// One single-source BFS per source of [s0, s0+n); visited bitmap in shared
-// memory, frontier queues (2V) in the block's scratch.
+// Single-source items: frontier entries per shared-memory queue half, and the
+// long edge lists of a level, set aside in pieces for whole warps.
+constexpr uint32_t BATCH_QH = 2048;
+constexpr uint32_t BIG_DEGREE = 128, BIG_PIECE = 1024, BIG_PIECES = 1024;
+constexpr size_t BATCH_ITEM_SMEM = (2 * BATCH_QH + 2 * BIG_PIECES) * sizeof(uint32_t);
+
+// One single-source BFS per source of [s0, s0+n); visited bitmap and queue
+// halves in shared memory, the rest of the queue (V words) in the block's
+// scratch. Bound: latency of the level's steps and instruction issue; a level
+// is one pass over the frontier with lane pairs (cta_expand) and one over the
+// pieces of long lists with whole warps, so that no thread walks a hub's
+// edges alone. ms of 36 Erdos-Renyi graphs / 18 road-like grids / 6 R-MAT 16
+// graphs / all 60 at once (2,740 sources): a thread per frontier vertex and a
+// counter atomic per discovery 1.56 / 1.73 / 3.93 / 4.57; this 0.79 / 1.22 /
+// 1.98 / 2.82; with 3 or 2 blocks per SM instead of 4 all take 3.05 / 3.62,
+// blocks of 256 threads 3.82, of 1,024 5.19, 1 or 4 lanes a vertex 3.13 / 2.84,
+// lists set aside from 32 edges 3.24.
 __device__ void cta_item(const BatchGraph& g, uint32_t s0, uint32_t n, uint32_t* scr,
                          uint32_t* bitmap, uint32_t* s_cnt) {
-  const uint32_t V = g.V, tid = threadIdx.x, bs = blockDim.x;
+  const uint32_t V = g.V, tid = threadIdx.x, bs = BATCH_BLOCK;
   const uint32_t bwords = (V + 31) / 32;
+  const uint32_t sbits = smem_addr(bitmap), scnt = smem_addr(s_cnt);
+  const uint32_t squeue = sbits + (bwords + 1) / 2 * 8, sbig = squeue + 8 * BATCH_QH;
+  const uint32_t spieces = scnt + 12;  // pieces set aside, by level parity
+  uint32_t snbig = spieces;
+  const CtaQueue<false> q{squeue, scr, BATCH_QH, V, g.off};
+  auto mark = [&](uint32_t v, uint32_t bit) { return atoms_or(sbits + (v >> 5) * 4, bit); };
+  auto big = [&](uint32_t e, uint32_t d) {
+    if (d <= BIG_DEGREE) return false;
+    const uint32_t pieces = (d + BIG_PIECE - 1) / BIG_PIECE;
+    const uint32_t at = atoms_add(snbig, pieces);
+    const bool fits = at + pieces <= BIG_PIECES;
+    for (uint32_t k = 0; k < pieces && at + k < BIG_PIECES; ++k) {
+      sts32(sbig + 8 * (at + k), e + k * BIG_PIECE);
+      sts32(sbig + 8 * (at + k) + 4, fits ? min(BIG_PIECE, d - k * BIG_PIECE) : 0u);
+    }
+    return fits;
+  };
   for (uint32_t si = s0; si < s0 + n; ++si) {
     for (uint32_t i = tid; i < bwords; i += bs) bitmap[i] = 0;
+    if (tid < 5) s_cnt[tid] = 0;  // three rotating frontier counters, the pieces' two
     __syncthreads();
     const uint32_t src = g.src[si];
     uint32_t* row = g.dist + (size_t)si * V;
-    uint32_t* qin = scr;
-    uint32_t* qout = scr + V;
     if (tid == 0) {
       bitmap[src >> 5] = 1u << (src & 31);
       row[src] = 0;
-      qin[0] = src;
-      s_cnt[1] = 0;
+      sts32(squeue, src);
     }
-    uint32_t n_in = 1;
+    uint32_t n_in = 1, level = 0, reached = 0, slot = 0;  // slot: 4 * (level % 3)
     __syncthreads();
-    for (uint32_t L = 0; n_in; ++L) {
-      for (uint32_t i = tid; i < n_in; i += bs) {
-        const uint32_t u = qin[i];
-        for (uint32_t e = g.off[u]; e < g.off[u + 1]; ++e) {
-          const uint32_t v = g.idx[e];
-          const uint32_t bit = 1u << (v & 31);
-          if (bitmap[v >> 5] & bit) continue;
-          if (atomicOr(&bitmap[v >> 5], bit) & bit) continue;
-          row[v] = L + 1;
-          qout[atomicAdd(&s_cnt[1], 1u)] = v;
-        }
+    while (n_in) {
+      reached += n_in;
+      const uint32_t nslot = slot == 8 ? 0 : slot + 4;
+      snbig = spieces + (level & 1) * 4;
+      if (tid == 0) {
+        sts32(scnt + nslot, 0);
+        sts32(spieces + (~level & 1) * 4, 0);  // last read before this level began, unless 0
       }
+      cta_expand<false, BATCH_BLOCK, 2, 2>(nullptr, g.idx, q, level, n_in, scnt + slot, row, mark,
+                                           big);
       __syncthreads();
-      n_in = s_cnt[1];
-      __syncthreads();
-      if (tid == 0) s_cnt[1] = 0;
-      uint32_t* t = qin;
-      qin = qout;
-      qout = t;
-      __syncthreads();
+      const uint32_t nbig = min(lds32(snbig), BIG_PIECES);
+      if (nbig) {
+        for (uint32_t b = tid / 32; b < nbig; b += BATCH_BLOCK / 32) {
+          const uint32_t e = lds32(sbig + 8 * b), len = lds32(sbig + 8 * b + 4);
+          for (uint32_t j = tid & 31; j - (tid & 31) < len; j += 128) {
+            uint32_t v[4];
+            bool fresh[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              fresh[k] = j + 32 * k < len;
+              v[k] = fresh[k] ? __ldg(g.idx + e + j + 32 * k) : 0u;
+            }
+            cta_discover<false, 4>(q, level + 1, scnt + slot, row, v, v, fresh, mark);
+          }
+        }
+        __syncthreads();
+      }
+      n_in = lds32(scnt + slot);
+      slot = nslot;
+      ++level;
     }
-    for (uint32_t v = tid; v < V; v += bs)
-      if (!((bitmap[v >> 5] >> (v & 31)) & 1u)) row[v] = BATCH_DIST_MAX;
+    if (reached < V)
+      for (uint32_t v = tid; v < V; v += bs)
+        if (!((bitmap[v >> 5] >> (v & 31)) & 1u)) row[v] = BATCH_DIST_MAX;
     __syncthreads();
   }
 }
@@ -323,10 +366,10 @@ __device__ void cta_item(const BatchGraph& g, uint32_t s0, uint32_t n, uint32_t*
 // word arrays double the kernel's registers (and halve its occupancy), so
 // a launch takes that form only when some graph's class runs vertex tiles.
 template <bool VT>
-__global__ void __launch_bounds__(BATCH_BLOCK) batch_kernel(BatchParams p) {
+__global__ void __launch_bounds__(BATCH_BLOCK, VT ? 2 : 4) batch_kernel(BatchParams p) {
   extern __shared__ uint32_t sbits[];
   __shared__ uint32_t s_item;
-  __shared__ uint32_t s_cnt[2];
+  __shared__ uint32_t s_cnt[5];
   uint32_t* scr = p.scratch + (size_t)blockIdx.x * p.scratch_words;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(p.cursor, 1u);
@@ -580,7 +623,9 @@ int msbfs_batch_create(int device, const msbfs_batch_graph* graphs, size_t n, ms
   // Scratch per resident block: the larger of ALG_BP (3*V*8 words + 2V) and
   // ALG_CTA (2V) for the largest graph.
   b->scratch_words = 3 * maxVW * 8 + 2 * maxVW + 64;
-  b->smem = ((b->max_V + 31) / 32) * 4;
+  // Shared memory: the bitmap, then a single-source item's queue halves and
+  // pieces (a bit-parallel item uses the bitmap only).
+  b->smem = ((b->max_V + 31) / 32 + 1) / 2 * 8 + BATCH_ITEM_SMEM;
   BCK(cudaFuncSetAttribute(batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)std::max<size_t>(b->smem, 4)));
   BCK(cudaFuncSetAttribute(batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -657,7 +702,8 @@ int msbfs_batch_autotune(msbfs_batch* b, size_t samples_per_class, const char* c
       int rc = launch_batch(b, sample, &ms);  // warm
       if (rc) return rc;
       if ((rc = launch_batch(b, sample, &ms))) return rc;
-      if (ms < best.ms) {
+      // (within 3% is timing noise on a sample: the earlier candidate stays)
+      if (ms < best.ms * 0.97) {
         best = c;
         best.ms = ms;
       }

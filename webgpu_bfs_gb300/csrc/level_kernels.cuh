@@ -965,7 +965,8 @@ struct LevelShared {
 // L-1 (not read or written this level), runs the bottom-up or top-down step,
 // appends the block's discoveries to the next queue and adds its counts to
 // the control block. Starts and ends with the block's threads in step.
-template <int W, uint32_t DIR, bool COUNT>
+// HOST: a launch of its own, whose record holds the level's discovered pairs.
+template <int W, uint32_t DIR, bool HOST, bool COUNT>
 __device__ __forceinline__ void run_level(const LevelParams& p, LevelShared<W>& sh, uint32_t L) {
   LevelCtl* c = p.ctl;
   if (threadIdx.x == 0) sh.bq.count = 0;
@@ -1008,12 +1009,12 @@ __device__ __forceinline__ void run_level(const LevelParams& p, LevelShared<W>& 
       for (int w = 0; w < LEVEL_BLOCK / 32; ++w) tot += sh.red[i][w];
     if (tot) {
       if (i == 3) atomicAdd(&c->pairs, tot);
+      if (HOST && i == 3) atomicAdd(&c->c_pairs, tot);
       if (i == 2 && DIR == DIR_PULL) atomicAdd(&c->qverts[(L + 1) % 3], (uint32_t)tot);
-      if constexpr (COUNT)
+      if (COUNT && i != 3)
         atomicAdd(i == 0   ? &c->c_active
                   : i == 1 ? &c->c_edges
                   : i == 2 ? &c->c_newv
-                  : i == 3 ? &c->c_pairs
                            : &c->c_rows,
                   tot);
     }
@@ -1036,7 +1037,7 @@ __global__ void __launch_bounds__(LEVEL_BLOCK, DIR == DIR_PULL ? MSBFS_LEVEL_MIN
   if (c->terminated || c->dir != DIR || (DIR == DIR_PUSH && c->build_queue)) return;
   const uint32_t L = c->level;
   if (COUNT && threadIdx.x == 0) atomicMin(&p.ctl->t_start, globaltimer());
-  run_level<W, DIR, COUNT>(p, sh, L);
+  run_level<W, DIR, true, COUNT>(p, sh, L);
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -1144,9 +1145,9 @@ __global__ void __launch_bounds__(LEVEL_BLOCK, MSBFS_LEVEL_MIN_BLOCKS)
         return;
     }
     if (dir == DIR_PULL)
-      run_level<W, DIR_PULL, false>(p, sh, L);
+      run_level<W, DIR_PULL, false, false>(p, sh, L);
     else
-      run_level<W, DIR_PUSH, false>(p, sh, L);
+      run_level<W, DIR_PUSH, false, false>(p, sh, L);
     if (!level_barrier<W>(p, sh, [&] { controller(p, L, dir, false); })) return;
     if (__ldcg(&c->terminated)) break;
     ++L;
