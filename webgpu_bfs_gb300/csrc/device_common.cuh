@@ -220,7 +220,7 @@ struct CtaParams {
   const uint32_t* sources;
   uint32_t num_sources;
   uint32_t* dist;        // row s at dist + s * V (null when stats is set)
-  uint32_t* gqueue;      // per resident block: V u32
+  uint32_t* gqueue;      // per resident block: V u32 (unused when V <= qh)
   uint32_t* work;        // source cursor (zeroed before launch)
   SourceStats* stats;    // non-null: per-source reductions instead of rows
   uint32_t* gbits;       // global-bitmap mode: per resident block ceil(V/32) u32

@@ -138,7 +138,7 @@ struct msbfs_engine {
   std::mutex mu;
   std::string last_error;
   uint32_t max_words = 0;   // words per vertex of a pass at most (0: widest_pass)
-  size_t total_mem = 0;     // device memory
+  size_t total_mem = 0;     // device memory, once a call may want a wide pass
   uint32_t alpha = 14;
   uint32_t beta = 24;
   uint32_t seg = MSBFS_PUSH_SEG;  // out-edges per top-down queue entry
@@ -297,7 +297,7 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   // Blocks that a small graph cannot feed only make the grid barriers of its
   // levels longer: a block per 1,024 lane loads (visited pieces and edges).
   const uint64_t loads = (uint64_t)g->V * std::max(1u, W / 4) + g->E;
-  w->k.traverse_grid = (int)std::min<uint64_t>(w->k.traverse_grid, std::max<uint64_t>(32, loads / 1024));
+  w->k.traverse_grid = (int)std::min<uint64_t>(w->k.traverse_grid, std::max<uint64_t>(64, loads / 1024));
   w->k.traverse_grid = std::max(1, (int)((uint64_t)w->k.traverse_grid * eng->sm_share / 100));
   LevelParams& p = w->p;
   p.V = (uint32_t)g->V;
@@ -466,15 +466,20 @@ int run_pass_host_loop(msbfs_engine* eng, Workspace* w, bool reduce) {
 // 16, S=700 0.525 / 0.421 / -, S=2,048 1.125 / 0.893 / 0.705; R-MAT 20, S=513
 // 2.00 / 2.05 / -, S=2,048 5.99 / 4.92 / 4.38. Passes above 16 words keep
 // their traversal state within an eighth of the device memory.
-uint32_t widest_pass(const msbfs_engine* eng, const msbfs_graph* g) {
+uint32_t widest_pass(msbfs_engine* eng, const msbfs_graph* g) {
   if (eng->max_words) return eng->max_words;
+  if (size_t free_mem; !eng->total_mem && cudaMemGetInfo(&free_mem, &eng->total_mem) != cudaSuccess) {
+    cudaGetLastError();
+    return 16;
+  }
   uint32_t W = 64;
   while (W > 16 && (uint64_t)g->V * W * 4 * (5 + level_planes(g)) > eng->total_mem / 8) W >>= 1;
   return W;
 }
 
-uint32_t choose_words(const msbfs_engine* eng, const msbfs_graph* g, size_t S) {
-  size_t lanes = std::min<size_t>(S, (size_t)widest_pass(eng, g) * 32);
+uint32_t choose_words(msbfs_engine* eng, const msbfs_graph* g, size_t S) {
+  const uint32_t widest = S > 512 || eng->max_words ? widest_pass(eng, g) : 16;
+  size_t lanes = std::min<size_t>(S, (size_t)widest * 32);
   uint32_t need = (uint32_t)((lanes + 31) / 32);
   uint32_t W = 1;
   while (W < need) W <<= 1;
@@ -554,7 +559,8 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
     // queue slab per cluster.
     const int cl = std::max(1, cta.cluster);
     const int blocks = std::max(cl, std::min<int>(cta_grid, (int)std::min<size_t>(S * cl, 1u << 30)) / cl * cl);
-    if ((rc = grow(eng, &eng->d_cta_queue, &eng->d_cta_queue_cap, (size_t)(blocks / cl) * V)))
+    if (V > cta.qh &&  // else every frontier fits the shared-memory halves
+        (rc = grow(eng, &eng->d_cta_queue, &eng->d_cta_queue_cap, (size_t)(blocks / cl) * V)))
       return rc;
     if (cta.global_bits &&
         (rc = grow(eng, &eng->d_cta_bits, &eng->d_cta_bits_cap, (size_t)blocks * ((V + 31) / 32))))
@@ -1152,8 +1158,6 @@ int msbfs_engine_create(int device, int method, msbfs_engine** out) {
       cudaMalloc((void**)&e->d_counter, sizeof(unsigned long long)) != cudaSuccess)
     return MSBFS_ERR_CUDA;
   e->stream = e->own_stream;
-  size_t free_mem = 0;
-  cudaMemGetInfo(&free_mem, &e->total_mem);
   const char* hl = getenv("MSBFS_HOST_LOOP");
   int coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);

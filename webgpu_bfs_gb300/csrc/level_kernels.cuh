@@ -275,10 +275,10 @@ __device__ __forceinline__ void record_level(const LevelParams& p, uint32_t v, u
                                              const Words<VEC>& newly, uint32_t d) {
   const size_t VW = (size_t)p.V * p.W;
   const size_t off = (size_t)v * p.W + k0;
+  if (p.d.reach) return;  // visited words are the result
   if (d < (1u << p.NP)) {
-    for (uint32_t b = 0; b < p.NP; ++b) {
-      if (!((d >> b) & 1u)) continue;
-      uint32_t* pb = p.planes + b * VW + off;
+    for (uint32_t bits = d; bits; bits &= bits - 1) {
+      uint32_t* pb = p.planes + (__ffs(bits) - 1) * VW + off;
       if constexpr (ATOMIC) {
 #pragma unroll
         for (int j = 0; j < VEC; ++j)
@@ -1636,8 +1636,10 @@ __global__ void __launch_bounds__(MAT_BLOCK, MAT_MIN_BLOCKS)
   const uint32_t P = dsc->num_sources;
   const uint32_t Wu = (P + 31) / 32;
   const uint32_t dmax = p.ctl->level;
-  const uint32_t npu = min(min(p.NP, bit_length(dmax)), (uint32_t)MAT_NPMAX);
-  const bool use_ovf = dmax >= (1u << p.NP);
+  // (a reachability pass records no levels)
+  const uint32_t npu =
+      dsc->reach ? 0u : min(min(p.NP, bit_length(dmax)), (uint32_t)MAT_NPMAX);
+  const bool use_ovf = !dsc->reach && dmax >= (1u << p.NP);
   // Every reached distance fits the planes and stays below the 0xFF marker.
   const bool packed = !use_ovf && dmax < 255u;
   // Byte rows when the pass asks for them and every distance fits a byte
