@@ -773,13 +773,17 @@ int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, ui
   g->split = split;
   g->heavy = heavy;
   g->n_heavy = 0;
-  // A slice is one warp's serial work. With fewer than two full slices of
-  // edges per resident warp, shorter ones: a level of a small graph lasts as
-  // long as its longest slice (directed R-MAT 18, S=333: bottom-up levels of
-  // 220 us behind warps that scanned up to 16 vertices of <= 512 in-edges).
+  // A slice is one warp's serial work. With less than a full slice of edges
+  // per resident warp, shorter ones: a level of a small graph lasts as long
+  // as its longest slice (directed R-MAT 18, S=333: bottom-up levels of 220 us
+  // behind warps that scanned up to 16 vertices of <= 512 in-edges). Not below
+  // 256: a list's slices meet in its candidate words, two fences and an atomic
+  // each. us of a traversal with at least 64 / 128 / 256 / 512: directed R-MAT
+  // 18 S=333 359 / 343 / 334 / 355, R-MAT 16 S=100 231 / 200 / 198 / 220, R-MAT
+  // 14 S=64 147 / 136 / 134 / 124, R-MAT 10 S=300 109 / 118 / 122 / 121.
   uint32_t len = split;
   const uint64_t warps = (uint64_t)eng->num_sms * 64;
-  while (len > 64 && (uint64_t)len * 2 * warps > g->E) len /= 2;
+  while (len > 256 && (uint64_t)len * warps > g->E) len /= 2;
   // Heavy vertices by in-degree, descending (a counting sort; those beyond
   // its range keep their order in front).
   constexpr uint32_t TOP = 1u << 16;
