@@ -45,8 +45,9 @@ constexpr uint32_t CTA_DIST_MAX = 0xffffffffu;
 //   four or more        road 339x338 S=2,048: 256 threads x 2 lanes x 8 blocks
 //     CTA_TPUT          2.84, 192 x 2 x 9 2.80, 256 x 1 x 7 3.07, 256 x 2 x 7
 //                       2.90, 256 x 4 x 7 3.11, 128 x 2 x 14 3.60
-// Global-bitmap mode (graphs whose bitmap does not fit shared memory) uses
-// CTA_MID and CTA_TPUT.
+// Global-bitmap mode (graphs whose bitmap does not fit shared memory, with
+// wider frontiers) always uses CTA_MID: road 1448x1448 S=512 42 ms, CTA_WIDE 44,
+// CTA_TPUT 73.
 #ifndef MSBFS_CTA_TPUT_THREADS
 #define MSBFS_CTA_TPUT_THREADS 256
 #endif
@@ -278,8 +279,8 @@ size_t cta_max_vertices(int device) {
 
 template <bool GB, bool ER>
 static void* cta_fn(int form) {
-  if (form == CTA_TPUT) return (void*)cta_bfs_kernel<GB, ER, CTA_TPUT>;
   if constexpr (!GB) {
+    if (form == CTA_TPUT) return (void*)cta_bfs_kernel<GB, ER, CTA_TPUT>;
     if (form == CTA_WIDE) return (void*)cta_bfs_kernel<GB, ER, CTA_WIDE>;
     if (form == CTA_SMALL) return (void*)cta_bfs_kernel<GB, ER, CTA_SMALL>;
   }
@@ -392,7 +393,7 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   const size_t slack = 2048;  // static shared variables + the driver's per-block reserve
   const size_t fit = std::max<size_t>(1, (size_t)per_sm / (bitmap + slack));
   const size_t per = std::min(fit, (num_sources + sms - 1) / std::max(sms, 1));
-  if (per > CTA_MID_BLOCKS) {
+  if (shared_bits && per > CTA_MID_BLOCKS) {
     sh.form = CTA_TPUT;
     sh.block = CtaForm<CTA_TPUT>::THREADS;
     sh.minb = CtaForm<CTA_TPUT>::MINB;
@@ -420,6 +421,17 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   if (occ < 1) return false;
   sh.grid = sms * occ;
   if (!shared_bits) {
+    // Every edge is an atomic on a bitmap: more blocks than have theirs in
+    // two thirds of the L2 slow each other down, but not fewer than one per
+    // SM. Road 1448x1448 (262 KB bitmaps), S=512 / 2,048, ms with 152, 228,
+    // 304, 456 blocks: 62 / 222, 52 / 175, 42 / 158, 54 / 167. About as many
+    // sources per block each: the nearest whole number of rounds.
+    int l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device);
+    const size_t in_l2 = (size_t)l2 / 3 * 2 / (words * sizeof(uint32_t)) / sms * sms;
+    const size_t most = std::max<size_t>(in_l2, sms);
+    const size_t rounds = std::max<size_t>((num_sources + most / 2) / most, 1);
+    sh.grid = (int)std::min<size_t>((size_t)sh.grid, (num_sources + rounds - 1) / rounds);
     const size_t per_block = ((size_t)V + words) * sizeof(uint32_t);
     sh.grid = (int)std::max<size_t>(
         1, std::min<size_t>((size_t)sh.grid, CTA_GLOBAL_SCRATCH_BYTES / per_block));
