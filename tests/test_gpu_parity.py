@@ -490,11 +490,19 @@ def test_cta_block_forms(native, gpu_engine, oracle, graph):
     assert np.array_equal(st["distance_sum"].astype(np.int64), rows.sum(1))  # connected graphs
     assert np.array_equal(st["eccentricity"], rows.max(1))
     assert (st["reached"] == g.num_vertices).all()
-    # no edge records: the same structure with one hub beyond road-like degrees
-    hub = native.star_graph(600)
-    src = np.arange(0, 600, 7, dtype=np.uint32)
-    got = gpu_engine.run_ms_bfs_with_method(native.GpuBfsMethod.WorkgroupPersistentBfs, hub, src)
-    assert_same(got, oracle.ms_bfs_fifo(600, hub.row_offsets, hub.col_indices, src), hub, src, "star")
+    # no edge records: lists around the length from which whole warps take
+    # them (128) and around their pieces (1,024), more pieces than are set aside
+    hubs = 600
+    fan = np.array([(h, hubs + i) for h in range(hubs) for i in range(1100)])
+    for hub in [native.star_graph(n + 1) for n in (127, 128, 129, 1024, 1025, 9000)] + \
+            [native.CsrGraph.from_edge_list(hubs + 1100, np.concatenate([fan, fan[:, ::-1]]))]:
+        V = hub.num_vertices
+        for S in (3, 3 * sms + 1):
+            src = np.linspace(0, V - 1, S).astype(np.uint32)
+            got = gpu_engine.run_ms_bfs_with_method(native.GpuBfsMethod.WorkgroupPersistentBfs,
+                                                    hub, src)
+            want = oracle.ms_bfs_threaded(V, hub.row_offsets, hub.col_indices, src)
+            assert_same(got, want, hub, src, f"hub lists V={V} S={S}")
 
 
 def test_level_records_of_both_forms_agree(native):

@@ -272,11 +272,9 @@ __device__ void bp_item(const BatchGraph& g, uint32_t s0, uint32_t P, uint32_t* 
   __syncthreads();
 }
 
-// Single-source items: frontier entries per shared-memory queue half, and the
-// long edge lists of a level, set aside in pieces for whole warps.
+// Single-source items: frontier entries per shared-memory queue half.
 constexpr uint32_t BATCH_QH = 2048;
-constexpr uint32_t BIG_DEGREE = 128, BIG_PIECE = 1024, BIG_PIECES = 1024;
-constexpr size_t BATCH_ITEM_SMEM = (2 * BATCH_QH + 2 * BIG_PIECES) * sizeof(uint32_t);
+constexpr size_t BATCH_ITEM_SMEM = 2 * BATCH_QH * sizeof(uint32_t) + BIG_BYTES;
 
 // One single-source BFS per source of [s0, s0+n); visited bitmap and queue
 // halves in shared memory, the rest of the queue (V words) in the block's
@@ -295,21 +293,8 @@ __device__ void cta_item(const BatchGraph& g, uint32_t s0, uint32_t n, uint32_t*
   const uint32_t bwords = (V + 31) / 32;
   const uint32_t sbits = smem_addr(bitmap), scnt = smem_addr(s_cnt);
   const uint32_t squeue = sbits + (bwords + 1) / 2 * 8, sbig = squeue + 8 * BATCH_QH;
-  const uint32_t spieces = scnt + 12;  // pieces set aside, by level parity
-  uint32_t snbig = spieces;
   const CtaQueue<false> q{squeue, scr, BATCH_QH, V, g.off};
   auto mark = [&](uint32_t v, uint32_t bit) { return atoms_or(sbits + (v >> 5) * 4, bit); };
-  auto big = [&](uint32_t e, uint32_t d) {
-    if (d <= BIG_DEGREE) return false;
-    const uint32_t pieces = (d + BIG_PIECE - 1) / BIG_PIECE;
-    const uint32_t at = atoms_add(snbig, pieces);
-    const bool fits = at + pieces <= BIG_PIECES;
-    for (uint32_t k = 0; k < pieces && at + k < BIG_PIECES; ++k) {
-      sts32(sbig + 8 * (at + k), e + k * BIG_PIECE);
-      sts32(sbig + 8 * (at + k) + 4, fits ? min(BIG_PIECE, d - k * BIG_PIECE) : 0u);
-    }
-    return fits;
-  };
   for (uint32_t si = s0; si < s0 + n; ++si) {
     for (uint32_t i = tid; i < bwords; i += bs) bitmap[i] = 0;
     if (tid < 5) s_cnt[tid] = 0;  // three rotating frontier counters, the pieces' two
@@ -326,31 +311,9 @@ __device__ void cta_item(const BatchGraph& g, uint32_t s0, uint32_t n, uint32_t*
     while (n_in) {
       reached += n_in;
       const uint32_t nslot = slot == 8 ? 0 : slot + 4;
-      snbig = spieces + (level & 1) * 4;
-      if (tid == 0) {
-        sts32(scnt + nslot, 0);
-        sts32(spieces + (~level & 1) * 4, 0);  // last read before this level began, unless 0
-      }
-      cta_expand<false, BATCH_BLOCK, 2, 2>(nullptr, g.idx, q, level, n_in, scnt + slot, row, mark,
-                                           big);
-      __syncthreads();
-      const uint32_t nbig = min(lds32(snbig), BIG_PIECES);
-      if (nbig) {
-        for (uint32_t b = tid / 32; b < nbig; b += BATCH_BLOCK / 32) {
-          const uint32_t e = lds32(sbig + 8 * b), len = lds32(sbig + 8 * b + 4);
-          for (uint32_t j = tid & 31; j - (tid & 31) < len; j += 128) {
-            uint32_t v[4];
-            bool fresh[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              fresh[k] = j + 32 * k < len;
-              v[k] = fresh[k] ? __ldg(g.idx + e + j + 32 * k) : 0u;
-            }
-            cta_discover<false, 4>(q, level + 1, scnt + slot, row, v, v, fresh, mark);
-          }
-        }
-        __syncthreads();
-      }
+      if (tid == 0) sts32(scnt + nslot, 0);
+      cta_level<false, BATCH_BLOCK, 2>(nullptr, g.idx, q, level, n_in, scnt + slot, row, mark, sbig,
+                                       scnt + 12);
       n_in = lds32(scnt + slot);
       slot = nslot;
       ++level;

@@ -206,4 +206,60 @@ __device__ __forceinline__ void cta_expand(const uint2* erec, const uint32_t* id
   }
 }
 
+// Long edge lists of a level, set aside in pieces for whole warps, so that no
+// few lanes walk a hub's edges alone.
+constexpr uint32_t BIG_DEGREE = 128, BIG_PIECE = 1024, BIG_PIECES = 1024;
+constexpr size_t BIG_BYTES = BIG_PIECES * 2 * sizeof(uint32_t);
+
+// One level of a block's traversal, up to the barrier after which the next
+// frontier's size, counted at shared address `cnt`, can be read. Graphs without
+// edge records keep lists of more than BIG_DEGREE edges for a second sweep
+// (sbig: shared address of BIG_BYTES, 0 for none; spieces: of two counters, by
+// level parity, both 0 before level 0).
+template <bool ER, int THREADS, int LPV, typename Mark>
+__device__ __forceinline__ void cta_level(const uint2* erec, const uint32_t* idx,
+                                          const CtaQueue<ER>& q, uint32_t level, uint32_t n_in,
+                                          uint32_t cnt, uint32_t* row, Mark&& mark, uint32_t sbig,
+                                          uint32_t spieces) {
+  if constexpr (ER) {
+    cta_expand<ER, THREADS, LPV, 4 / LPV>(erec, idx, q, level, n_in, cnt, row, mark);
+    __syncthreads();
+  } else {
+    const uint32_t snbig = spieces + (level & 1) * 4;
+    // The other parity's counter was last read before this level began.
+    if (threadIdx.x == 0) sts32(spieces + (~level & 1) * 4, 0);
+    cta_expand<ER, THREADS, LPV, 4 / LPV>(
+        erec, idx, q, level, n_in, cnt, row, mark, [&](uint32_t e, uint32_t d) {
+          if (d <= BIG_DEGREE || !sbig) return false;
+          const uint32_t pieces = (d + BIG_PIECE - 1) / BIG_PIECE;
+          const uint32_t at = atoms_add(snbig, pieces);
+          const bool fits = at + pieces <= BIG_PIECES;
+          for (uint32_t k = 0; k < pieces && at + k < BIG_PIECES; ++k) {
+            sts32(sbig + 8 * (at + k), e + k * BIG_PIECE);
+            sts32(sbig + 8 * (at + k) + 4, fits ? min(BIG_PIECE, d - k * BIG_PIECE) : 0u);
+          }
+          return fits;
+        });
+    __syncthreads();
+    const uint32_t nbig = min(lds32(snbig), BIG_PIECES);
+    if (nbig) {
+      for (uint32_t b = threadIdx.x / 32; b < nbig; b += THREADS / 32) {
+        const uint32_t e = lds32(sbig + 8 * b), len = lds32(sbig + 8 * b + 4);
+        for (uint32_t j0 = 0; j0 < len; j0 += 128) {
+          const uint32_t j = j0 + (threadIdx.x & 31);
+          uint32_t v[4];
+          bool fresh[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            fresh[k] = j + 32 * k < len;
+            v[k] = fresh[k] ? __ldg(idx + e + j + 32 * k) : 0u;
+          }
+          cta_discover<ER, 4>(q, level + 1, cnt, row, v, v, fresh, mark);
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
 }  // namespace msbfs

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(CtaForm<FORM>::THREADS, CtaForm<FORM>::MINB)
   constexpr int THREADS = CtaForm<FORM>::THREADS, LPV = CtaForm<FORM>::LPV;
   extern __shared__ __align__(16) uint32_t smem_dyn[];
   __shared__ uint32_t s_src_idx;
-  __shared__ uint32_t s_cnt[3];
+  __shared__ uint32_t s_cnt[5];  // frontier sizes of three levels, pieces of two
   const uint32_t V = p.V;
   const uint32_t words = (V + 31) / 32;
   uint32_t* bits = GB ? p.gbits + (size_t)blockIdx.x * words : smem_dyn;
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(CtaForm<FORM>::THREADS, CtaForm<FORM>::MINB)
   for (;;) {
     if (threadIdx.x == 0) {
       s_src_idx = atomicAdd(p.work, 1u);
-      s_cnt[0] = s_cnt[1] = s_cnt[2] = 0;
+      for (int k = 0; k < 5; ++k) s_cnt[k] = 0;
     }
     for (uint32_t i = threadIdx.x; i < words; i += THREADS) bits[i] = 0;
     __syncthreads();
@@ -126,11 +126,12 @@ __global__ void __launch_bounds__(CtaForm<FORM>::THREADS, CtaForm<FORM>::MINB)
       sum += (unsigned long long)level * n_in;
       const uint32_t nslot = slot == 8 ? 0 : slot + 4;
       if (threadIdx.x == 0) sts32(scnt + nslot, 0);
-      cta_expand<ER, THREADS, LPV, 4 / LPV>(
-          p.erec, p.idx, q, level, n_in, scnt + slot, row, [&](uint32_t v, uint32_t bit) {
+      cta_level<ER, THREADS, LPV>(
+          p.erec, p.idx, q, level, n_in, scnt + slot, row,
+          [&](uint32_t v, uint32_t bit) {
             return GB ? atomicOr(&bits[v >> 5], bit) : atoms_or(sbits + (v >> 5) * 4, bit);
-          });
-      __syncthreads();
+          },
+          p.big ? q.sq + 8 * p.qh : 0u, scnt + 12);
       n_in = lds32(scnt + slot);
       slot = nslot;
       ++level;
@@ -411,9 +412,13 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   // A frontier beyond the halves continues in the global slab.
   const size_t blocks = std::min<size_t>((size_t)sh.minb, fit);
   const size_t budget = std::min<size_t>((size_t)per_sm / blocks, (size_t)optin) - slack;
-  const size_t room = budget > bitmap ? budget - bitmap : 0;
+  size_t room = budget > bitmap ? budget - bitmap : 0;
+  // Without edge records, room for long lists' pieces if some is left for the
+  // queue (ms: star of 100,000 leaves 15.3 -> 0.4, R-MAT 16 S=1 2.63 -> 1.39).
+  sh.big = !edge_records && room >= BIG_BYTES + 4096;
+  if (sh.big) room -= BIG_BYTES;
   sh.qh = (uint32_t)std::min<size_t>(CTA_SMEM_QUEUE, room / (2 * entry) / 32 * 32);
-  sh.smem = bitmap + 2 * (size_t)sh.qh * entry;
+  sh.smem = bitmap + 2 * (size_t)sh.qh * entry + (sh.big ? BIG_BYTES : 0);
   void* fn = cta_kernel(sh);
   int occ = 0;
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
@@ -443,6 +448,7 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
 void launch_cta(const CtaParams& params, const CtaShape& sh, int grid, cudaStream_t s) {
   CtaParams p = params;
   p.qh = sh.qh;  // the dynamic shared memory holds exactly these queue halves
+  p.big = sh.big;
   if (!sh.edge_records) p.erec = nullptr;
   if (sh.cluster > 1) {
     // grid: blocks, a multiple of the cluster size (checked by the caller)

@@ -224,6 +224,7 @@ struct CtaParams {
   uint32_t* work;        // source cursor (zeroed before launch)
   SourceStats* stats;    // non-null: per-source reductions instead of rows
   uint32_t* gbits;       // global-bitmap mode: per resident block ceil(V/32) u32
+  uint32_t big;          // long lists' pieces sit after the queue halves (set at launch)
   uint32_t qh;           // frontier entries per shared-memory queue half (set at launch)
   const uint2* erec;     // per edge {target, target's edge begin << 4 | count}, or null
 };
@@ -236,6 +237,7 @@ struct CtaShape {
   int minb = 1;           // resident blocks per SM the queue halves leave room for
   bool global_bits = false;
   bool edge_records = false;
+  bool big = false;       // room for long lists' pieces after the queue halves
   int cluster = 0;        // > 1: blocks per cluster sharing one source's bitmap
 };
 // Max V for the shared-memory visited bitmap; launch shape of the CTA kernel

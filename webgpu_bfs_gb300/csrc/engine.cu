@@ -65,6 +65,7 @@ struct msbfs_graph {
   uint32_t split = 0, heavy = 0;  // as asked for (the tables may use shorter slices)
   uint32_t n_heavy = 0;   // vertices of several slices
   uint32_t n_slices = 0;
+  void* tables = nullptr;  // the allocation that holds the following three
   uint4* slices = nullptr;
   uint32_t* hslices = nullptr;
   // Bottom-up work order: vertices with 0 < in-degree < heavy, ascending ids.
@@ -764,9 +765,8 @@ int finish_call(msbfs_engine* eng, msbfs_stats* stats) {
 int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, uint32_t heavy) {
   const size_t V = g->V;
   const std::vector<uint32_t>& coff = g->h_coff;
-  cudaFree(g->slices);
-  cudaFree(g->hslices);
-  cudaFree(g->order);
+  cudaFree(g->tables);
+  g->tables = nullptr;
   g->slices = nullptr;
   g->hslices = nullptr;
   g->order = nullptr;
@@ -786,7 +786,9 @@ int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, ui
   while (len > 256 && (uint64_t)len * warps > g->E) len /= 2;
   // Heavy vertices by in-degree, descending (a counting sort; those beyond
   // its range keep their order in front).
-  constexpr uint32_t TOP = 1u << 16;
+  uint32_t max_in = 0;
+  for (size_t v = 0; v < V; ++v) max_in = std::max(max_in, coff[v + 1] - coff[v]);
+  const uint32_t TOP = std::min(max_in + 2, 1u << 16);
   std::vector<uint32_t> at(TOP + 1, 0), by_degree;
   auto degree_rank = [&](size_t v) { return TOP - 1 - std::min(coff[v + 1] - coff[v], TOP - 1); };
   heavy = std::max(heavy, 1u);
@@ -809,9 +811,9 @@ int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, ui
   }
   // First slices first: by the time a vertex's later slices run, the lanes
   // its first ones found are published, and they can stop at once.
-  std::vector<uint4> slices;
+  std::vector<uint4> table;  // slices, then the work order, then the slice counts
   for (uint32_t j = 0;; ++j) {
-    const size_t before = slices.size();
+    const size_t before = table.size();
     for (size_t i = 0; i < (j ? many : by_degree.size()); ++i) {
       const uint32_t v = by_degree[i], d = coff[v + 1] - coff[v];
       const uint64_t first = (uint64_t)j * len;
@@ -821,34 +823,35 @@ int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, ui
       }
       const uint32_t sb = coff[v] + (uint32_t)first;
       const uint32_t se = d - first > len ? sb + len : coff[v + 1];
-      slices.push_back(make_uint4(v, sb, se, h[i] | (j ? 0u : SLICE_FIRST)));
+      table.push_back(make_uint4(v, sb, se, h[i] | (j ? 0u : SLICE_FIRST)));
     }
-    if (slices.size() == before) break;
+    if (table.size() == before) break;
   }
-  g->n_slices = (uint32_t)slices.size();
+  g->n_slices = (uint32_t)table.size();
   // Bottom-up work list: the other vertices with in-edges, ascending ids
   // (neighbouring vertices share cache lines of the visited and frontier
   // rows; sorting them by in-degree within windows of 256 or 1,024 entries,
   // for groups of similar length, cost 8 and 10% on R-MAT scale 22, S=512).
   // Each entry carries the vertex and its in-edge range, so a bottom-up
   // step starts a vertex's scan one dependent load earlier.
-  std::vector<uint4> order;
-  order.reserve(V);
+  table.reserve(table.size() + V + per_vertex.size() / 4 + 1);
   for (size_t v = 0; v < V; ++v) {
     const uint32_t b = coff[v], e = coff[v + 1];
-    if (e > b && e - b < heavy) order.push_back(make_uint4((uint32_t)v, b, e, 0u));
+    if (e > b && e - b < heavy) table.push_back(make_uint4((uint32_t)v, b, e, 0u));
   }
-  g->n_order = (uint32_t)order.size();
-  auto upload = [&](const void* src, size_t bytes, void** dst) -> int {
-    CK(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
-    if (bytes) CK(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
-    return MSBFS_OK;
-  };
-  int rc;
-  if ((rc = upload(slices.data(), slices.size() * sizeof(uint4), (void**)&g->slices)) ||
-      (rc = upload(per_vertex.data(), per_vertex.size() * sizeof(uint32_t), (void**)&g->hslices)) ||
-      (rc = upload(order.data(), order.size() * sizeof(uint4), (void**)&g->order)))
-    return rc;
+  const size_t counts = table.size();
+  g->n_order = (uint32_t)(counts - g->n_slices);
+  for (size_t i = 0; i < per_vertex.size(); i += 4) {
+    uint32_t c[4] = {};
+    for (size_t k = i; k < std::min(i + 4, per_vertex.size()); ++k) c[k - i] = per_vertex[k];
+    table.push_back(make_uint4(c[0], c[1], c[2], c[3]));
+  }
+  const size_t bytes = table.size() * sizeof(uint4);
+  CK(cudaMalloc(&g->tables, std::max<size_t>(bytes, 16)));
+  if (bytes) CK(cudaMemcpy(g->tables, table.data(), bytes, cudaMemcpyHostToDevice));
+  g->slices = static_cast<uint4*>(g->tables);
+  g->order = g->slices + g->n_slices;
+  g->hslices = reinterpret_cast<uint32_t*>(g->slices + counts);
   return MSBFS_OK;
 }
 
@@ -921,9 +924,7 @@ void free_graph(msbfs_graph* g) {
   }
   cudaFree(g->off);
   cudaFree(g->idx);
-  cudaFree(g->slices);
-  cudaFree(g->hslices);
-  cudaFree(g->order);
+  cudaFree(g->tables);
   cudaFree(g->erec);
   delete g;
 }
