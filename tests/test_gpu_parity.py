@@ -524,3 +524,25 @@ def test_level_records_of_both_forms_agree(native):
         assert {r[1] for r in logs[0]} == {0, 1}
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("kind,S", [("mid", 1), ("mid", 70), ("mid", 300), ("few", 70), ("long", 5)])
+def test_bottom_up_list_lengths(native, gpu_engine, oracle, kind, S):
+    """In-degrees on both sides of the lengths from which a whole warp scans a
+    list (64 where many vertices have 32 to 63 in-edges, else 32), and a graph
+    large enough for slices of 1,024."""
+    if kind == "long":
+        g = native.generate_graph500_rmat(19, 16, 12)
+    else:
+        degrees = (31, 32, 63, 64) if kind == "mid" else (5, 31, 32, 63, 64, 5, 5, 5)
+        V = 60000
+        hops = np.random.default_rng(5).permutation(V - 1)[:64] + 1
+        edges = []
+        for r, d in enumerate(degrees):
+            v = np.arange(r, V, len(degrees))
+            edges.append(np.stack([(v[:, None] + hops[:d]) % V, np.repeat(v[:, None], d, 1)], 2).reshape(-1, 2))
+        g = native.CsrGraph.from_edge_list(V, np.concatenate(edges))
+    src = native.sample_sources(g, S, 3, min_degree=1)
+    got = gpu_engine.run_ms_bfs_with_method(native.GpuBfsMethod.PushPullAdaptive, g, src)
+    want = oracle.ms_bfs_threaded(g.num_vertices, g.row_offsets, g.col_indices, src)
+    assert_same(got, want, g, src, f"{kind} S={S}")

@@ -144,13 +144,15 @@ struct msbfs_engine {
   uint32_t beta = 24;
   uint32_t seg = MSBFS_PUSH_SEG;  // out-edges per top-down queue entry
 #ifndef MSBFS_HEAVY
-#define MSBFS_HEAVY 32
+#define MSBFS_HEAVY 0
 #endif
-  uint32_t heavy = MSBFS_HEAVY;  // in-degree from which a whole warp scans a vertex
+  // In-degree from which a whole warp scans a vertex (0: warp_scan_degree).
+  uint32_t heavy = MSBFS_HEAVY;
 #ifndef MSBFS_SPLIT
-// At 8 resident level blocks per SM (R-MAT scale 22, S=512, 2 tiles per
-// claim): 512 8.59 ms per step, 384 8.73, 640 8.53, 1,024 9.67, 256 9.41.
-#define MSBFS_SPLIT 512
+// ms of a traversal with slices of at most 512 / 1,024 / 2,048 (in-degree 64
+// on): R-MAT 22 S=512 4.94 / 4.81 / 4.77, S=64 1.70 / 1.57 / 1.55; R-MAT 21 S=64
+// statistics 0.981 / 0.889 / 0.895. Smaller graphs get shorter ones.
+#define MSBFS_SPLIT 1024
 #endif
   uint32_t split = MSBFS_SPLIT;  // in-edge slice length of bottom-up steps
   uint32_t bits_div = 64;
@@ -757,6 +759,25 @@ int finish_call(msbfs_engine* eng, msbfs_stats* stats) {
   return MSBFS_OK;
 }
 
+// From which in-degree a whole warp scans a vertex: 64 on graphs with at least
+// 3 vertices of in-degree 32-63 per resident warp, else 32. Such a list fills
+// one or two rounds of a warp, each as long as the latency of its dependent
+// loads; vertices side by side in a tile share that latency, but a tile lasts
+// as long as its longest list, which only evens out over many. ms of a
+// traversal with 32 / 64 (vertices per warp): Erdos-Renyi of degree 40, 1 M
+// vertices, S=512 (125) 3.80 / 2.32, S=64 2.18 / 1.17; of degree 32, 400 K, S=64
+// (29) 0.650 / 0.469; of degree 24, 400 K, S=512 (3.7) 0.824 / 0.774; R-MAT 20 S=1
+// (10) 0.277 / 0.244, R-MAT 20 of edge factor 32, S=512 (3.7) 1.63 / 1.59; below
+// the line R-MAT 18 S=512 (1.9) 0.515 / 0.553, R-MAT 20 of edge factor 8, S=64
+// (1.7) 0.421 / 0.467, R-MAT 13 S=200 (0.03) 0.110 / 0.133. Against 64, 128 is
+// 1-2% slower on R-MAT 21 and 22; 16 loses to 32 on R-MAT 20 and larger.
+uint32_t warp_scan_degree(const msbfs_engine* eng, const std::vector<uint32_t>& coff) {
+  constexpr size_t LEVEL_WARPS_PER_SM = 48;
+  size_t mid = 0;
+  for (size_t v = 0; v + 1 < coff.size(); ++v) mid += coff[v + 1] - coff[v] - 32 < 32;
+  return mid >= 3 * LEVEL_WARPS_PER_SM * (size_t)eng->num_sms ? 64 : 32;
+}
+
 // Slice table of the vertices of in-degree >= heavy and the bottom-up work
 // list of the other vertices with in-edges, from the graph's host CSC
 // offsets. Rebuilt when the autotuner changes the slice length or the
@@ -765,6 +786,7 @@ int finish_call(msbfs_engine* eng, msbfs_stats* stats) {
 int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, uint32_t heavy) {
   const size_t V = g->V;
   const std::vector<uint32_t>& coff = g->h_coff;
+  if (!heavy) heavy = warp_scan_degree(eng, coff);
   cudaFree(g->tables);
   g->tables = nullptr;
   g->slices = nullptr;
