@@ -148,7 +148,9 @@ const char *msbfs_engine_last_error(const msbfs_engine *engine);
 int msbfs_engine_set_stream(msbfs_engine *engine, void *cuda_stream);
 /* Tuning knobs of the level-synchronous path (no reference counterpart; the
  * reference hard-codes alpha=14/beta=24 in push_pull.rs:29-36 and 512-source
- * chunks in multi_word_bp.rs:630). Zero keeps the current value. */
+ * chunks in multi_word_bp.rs:630). Zero keeps the current value. A new engine
+ * takes passes of up to 64 words (2,048 sources) while their state stays
+ * within an eighth of the device memory, and of 16 words otherwise. */
 int msbfs_engine_set_tuning(msbfs_engine *engine, uint32_t max_words_per_pass,
                             uint32_t alpha, uint32_t beta);
 /* Autotuner of the level-synchronous path. No single reference
@@ -205,10 +207,9 @@ int msbfs_engine_set_sm_share(msbfs_engine *engine, uint32_t percent);
 int msbfs_engine_set_level_cap(msbfs_engine *engine, uint32_t max_levels);
 
 /* Profiling: 0 off; 1 keep a per-level record of every call (device timers
- * and the work counters of the algorithmic-bytes model; the level loop stays
- * on the device and runs the level kernels' counting form); 2 as 1, but the
- * level loop is driven from the host one launch at a time with CUDA events
- * around each launch; 3 as 2 with the production level kernels, which keep
+ * and the work counters of the algorithmic-bytes model; the level loop is
+ * driven from the host, one launch of the level kernels' counting form a
+ * level); 2 as 1, with CUDA events around each launch; 3 as 2 with the production level kernels, which keep
  * no work counters (the records carry durations, frontier sizes and
  * discovered pairs only). msbfs_engine_level_log copies the last call's
  * records. */
