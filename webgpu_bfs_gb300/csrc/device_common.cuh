@@ -116,6 +116,11 @@ struct PassDesc {
 struct GridSync {
   uint32_t arrive;            // blocks that have arrived
   alignas(128) uint32_t gen;  // barriers passed
+  // Set for good by a block that gave up waiting: `arrive` and the frontier
+  // state are then no base for another level, so blocks stop at their next
+  // barrier, those of the passes queued behind at their first, until the host
+  // drops the workspace. (Beside gen: one load reads both.)
+  uint32_t stuck;
 };
 
 struct LevelParams {
@@ -137,6 +142,8 @@ struct LevelParams {
   LevelRec* log;      // LOG_CAP records
   PassDesc d;
   GridSync* sync;
+  uint32_t spins;     // polls of a grid barrier before a block gives up
+  uint32_t* h_stuck;  // the engine's word of host memory that it then sets
   uint32_t epoch;     // stamp of level 0 of this pass
   uint32_t NP;        // planes allocated
   uint32_t qcap;      // entries per queue slot (slots 1, 2)

@@ -170,6 +170,10 @@ struct msbfs_engine {
   uint32_t mat_waves = MSBFS_MAT_WAVES;
   uint32_t level_cap = 0;   // levels per pass before MSBFS_ERR_TIMEOUT (0: V + 2)
   bool host_loop = false;
+  // Polls of a grid barrier before the traversal gives up (tens of seconds;
+  // MSBFS_BARRIER_SPINS), and the word that it then sets (page-locked).
+  uint32_t barrier_spins = 1u << 26;
+  uint32_t* h_stuck = nullptr;
   bool zero_copy = true;  // MSBFS_ZERO_COPY=0 stages host output in HBM instead
   bool narrow = true;     // MSBFS_NARROW=0 keeps host-bound rows u32 over the link
   int profiling = 0;
@@ -278,6 +282,10 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   }
   // One pooled workspace per graph: drop any other (W, mode) of this graph
   // only if memory runs short (allocation failure below retries once).
+  if (!eng->h_stuck) {
+    CK(cudaHostAlloc((void**)&eng->h_stuck, sizeof(uint32_t), cudaHostAllocMapped));
+    *eng->h_stuck = 0;
+  }
   auto w = std::make_unique<Workspace>();
   w->graph_id = g->id;
   w->W = W;
@@ -356,6 +364,8 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   p.ctl = w->d_ctl;
   if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(GridSync)))) return rc;
   p.sync = (GridSync*)ptr;
+  p.spins = eng->barrier_spins;
+  CK(cudaHostGetDevicePointer((void**)&p.h_stuck, eng->h_stuck, 0));
   if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(LevelRec) * LOG_CAP))) return rc;
   w->d_log = (LevelRec*)ptr;
   p.log = w->d_log;
@@ -749,9 +759,12 @@ int finish_call(msbfs_engine* eng, msbfs_stats* stats) {
   if (status & STATUS_CHECK)
     return set_err(eng, MSBFS_ERR_CUDA,
                    "bounds check failed at site " + std::to_string(check_site));
-  if (status & STATUS_STUCK) {
+  // Also when it was an earlier asynchronous call that got stuck: its rows are
+  // void, and the calls queued behind it on the same workspace did nothing.
+  if ((status & STATUS_STUCK) || (eng->h_stuck && *(volatile uint32_t*)eng->h_stuck)) {
     CK(cudaStreamSynchronize(eng->stream));
     eng->ws.clear();  // the pass left its traversal state as it was
+    *eng->h_stuck = 0;
     return set_err(eng, MSBFS_ERR_TIMEOUT, "a level's grid barrier ran out of time");
   }
   if (status & STATUS_LEVEL_CAP) return set_err(eng, MSBFS_ERR_TIMEOUT, "level cap reached");
@@ -1189,6 +1202,8 @@ int msbfs_engine_create(int device, int method, msbfs_engine** out) {
   int coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
   e->host_loop = !coop || (hl && hl[0] == '1');
+  const char* bs = getenv("MSBFS_BARRIER_SPINS");
+  if (bs) e->barrier_spins = (uint32_t)std::max(1, atoi(bs));
   const char* zc = getenv("MSBFS_ZERO_COPY");
   e->zero_copy = !(zc && zc[0] == '0');
   const char* nr = getenv("MSBFS_NARROW");
@@ -1221,6 +1236,7 @@ void msbfs_engine_destroy(msbfs_engine* e) {
   cudaFree(e->d_sstats);
   if (e->h_ctl) cudaFreeHost(e->h_ctl);
   if (e->h_log) cudaFreeHost(e->h_log);
+  if (e->h_stuck) cudaFreeHost(e->h_stuck);
   for (cudaEvent_t ev : e->lvl_events) cudaEventDestroy(ev);
   cudaEventDestroy(e->ev_start);
   cudaEventDestroy(e->ev_stop);

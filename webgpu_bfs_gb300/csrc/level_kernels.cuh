@@ -942,6 +942,13 @@ __device__ __forceinline__ void init_sources(const LevelParams& p) {
 
 template <int W>
 __global__ void init_kernel(const __grid_constant__ LevelParams p) {
+  if (__ldcg(&p.sync->stuck)) {  // nothing for the level kernels to do
+    if (threadIdx.x == 0) {
+      p.ctl->status = STATUS_STUCK;
+      p.ctl->terminated = 1;
+    }
+    return;
+  }
   init_sources<W>(p);
 }
 
@@ -1069,9 +1076,10 @@ __global__ void __launch_bounds__(LEVEL_BLOCK) queue_kernel(const __grid_constan
 
 // Grid barrier of the traversal kernel between levels, with the controller
 // run by the last block to arrive. Only valid in a cooperative launch (every
-// block resident). The wait is bounded: a block that gives up flags
-// STATUS_STUCK and returns false.
-constexpr uint32_t BARRIER_SPINS = 1u << 26;  // tens of seconds
+// block resident). The wait is bounded: a block that gives up flags the pass,
+// the workspace and the engine (STATUS_STUCK, GridSync::stuck, h_stuck) and
+// returns false; blocks that come to a barrier of a stuck workspace do not
+// arrive, so it opens no more.
 template <int W, typename Last>
 __device__ __forceinline__ bool level_barrier(const LevelParams& p, LevelShared<W>& sh,
                                               Last&& last_block) {
@@ -1079,13 +1087,15 @@ __device__ __forceinline__ bool level_barrier(const LevelParams& p, LevelShared<
   if (threadIdx.x < 32) {
     GridSync* g = p.sync;
     uint32_t gen = 0, last = 0;
+    bool ok = true;
     if (threadIdx.x == 0) {
-      gen = __ldcg(&g->gen);  // cannot advance before this block arrives
+      const uint2 s = __ldcg(reinterpret_cast<const uint2*>(&g->gen));
+      gen = s.x;  // cannot advance before this block arrives
+      ok = s.y == 0;
       __threadfence();
-      last = atomicAdd(&g->arrive, 1u) == gridDim.x - 1;
+      if (ok) last = atomicAdd(&g->arrive, 1u) == gridDim.x - 1;
     }
     last = __shfl_sync(FULL, last, 0);
-    bool ok = true;
     if (last) {
       __threadfence();
       last_block();
@@ -1097,11 +1107,14 @@ __device__ __forceinline__ bool level_barrier(const LevelParams& p, LevelShared<
       }
     } else if (threadIdx.x == 0) {
       uint32_t now = gen, spins = 0;
-      do {
+      if (ok) do {
         asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(&g->gen) : "memory");
-      } while (now == gen && ++spins < BARRIER_SPINS);
+      } while (now == gen && ++spins < p.spins);
       if (now == gen) {
         atomicOr(&p.ctl->status, STATUS_STUCK);
+        atomicOr(&g->stuck, 1u);
+        *(volatile uint32_t*)p.h_stuck = 1;
+        __threadfence_system();
         ok = false;
       }
     }
