@@ -275,6 +275,10 @@ __device__ void bp_item(const BatchGraph& g, uint32_t s0, uint32_t P, uint32_t* 
 // Single-source items: frontier entries per shared-memory queue half.
 constexpr uint32_t BATCH_QH = 2048;
 constexpr size_t BATCH_ITEM_SMEM = 2 * BATCH_QH * sizeof(uint32_t) + BIG_BYTES;
+// Dynamic shared memory of a block, for graphs of at most V vertices: the
+// bitmap, then a single-source item's queue halves and pieces (a bit-parallel
+// item uses the bitmap only).
+constexpr size_t batch_smem(size_t V) { return ((V + 31) / 32 + 1) / 2 * 8 + BATCH_ITEM_SMEM; }
 
 // One single-source BFS per source of [s0, s0+n); visited bitmap and queue
 // halves in shared memory, the rest of the queue (V words) in the block's
@@ -586,13 +590,12 @@ int msbfs_batch_create(int device, const msbfs_batch_graph* graphs, size_t n, ms
   // Scratch per resident block: the larger of ALG_BP (3*V*8 words + 2V) and
   // ALG_CTA (2V) for the largest graph.
   b->scratch_words = 3 * maxVW * 8 + 2 * maxVW + 64;
-  // Shared memory: the bitmap, then a single-source item's queue halves and
-  // pieces (a bit-parallel item uses the bitmap only).
-  b->smem = ((b->max_V + 31) / 32 + 1) / 2 * 8 + BATCH_ITEM_SMEM;
-  BCK(cudaFuncSetAttribute(batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)std::max<size_t>(b->smem, 4)));
-  BCK(cudaFuncSetAttribute(batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)std::max<size_t>(b->smem, 4)));
+  b->smem = batch_smem(b->max_V);
+  // A kernel has one limit in the whole process, so it is the largest batch's,
+  // whichever batches are alive.
+  constexpr int SMEM_MAX = (int)batch_smem(MSBFS_BATCH_MAX_VERTICES);
+  BCK(cudaFuncSetAttribute(batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+  BCK(cudaFuncSetAttribute(batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
   int occ = 0, occ_vt = 0, sms = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, BATCH_BLOCK, b->smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_vt, batch_kernel<true>, BATCH_BLOCK, b->smem);
