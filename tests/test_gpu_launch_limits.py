@@ -1,6 +1,8 @@
 """Launches whose shared-memory limits another object of the process also
 sets (GPU): the limit belongs to the kernel, so objects of different size
 must not take it from one another."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -31,3 +33,38 @@ def test_batches_of_different_size_alive_at_once(native, tmp_path, alg):
     finally:
         small.close()
         big.close()
+
+def test_cta_calls_of_different_size_from_two_threads(native):
+    """One-source calls on a tree of 40,000 vertices (seven levels, so many
+    calls) and on a 1,000 x 1,200 grid, each from a thread with an engine of
+    its own: one kernel, with 37 KB and 183 KB of shared memory."""
+    n = 40_000
+    v = np.arange(1, n)
+    up = np.stack([v, (v - 1) // 7], 1)
+    tree = native.CsrGraph.from_edge_list(n, np.concatenate([up, up[:, ::-1]]))
+    w, h = 1000, 1200
+    grid = native.Grid2D(w, h).graph
+    done = threading.Event()
+    failures = []
+
+    def serve(g, calls, ecc):
+        eng = native.GpuBfsEngine(native.GpuBfsMethod.WorkgroupPersistentBfs)
+        try:
+            for _ in range(calls):
+                st = eng.run_ms_bfs_stats(g, [0])[0]
+                assert st["reached"] == g.num_vertices and st["eccentricity"] == ecc
+                if done.is_set():
+                    break
+        except Exception as e:
+            failures.append(f"V={g.num_vertices}: {e}")
+        finally:
+            eng.close()
+
+    small = [threading.Thread(target=serve, args=(tree, 10 ** 9, 6)) for _ in range(2)]
+    for t in small:
+        t.start()
+    serve(grid, 400, w + h - 2)
+    done.set()
+    for t in small:
+        t.join()
+    assert not failures, failures

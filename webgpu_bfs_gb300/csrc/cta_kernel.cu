@@ -270,12 +270,21 @@ void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, u
   edge_records_kernel<<<1024, 256, 0, s>>>(V, off, idx, erec);
 }
 
+constexpr size_t CTA_SMEM_RESERVE = 1024;  // static shared variables and slack
+
 size_t cta_max_vertices(int device) {
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  const size_t reserve = 1024;  // static shared variables and slack
-  if (optin <= (int)reserve) return 0;
-  return ((size_t)optin - reserve) * 8;
+  if (optin <= (int)CTA_SMEM_RESERVE) return 0;
+  return ((size_t)optin - CTA_SMEM_RESERVE) * 8;
+}
+
+// Lets launches of the kernel take all the dynamic shared memory a block can
+// have. The limit belongs to the kernel, which calls of other sizes launch from
+// other threads: set to each call's size, one call could lower it under another.
+static cudaError_t allow_smem(void* fn, int optin) {
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              optin - (int)CTA_SMEM_RESERVE);
 }
 
 template <bool GB, bool ER>
@@ -310,11 +319,10 @@ static void* cluster_kernel(int cl, bool er) {
 
 // Clusters that can be resident at once for a cluster launch of `cl` blocks
 // with `smem` bytes of dynamic shared memory each (0 if it cannot launch).
-static int cluster_capacity(int cl, bool er, size_t smem, int block) {
+static int cluster_capacity(int cl, bool er, size_t smem, int block, int optin) {
   void* fn = cluster_kernel(cl, er);
   if (!fn) return 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess) {
+  if (allow_smem(fn, optin) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -359,7 +367,7 @@ static bool cta_cluster_shape(uint32_t V, int sms, int optin, bool edge_records,
     sh.cluster = cl;
     sh.qh = (uint32_t)std::min<size_t>(CTA_SMEM_QUEUE, room / (2 * entry) / 32 * 32);
     sh.smem = slice + 2 * (size_t)sh.qh * entry;
-    const int n = cluster_capacity(cl, edge_records, sh.smem, sh.block);
+    const int n = cluster_capacity(cl, edge_records, sh.smem, sh.block, optin);
     if (n < 1) continue;
     // A cluster traverses a source faster than a global-bitmap block, but a
     // global-bitmap launch keeps several blocks per SM busy: clusters pay
@@ -421,7 +429,7 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   sh.smem = bitmap + 2 * (size_t)sh.qh * entry + (sh.big ? BIG_BYTES : 0);
   void* fn = cta_kernel(sh);
   int occ = 0;
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+  if (allow_smem(fn, optin) != cudaSuccess) cudaGetLastError();
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, sh.block, sh.smem);
   if (occ < 1) return false;
   sh.grid = sms * occ;
