@@ -150,7 +150,8 @@ int msbfs_engine_set_stream(msbfs_engine *engine, void *cuda_stream);
  * reference hard-codes alpha=14/beta=24 in push_pull.rs:29-36 and 512-source
  * chunks in multi_word_bp.rs:630). Zero keeps the current value. A new engine
  * takes passes of up to 64 words (2,048 sources) while their state stays
- * within an eighth of the device memory, and of 16 words otherwise. */
+ * within an eighth of the device memory and half of what is free, and narrower
+ * ones, down to 16 words, otherwise or when an allocation fails. */
 int msbfs_engine_set_tuning(msbfs_engine *engine, uint32_t max_words_per_pass,
                             uint32_t alpha, uint32_t beta);
 /* Autotuner of the level-synchronous path. No single reference

@@ -81,6 +81,7 @@ namespace {
 struct Workspace {
   uint64_t graph_id = 0;
   uint32_t W = 0;
+  uint64_t wide_bytes = 0;  // state_bytes of its graph and width
   uint32_t mode = 0;
   bool count = false;  // level kernels keep the profiling counters
   LevelParams p{};
@@ -138,8 +139,8 @@ struct msbfs_engine {
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr, ev_pass = nullptr, ev_copies = nullptr;
   std::mutex mu;
   std::string last_error;
-  uint32_t max_words = 0;   // words per vertex of a pass at most (0: widest_pass)
-  size_t total_mem = 0;     // device memory, once a call may want a wide pass
+  uint32_t max_words = 0;   // words per vertex of a pass at most (0: choose_words)
+  size_t total_mem = 0;     // device memory, once a call wanted a wide pass
   uint32_t alpha = 14;
   uint32_t beta = 24;
   uint32_t seg = MSBFS_PUSH_SEG;  // out-edges per top-down queue entry
@@ -238,6 +239,20 @@ int cuda_fail(msbfs_engine* e, cudaError_t err, const char* what) {
     if (_e != cudaSuccess) return cuda_fail(eng, _e, #call); \
   } while (0)
 
+// cudaMalloc that gives the engine's pooled workspaces back when the device is
+// out of memory, and tries once more.
+cudaError_t device_alloc(msbfs_engine* eng, void** ptr, size_t bytes) {
+  cudaError_t err = cudaMalloc(ptr, bytes);
+  if (err != cudaErrorMemoryAllocation || eng->ws.empty()) return err;
+  cudaGetLastError();
+  // Earlier asynchronous calls may still run on them.
+  if ((err = cudaStreamSynchronize(eng->stream)) != cudaSuccess ||
+      (err = cudaStreamSynchronize(eng->copy_stream)) != cudaSuccess)
+    return err;
+  eng->ws.clear();
+  return cudaMalloc(ptr, bytes);
+}
+
 template <typename T>
 int grow(msbfs_engine* eng, T** ptr, size_t* cap, size_t need) {
   if (need <= *cap && *ptr) return MSBFS_OK;
@@ -250,14 +265,14 @@ int grow(msbfs_engine* eng, T** ptr, size_t* cap, size_t need) {
   *ptr = nullptr;
   *cap = 0;
   size_t n = std::max(need, (size_t)1);
-  CK(cudaMalloc((void**)ptr, n * sizeof(T)));
+  CK(device_alloc(eng, (void**)ptr, n * sizeof(T)));
   *cap = n;
   return MSBFS_OK;
 }
 
 int dev_alloc(msbfs_engine* eng, Workspace* w, void** ptr, size_t bytes) {
   if (bytes == 0) bytes = 16;
-  CK(cudaMalloc(ptr, bytes));
+  CK(device_alloc(eng, ptr, bytes));
   w->allocs.push_back(*ptr);
   CK(cudaMemsetAsync(*ptr, 0, bytes, eng->stream));
   return MSBFS_OK;
@@ -265,6 +280,29 @@ int dev_alloc(msbfs_engine* eng, Workspace* w, void** ptr, size_t bytes) {
 
 uint32_t level_planes(const msbfs_graph* g) {
   return std::min<uint32_t>(bit_length_u64(g->V > 1 ? g->V - 1 : 1), 8);
+}
+
+// Traversal state of a pass of W words a vertex (the parts that grow with W).
+uint64_t state_bytes(const msbfs_graph* g, uint32_t W) {
+  return (uint64_t)g->V * W * 4 * (5 + level_planes(g));
+}
+
+// Passes above this width are taken for speed only, where memory allows.
+constexpr uint32_t PLAIN_WORDS = 16;
+
+// The default width above PLAIN_WORDS keeps the state of an engine's wide passes
+// within an eighth of the device memory, and takes at most half of what is free.
+bool wide_pass_fits(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t mode) {
+  const auto it = eng->ws.find(std::make_tuple(g->id, W, mode));
+  if (it != eng->ws.end() && !it->second->dirty) return true;
+  const uint64_t need = state_bytes(g, W);
+  if (eng->total_mem && need > eng->total_mem / 8) return false;
+  size_t free_mem = 0;
+  if (cudaMemGetInfo(&free_mem, &eng->total_mem) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return need <= eng->total_mem / 8 && need <= free_mem / 2;
 }
 
 int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t mode,
@@ -280,8 +318,19 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
     CK(cudaStreamSynchronize(eng->copy_stream));
     eng->ws.erase(it);
   }
-  // One pooled workspace per graph: drop any other (W, mode) of this graph
-  // only if memory runs short (allocation failure below retries once).
+  // Workspaces stay pooled until memory runs short (device_alloc); those of wide
+  // passes only while they fit the engine's share together.
+  if (W > PLAIN_WORDS && !eng->max_words) {
+    uint64_t wide = state_bytes(g, W);
+    for (auto& kv : eng->ws)
+      if (kv.second->W > PLAIN_WORDS) wide += kv.second->wide_bytes;
+    if (wide > eng->total_mem / 8) {
+      CK(cudaStreamSynchronize(eng->stream));
+      CK(cudaStreamSynchronize(eng->copy_stream));
+      for (auto o = eng->ws.begin(); o != eng->ws.end();)
+        o = o->second->W > PLAIN_WORDS ? eng->ws.erase(o) : std::next(o);
+    }
+  }
   if (!eng->h_stuck) {
     CK(cudaHostAlloc((void**)&eng->h_stuck, sizeof(uint32_t), cudaHostAllocMapped));
     *eng->h_stuck = 0;
@@ -289,6 +338,7 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   auto w = std::make_unique<Workspace>();
   w->graph_id = g->id;
   w->W = W;
+  w->wide_bytes = state_bytes(g, W);
   w->mode = mode;
   const uint32_t NP = level_planes(g);
   if (!level_kernel_info(W, NP, eng->num_sms, &w->k))
@@ -472,31 +522,31 @@ int run_pass_host_loop(msbfs_engine* eng, Workspace* w, bool reduce) {
   return MSBFS_OK;
 }
 
-// Words per vertex of the widest pass when the caller sets none. A pass costs
-// far less than twice one of half its width (the levels' latency and fixed
-// parts are shared, and a gathered row of 128 bytes costs little more than
-// one of 64). ms of a call at up to 16 / 32 / 64 words: Erdos-Renyi 100,000 x
-// 16, S=700 0.525 / 0.421 / -, S=2,048 1.125 / 0.893 / 0.705; R-MAT 20, S=513
-// 2.00 / 2.05 / -, S=2,048 5.99 / 4.92 / 4.38. Passes above 16 words keep
-// their traversal state within an eighth of the device memory.
 uint32_t widest_pass(msbfs_engine* eng, const msbfs_graph* g) {
   if (eng->max_words) return eng->max_words;
   if (size_t free_mem; !eng->total_mem && cudaMemGetInfo(&free_mem, &eng->total_mem) != cudaSuccess) {
     cudaGetLastError();
-    return 16;
+    return PLAIN_WORDS;
   }
   uint32_t W = 64;
-  while (W > 16 && (uint64_t)g->V * W * 4 * (5 + level_planes(g)) > eng->total_mem / 8) W >>= 1;
+  while (W > PLAIN_WORDS && state_bytes(g, W) > eng->total_mem / 8) W >>= 1;
   return W;
 }
 
-uint32_t choose_words(msbfs_engine* eng, const msbfs_graph* g, size_t S) {
-  const uint32_t widest = S > 512 || eng->max_words ? widest_pass(eng, g) : 16;
-  size_t lanes = std::min<size_t>(S, (size_t)widest * 32);
-  uint32_t need = (uint32_t)((lanes + 31) / 32);
+// Words per vertex of a call's passes: up to 64 by default. A pass costs far
+// less than twice one of half its width (the levels' latency and fixed parts
+// are shared, and a gathered row of 128 bytes costs little more than one of
+// 64). ms of a call at up to 16 / 32 / 64 words: Erdos-Renyi 100,000 x 16,
+// S=700 0.525 / 0.421 / -, S=2,048 1.125 / 0.893 / 0.705; R-MAT 20, S=513
+// 2.00 / 2.05 / -, S=2,048 5.99 / 4.92 / 4.38.
+uint32_t choose_words(msbfs_engine* eng, const msbfs_graph* g, size_t S, uint32_t mode) {
+  const uint32_t most = eng->max_words ? eng->max_words : 64;
+  const uint32_t need = (uint32_t)((std::min<size_t>(S, (size_t)most * 32) + 31) / 32);
   uint32_t W = 1;
   while (W < need) W <<= 1;
-  return std::min<uint32_t>(W, 64);
+  if (!eng->max_words)
+    while (W > PLAIN_WORDS && !wide_pass_fits(eng, g, W, mode)) W >>= 1;
+  return W;
 }
 
 int validate_call(msbfs_engine* eng, const msbfs_graph* g, const uint32_t* sources, size_t S) {
@@ -607,11 +657,14 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
   const uint32_t mode = path == MSBFS_PATH_PUSH   ? MODE_PUSH
                         : path == MSBFS_PATH_PULL ? MODE_PULL
                                                   : MODE_HYBRID;
-  const uint32_t W = choose_words(eng, g, S);
+  uint32_t W = choose_words(eng, g, S, mode);
+  Workspace* w = nullptr;
+  rc = get_workspace(eng, g, W, mode, &w);
+  while (rc == MSBFS_ERR_OOM && W > PLAIN_WORDS && !eng->max_words)
+    rc = get_workspace(eng, g, W >>= 1, mode, &w);
+  if (rc) return rc;
   const size_t PW = (size_t)W * 32;
   const size_t passes = (S + PW - 1) / PW;
-  Workspace* w = nullptr;
-  if ((rc = get_workspace(eng, g, W, mode, &w))) return rc;
   const bool reduce = stats_dev != nullptr;
   // Split materialisation (one-launch traversal only): the u32 rows follow
   // the byte rows in a second launch, while the host widens the bytes.
@@ -882,7 +935,7 @@ int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, ui
     table.push_back(make_uint4(c[0], c[1], c[2], c[3]));
   }
   const size_t bytes = table.size() * sizeof(uint4);
-  CK(cudaMalloc(&g->tables, std::max<size_t>(bytes, 16)));
+  CK(device_alloc(eng, &g->tables, std::max<size_t>(bytes, 16)));
   if (bytes) CK(cudaMemcpy(g->tables, table.data(), bytes, cudaMemcpyHostToDevice));
   g->slices = static_cast<uint4*>(g->tables);
   g->order = g->slices + g->n_slices;
@@ -908,16 +961,16 @@ int upload_graph(msbfs_engine* eng, size_t V, size_t E, const uint32_t* off, con
   g->sym = std::equal(t.off.begin(), t.off.end(), off) &&
            (E == 0 || std::memcmp(t.idx.data(), idx, E * 4) == 0);
   CK(cudaSetDevice(eng->device));
-  CK(cudaMalloc((void**)&g->off, (V + 1) * 4));
-  CK(cudaMalloc((void**)&g->idx, std::max<size_t>(E, 1) * 4));
+  CK(device_alloc(eng, (void**)&g->off, (V + 1) * 4));
+  CK(device_alloc(eng, (void**)&g->idx, std::max<size_t>(E, 1) * 4));
   CK(cudaMemcpy(g->off, off, (V + 1) * 4, cudaMemcpyHostToDevice));
   if (E) CK(cudaMemcpy(g->idx, idx, E * 4, cudaMemcpyHostToDevice));
   if (g->sym) {
     g->coff = g->off;
     g->cidx = g->idx;
   } else {
-    CK(cudaMalloc((void**)&g->coff, (V + 1) * 4));
-    CK(cudaMalloc((void**)&g->cidx, std::max<size_t>(E, 1) * 4));
+    CK(device_alloc(eng, (void**)&g->coff, (V + 1) * 4));
+    CK(device_alloc(eng, (void**)&g->cidx, std::max<size_t>(E, 1) * 4));
     CK(cudaMemcpy(g->coff, t.off.data(), (V + 1) * 4, cudaMemcpyHostToDevice));
     if (E) CK(cudaMemcpy(g->cidx, t.idx.data(), E * 4, cudaMemcpyHostToDevice));
   }
@@ -929,7 +982,7 @@ int upload_graph(msbfs_engine* eng, size_t V, size_t E, const uint32_t* off, con
   // round trip instead of three. The packed edge range holds 28 bits of edge
   // index and at most 15 out-edges (road-like: at most 8).
   if (is_road_like(g.get()) && E > 0 && E < (size_t(1) << 28)) {
-    CK(cudaMalloc((void**)&g->erec, E * sizeof(uint2)));
+    CK(device_alloc(eng, (void**)&g->erec, E * sizeof(uint2)));
     launch_edge_records((uint32_t)V, g->off, g->idx, g->erec, eng->stream);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(eng->stream));
