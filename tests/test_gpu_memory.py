@@ -75,3 +75,25 @@ def test_wide_state_is_given_back_to_later_calls(native, torch, mesh):
                               want["distance_sum"][:600])
     finally:
         eng.close()
+
+
+def test_tuning_a_small_graph_keeps_the_rule_for_large_ones(native, torch):
+    """A graph whose state at 64 words is just beyond an eighth of the device
+    memory: 32 words, also on an engine that was tuned on a small graph."""
+    total = torch.cuda.mem_get_info()[1]
+    V = int(total / 8 / (64 * 4 * 13) * 1.05)
+    ring = np.arange(1000, dtype=np.int64)
+    big = native.CsrGraph.from_edge_list(
+        V, np.concatenate([np.stack([ring, (ring + k) % 1000], 1) for k in range(1, 12)]))
+    small = native.generate_graph500_rmat(12, 8, 3)
+    src = np.arange(2048, dtype=np.uint32) % 1000
+    for tuned in (False, True):
+        eng = native.GpuBfsEngine(native.GpuBfsMethod.PushPullAdaptive)
+        try:
+            if tuned:
+                eng.autotune(small, native.sample_sources(small, 1, 2, min_degree=1))
+            st = eng.run_ms_bfs_stats(big, src)
+            assert (st["reached"] == 1000).all()
+            assert eng.last_stats["words_per_vertex"] == 32, tuned
+        finally:
+            eng.close()

@@ -546,3 +546,20 @@ def test_bottom_up_list_lengths(native, gpu_engine, oracle, kind, S):
     got = gpu_engine.run_ms_bfs_with_method(native.GpuBfsMethod.PushPullAdaptive, g, src)
     want = oracle.ms_bfs_threaded(g.num_vertices, g.row_offsets, g.col_indices, src)
     assert_same(got, want, g, src, f"{kind} S={S}")
+
+
+def test_tuning_one_graph_keeps_the_table_rule_for_others(native, tmp_path):
+    """The in-degree from which whole warps scan a list is each graph's own: 16,
+    tuned for one graph, is not what a graph uploaded later gets (32, by the rule)."""
+    g = native.generate_graph500_rmat(10, 8, 5)
+    src = native.sample_sources(g, 1, 1, min_degree=1)
+    road = native.wilson_grid(20, 20, 10, 2)
+    eng = native.GpuBfsEngine(native.GpuBfsMethod.Auto)
+    try:
+        cache = tmp_path / "tuning.txt"
+        name = eng.autotune(g, src)["class_name"]
+        cache.write_text(f"{name} 1 14 24 512 64 16 1.0\n")
+        assert eng.autotune(g, src, cache_path=str(cache))["warp_scan_degree"] == 16
+        assert eng.autotune(road, src)["warp_scan_degree"] == 32
+    finally:
+        eng.close()

@@ -62,7 +62,8 @@ struct msbfs_graph {
   uint32_t* cidx = nullptr;
   // Bottom-up steps: in-edge lists of `heavy` and more are scanned by whole
   // warps, in slices of at most `split`.
-  uint32_t split = 0, heavy = 0;  // as asked for (the tables may use shorter slices)
+  uint32_t split = 0, heavy = 0;  // as asked for (the tables may use shorter slices; heavy 0: by the rule)
+  uint32_t scan_degree = 0;       // `heavy` in use
   uint32_t n_heavy = 0;   // vertices of several slices
   uint32_t n_slices = 0;
   void* tables = nullptr;  // the allocation that holds the following three
@@ -125,6 +126,10 @@ uint32_t method_path(int m) {
     default:
       return MSBFS_PATH_HYBRID;
   }
+}
+
+uint32_t path_mode(uint32_t path) {
+  return path == MSBFS_PATH_PUSH ? MODE_PUSH : path == MSBFS_PATH_PULL ? MODE_PULL : MODE_HYBRID;
 }
 
 }  // namespace
@@ -522,17 +527,6 @@ int run_pass_host_loop(msbfs_engine* eng, Workspace* w, bool reduce) {
   return MSBFS_OK;
 }
 
-uint32_t widest_pass(msbfs_engine* eng, const msbfs_graph* g) {
-  if (eng->max_words) return eng->max_words;
-  if (size_t free_mem; !eng->total_mem && cudaMemGetInfo(&free_mem, &eng->total_mem) != cudaSuccess) {
-    cudaGetLastError();
-    return PLAIN_WORDS;
-  }
-  uint32_t W = 64;
-  while (W > PLAIN_WORDS && state_bytes(g, W) > eng->total_mem / 8) W >>= 1;
-  return W;
-}
-
 // Words per vertex of a call's passes: up to 64 by default. A pass costs far
 // less than twice one of half its width (the levels' latency and fixed parts
 // are shared, and a gathered row of 128 bytes costs little more than one of
@@ -654,9 +648,7 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
     return MSBFS_OK;
   }
 
-  const uint32_t mode = path == MSBFS_PATH_PUSH   ? MODE_PUSH
-                        : path == MSBFS_PATH_PULL ? MODE_PULL
-                                                  : MODE_HYBRID;
+  const uint32_t mode = path_mode(path);
   uint32_t W = choose_words(eng, g, S, mode);
   Workspace* w = nullptr;
   rc = get_workspace(eng, g, W, mode, &w);
@@ -852,14 +844,15 @@ uint32_t warp_scan_degree(const msbfs_engine* eng, const std::vector<uint32_t>& 
 int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, uint32_t heavy) {
   const size_t V = g->V;
   const std::vector<uint32_t>& coff = g->h_coff;
+  g->heavy = heavy;
   if (!heavy) heavy = warp_scan_degree(eng, coff);
+  g->scan_degree = heavy;
   cudaFree(g->tables);
   g->tables = nullptr;
   g->slices = nullptr;
   g->hslices = nullptr;
   g->order = nullptr;
   g->split = split;
-  g->heavy = heavy;
   g->n_heavy = 0;
   // A slice is one warp's serial work. With less than a full slice of edges
   // per resident warp, shorter ones: a level of a small graph lasts as long
@@ -1570,7 +1563,9 @@ int msbfs_traversed_edges_device(msbfs_engine* e, const msbfs_graph* g, const ui
 
 namespace {
 
-// Settings of the level-synchronous path that the autotuner varies.
+// Settings of the level-synchronous path that the autotuner varies. Words and
+// heavy are 0 where the default rules stand: these depend on the graph, and
+// the words (like alpha, beta and bits_div) apply to every graph of the engine.
 struct LevelSettings {
   uint32_t words, alpha, beta, split, bits_div, heavy;
   uint32_t& at(int i) {
@@ -1594,7 +1589,6 @@ int apply_settings(msbfs_engine* eng, msbfs_graph* g, const LevelSettings& s) {
   eng->alpha = s.alpha;
   eng->beta = s.beta;
   eng->bits_div = s.bits_div;
-  eng->heavy = s.heavy;
   if (s.split != g->split || s.heavy != g->heavy)
     return build_bottom_up_tables(eng, g, s.split, s.heavy);
   return MSBFS_OK;
@@ -1636,22 +1630,29 @@ extern "C" int msbfs_engine_autotune(msbfs_engine* e, msbfs_graph* g, const uint
       msbfs::graph_class(g->V, g->E, g->max_deg) + "/s" + std::to_string(bucket);
   msbfs_tuning t{};
   std::strncpy(t.class_name, key.c_str(), sizeof t.class_name - 1);
-  LevelSettings best{widest_pass(e, g), e->alpha, e->beta, g->split, e->bits_div, g->heavy};
+  LevelSettings best{e->max_words, e->alpha, e->beta, g->split, e->bits_div, g->heavy};
+  const int method = resolve_method(g, e->method, S);
+  const uint32_t mode = path_mode(method_path(method));
+  // What the words and the in-degree of a setting come to for this call (a cap
+  // above the words that the sources need makes no difference).
+  uint32_t wmax = 1;
+  while (wmax < (S + 31) / 32 && wmax < 64) wmax <<= 1;
+  auto words_of = [&](const LevelSettings& s) {
+    return s.words ? std::min(s.words, wmax) : choose_words(e, g, S, mode);
+  };
+  auto heavy_of = [&](const LevelSettings& s) {
+    return s.heavy ? s.heavy : warp_scan_degree(e, g->h_coff);
+  };
   auto report = [&](const LevelSettings& s) {
-    // The words a pass of this call uses (a cap above the sources' need
-    // makes no difference).
-    uint32_t need = 1;
-    while (need < (S + 31) / 32 && need < 64) need <<= 1;
-    t.max_words_per_pass = std::min(s.words, need);
+    t.max_words_per_pass = words_of(s);
     t.alpha = s.alpha;
     t.beta = s.beta;
     t.hub_split = s.split;
     t.bitmap_div = s.bits_div;
-    t.warp_scan_degree = s.heavy;
+    t.warp_scan_degree = g->scan_degree;
     if (out) *out = t;
     return MSBFS_OK;
   };
-  const int method = resolve_method(g, e->method, S);
   if (method_path(method) == MSBFS_PATH_CTA) return report(best);
   t.level_path = 1;
   const bool shared = !g->users.empty() || g->eng != e;  // other engines hold its tables
@@ -1678,8 +1679,6 @@ extern "C" int msbfs_engine_autotune(msbfs_engine* e, msbfs_graph* g, const uint
   if ((rc = time_stats_call(e, g, sources, S, method, &best_ms))) return rc;
   t.default_ms = best_ms;
   t.trials = 1;
-  uint32_t wmax = 1;
-  while (wmax < (S + 31) / 32 && wmax < 64) wmax <<= 1;
   const std::vector<std::vector<uint32_t>> cands = {
       {std::max(1u, wmax / 4), std::max(1u, wmax / 2), wmax},  // words per vertex
       {4, 8, 14, 28, 56},                                      // alpha
@@ -1687,6 +1686,7 @@ extern "C" int msbfs_engine_autotune(msbfs_engine* e, msbfs_graph* g, const uint
       {256, 512, 1024},                                        // slice length
       {16, 64, 256},                                           // bitmap divisor
       {8, 16, 32, 64}};                                        // warp-scan in-degree
+  const uint32_t start_words = words_of(best);  // (while the engine holds these settings)
   // One setting at a time, each from the best found so far; a change is
   // kept only when it is at least 2% faster (timing noise).
   for (int i = 0; i < 6; ++i) {
@@ -1695,7 +1695,7 @@ extern "C" int msbfs_engine_autotune(msbfs_engine* e, msbfs_graph* g, const uint
     for (uint32_t c : cands[i]) {
       LevelSettings s = base;
       s.at(i) = c;
-      if (s == base) continue;
+      if (s == base || (i == 0 && c == start_words) || (i == 5 && c == heavy_of(base))) continue;
       if ((rc = apply_settings(e, g, s))) return rc;
       double ms = 0;
       if ((rc = time_stats_call(e, g, sources, S, method, &ms))) return rc;
