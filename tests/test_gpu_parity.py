@@ -563,3 +563,32 @@ def test_tuning_one_graph_keeps_the_table_rule_for_others(native, tmp_path):
         assert eng.autotune(road, src)["warp_scan_degree"] == 32
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("blocks", ["1", "1000000"])
+def test_traversal_grids_that_do_and_do_not_launch(native, oracle, monkeypatch, blocks):
+    """A traversal of one block, and one whose blocks cannot all be resident:
+    the launch is refused, and the host drives the levels. Rows into pageable
+    and into page-locked memory (the latter written partly as bytes, two
+    passes), byte-deep and deeper distances, statistics and reachability."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("MSBFS_TRAVERSE_BLOCKS", blocks)
+    for g in (native.generate_graph500_rmat(11, 8, 4), native.path_graph(700)):
+        V, S = g.num_vertices, 100
+        src = native.sample_sources(g, S, 6, min_degree=1)
+        want = _oracle(oracle, g, src)
+        eng = native.GpuBfsEngine(native.GpuBfsMethod.PushPullAdaptive)
+        try:
+            eng.set_tuning(max_words_per_pass=2)
+            for pinned in (False, True, True):
+                out = torch.zeros(S * V, dtype=torch.int32, pin_memory=pinned).numpy().view(np.uint32)
+                eng.run_ms_bfs_into(g, src, out)
+                assert eng.last_stats["passes"] == 2
+                assert_same(out, want, g, src, f"pinned={pinned}")
+            rows = want.reshape(S, V)
+            st = eng.run_ms_bfs_stats(g, src)
+            assert np.array_equal(st["reached"], (rows != 0xFFFFFFFF).sum(1))
+            reach = eng.run_ms_reachability(g, src)
+            assert reach.total_reachable_pairs() == st["reached"].sum()
+        finally:
+            eng.close()

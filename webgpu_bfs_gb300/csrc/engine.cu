@@ -176,6 +176,7 @@ struct msbfs_engine {
   uint32_t mat_waves = MSBFS_MAT_WAVES;
   uint32_t level_cap = 0;   // levels per pass before MSBFS_ERR_TIMEOUT (0: V + 2)
   bool host_loop = false;
+  uint32_t traverse_blocks = 0;  // grid of the traversal (MSBFS_TRAVERSE_BLOCKS; 0: get_workspace)
   // Polls of a grid barrier before the traversal gives up (tens of seconds;
   // MSBFS_BARRIER_SPINS), and the word that it then sets (page-locked).
   uint32_t barrier_spins = 1u << 26;
@@ -365,6 +366,7 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   const uint64_t loads = (uint64_t)g->V * std::max(1u, W / 4) + g->E;
   w->k.traverse_grid = (int)std::min<uint64_t>(w->k.traverse_grid, std::max<uint64_t>(64, loads / 1024));
   w->k.traverse_grid = std::max(1, (int)((uint64_t)w->k.traverse_grid * eng->sm_share / 100));
+  if (eng->traverse_blocks) w->k.traverse_grid = (int)eng->traverse_blocks;
   LevelParams& p = w->p;
   p.V = (uint32_t)g->V;
   p.W = W;
@@ -716,14 +718,29 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
     } else if (!one_launch) {
       if ((rc = run_pass_host_loop(eng, w, reduce))) return rc;
     } else {
-      CK(launch_traverse(w->p, w->k, eng->stream));
+      const cudaError_t launched = launch_traverse(w->p, w->k, eng->stream);
+      const bool refused = launched == cudaErrorCooperativeLaunchTooLarge ||
+                           launched == cudaErrorLaunchOutOfResources ||
+                           launched == cudaErrorNotSupported;
+      if (refused) {
+        // Its blocks cannot all be resident (a process may be given a part of
+        // the device only): the host drives this engine's levels from now on.
+        // One materialisation then writes the pass, all its rows in one form.
+        cudaGetLastError();
+        eng->host_loop = true;
+        w->p.d.row_split = eng->split_rows[ps] = 0;
+        if ((rc = run_pass_host_loop(eng, w, reduce))) return rc;
+      } else {
+        CK(launched);
+        if (split) launch_materialize(w->p, w->k, false, eng->stream, MAT_BYTES);
+      }
       if (split) {
-        launch_materialize(w->p, w->k, false, eng->stream, MAT_BYTES);
         CK(cudaMemcpyAsync(&eng->h_ctl[ps], w->d_ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost,
                            eng->stream));
         CK(cudaEventRecord(eng->split_events[ps], eng->stream));
       }
-      launch_materialize(w->p, w->k, reduce, eng->stream, split ? MAT_WIDE : MAT_ALL);
+      if (!refused)
+        launch_materialize(w->p, w->k, reduce, eng->stream, split ? MAT_WIDE : MAT_ALL);
       CK(cudaGetLastError());
     }
     CK(cudaMemcpyAsync(&eng->h_ctl[ps], w->d_ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost,
@@ -1248,6 +1265,8 @@ int msbfs_engine_create(int device, int method, msbfs_engine** out) {
   int coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
   e->host_loop = !coop || (hl && hl[0] == '1');
+  const char* tb = getenv("MSBFS_TRAVERSE_BLOCKS");
+  if (tb) e->traverse_blocks = (uint32_t)std::max(0, atoi(tb));
   const char* bs = getenv("MSBFS_BARRIER_SPINS");
   if (bs) e->barrier_spins = (uint32_t)std::max(1, atoi(bs));
   const char* zc = getenv("MSBFS_ZERO_COPY");
