@@ -1058,8 +1058,9 @@ int widen_to_host(msbfs_engine* eng, const uint8_t* src, uint32_t* out, size_t n
   const size_t nchunks = (n + CHUNK - 1) / CHUNK;
   // A worker per 256 KB (us into fresh memory with 4 / 16 workers: 1 MB of
   // distances, R-MAT 14 S=64, 289 / 381; 17 MB, R-MAT 17 S=129, 2,114 / 1,616).
-  const unsigned T =
-      (unsigned)std::min<size_t>(HostPool::max_workers(), std::max<size_t>(n >> 18, 1));
+  const unsigned T = eng->pool.reserve(
+      (unsigned)std::min<size_t>(HostPool::max_workers(), std::max<size_t>(n >> 18, 1)));
+  if (!T) return set_err(eng, MSBFS_ERR_OOM, "no thread to widen the byte rows with");
   std::mutex mu;
   std::condition_variable cv;
   size_t issued = 0, widened = 0;  // chunks issued / widened by every worker (in order)

@@ -13,6 +13,7 @@
 #include <condition_variable>
 #include <cstddef>
 #include <cstdint>
+#include <exception>
 #include <functional>
 #include <mutex>
 #include <thread>
@@ -37,22 +38,32 @@ class HostPool {
     cv_.notify_all();
     for (std::thread& t : threads_) t.join();
   }
-  // Starts body(k) for every k < n (at most max_workers()) and returns; the
-  // threads are created on first use. Waits for the job before.
-  void start(unsigned n, std::function<void(unsigned)> body) {
+  // Creates threads up to n (at most max_workers()) and returns how many of n
+  // there are: fewer when the system gives no more. Waits for the job before.
+  unsigned reserve(unsigned n) {
     wait();
-    while (threads_.size() < n) {
-      const unsigned k = (unsigned)threads_.size();
-      threads_.emplace_back([this, k, seen = job_.load()] { work(k, seen); });
+    try {
+      while (threads_.size() < n) {
+        const unsigned k = (unsigned)threads_.size();
+        threads_.emplace_back([this, k, seen = job_.load()] { work(k, seen); });
+      }
+    } catch (const std::exception&) {  // callers are C entry points
     }
+    return std::min(n, (unsigned)threads_.size());
+  }
+  // Starts body(k) for every k < n on a thread each, and returns. Shares that no
+  // thread can be had for run here, before the return.
+  void start(unsigned n, std::function<void(unsigned)> body) {
+    const unsigned have = reserve(n);
     {
       std::lock_guard<std::mutex> lk(mu_);  // a worker takes job and share together
       body_ = std::move(body);
-      active_ = n;
-      left_.store(n);
+      active_ = have;
+      left_.store(have);
       job_.fetch_add(1);
     }
     cv_.notify_all();
+    for (unsigned k = have; k < n; ++k) body_(k);
   }
   void wait() {
     if (left_.load(std::memory_order_acquire) == 0) return;
