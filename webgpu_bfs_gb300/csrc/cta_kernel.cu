@@ -22,6 +22,7 @@
 
 #include "../../include/msbfs.h"
 #include "cta_expand.cuh"
+#include "cta_grid.h"
 #include "device_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -348,8 +349,8 @@ static int cluster_capacity(int cl, bool er, size_t smem, int block, int optin) 
 // Cluster mode for a call of few sources: the smallest cluster whose slices
 // hold the bitmap next to rank 0's queue halves. MSBFS_CTA_CLUSTER=0 turns
 // it off, =1 uses it whatever the number of sources.
-static bool cta_cluster_shape(uint32_t V, int sms, int optin, bool edge_records,
-                              size_t num_sources, CtaShape* out) {
+static bool cta_cluster_shape(uint32_t V, int optin, bool edge_records, size_t num_sources,
+                              uint32_t sm_share, CtaShape* out) {
   const char* env = getenv("MSBFS_CTA_CLUSTER");
   const int mode = env ? atoi(env) : -1;
   if (mode == 0) return false;
@@ -375,8 +376,7 @@ static bool cta_cluster_shape(uint32_t V, int sms, int optin, bool edge_records,
     // S=64 10.7 vs 18.8 ms; S=152, two sources per cluster, 21.2 vs 22.1;
     // S=256 46.3 vs 28.0 with a 512-thread rank 0).
     if (mode != 1 && num_sources > (size_t)n) return false;
-    sh.grid = n * cl;
-    (void)sms;
+    sh.grid = std::max(1, (int)((uint64_t)n * sm_share / 100)) * cl;
     *out = sh;
     return true;
   }
@@ -384,7 +384,7 @@ static bool cta_cluster_shape(uint32_t V, int sms, int optin, bool edge_records,
 }
 
 bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_records,
-                      size_t num_sources, CtaShape* out) {
+                      size_t num_sources, uint32_t sm_share, CtaShape* out) {
   int sms = 0, optin = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -393,7 +393,7 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   const size_t entry = sizeof(uint32_t);  // a vertex id or a packed edge range
   const bool shared_bits = (size_t)V <= cta_max_vertices(device);
   if (!shared_bits && !allow_global) return false;
-  if (!shared_bits && cta_cluster_shape(V, sms, optin, edge_records, num_sources, out))
+  if (!shared_bits && cta_cluster_shape(V, optin, edge_records, num_sources, sm_share, out))
     return true;
   CtaShape sh{};
   sh.edge_records = edge_records;
@@ -432,19 +432,13 @@ bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_recor
   if (allow_smem(fn, optin) != cudaSuccess) cudaGetLastError();
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, sh.block, sh.smem);
   if (occ < 1) return false;
-  sh.grid = sms * occ;
+  sh.grid = std::max(1, (int)((uint64_t)sms * occ * sm_share / 100));
   if (!shared_bits) {
-    // Every edge is an atomic on a bitmap: more blocks than have theirs in
-    // two thirds of the L2 slow each other down, but not fewer than one per
-    // SM. Road 1448x1448 (262 KB bitmaps), S=512 / 2,048, ms with 152, 228,
-    // 304, 456 blocks: 62 / 222, 52 / 175, 42 / 158, 54 / 167. About as many
-    // sources per block each: the nearest whole number of rounds.
+    // Two thirds of the L2 for bitmaps, but not fewer than one per SM.
     int l2 = 0;
     cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device);
     const size_t in_l2 = (size_t)l2 / 3 * 2 / (words * sizeof(uint32_t)) / sms * sms;
-    const size_t most = std::max<size_t>(in_l2, sms);
-    const size_t rounds = std::max<size_t>((num_sources + most / 2) / most, 1);
-    sh.grid = (int)std::min<size_t>((size_t)sh.grid, (num_sources + rounds - 1) / rounds);
+    sh.grid = (int)global_bitmap_grid(sh.grid, std::max<size_t>(in_l2, sms), num_sources);
     const size_t per_block = ((size_t)V + words) * sizeof(uint32_t);
     sh.grid = (int)std::max<size_t>(
         1, std::min<size_t>((size_t)sh.grid, CTA_GLOBAL_SCRATCH_BYTES / per_block));
@@ -562,7 +556,7 @@ extern "C" int msbfs_run_cta_noalloc(int device, size_t num_vertices,
   const uint32_t V = (uint32_t)num_vertices;
   CtaShape sh{};
   if (!cta_launch_shape(V, device, /*allow_global=*/false, /*edge_records=*/false, num_sources,
-                        &sh))
+                        /*sm_share=*/100, &sh))
     return MSBFS_ERR_SCRATCH_TOO_SMALL;
   const size_t slabs = (NOALLOC_WORDS - NOALLOC_Q_OFF) / (size_t)V;
   const cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);

@@ -236,7 +236,7 @@ struct CtaParams {
   const uint2* erec;     // per edge {target, target's edge begin << 4 | count}, or null
 };
 struct CtaShape {
-  int grid = 0;           // resident blocks
+  int grid = 0;           // blocks: those resident at the SM share, or fewer
   int block = 0;          // threads per block
   size_t smem = 0;        // dynamic shared memory: bitmap (shared mode) + queue halves
   uint32_t qh = 0;        // frontier entries per shared-memory queue half
@@ -251,11 +251,12 @@ struct CtaShape {
 // for a call of num_sources sources (above that V when allow_global: the
 // bitmap split over the shared memory of a thread-block cluster for calls of
 // few sources, an L2-resident global slab per block otherwise; edge-range
-// queue entries when the graph has edge records). In cluster mode `grid`
+// queue entries when the graph has edge records), on sm_share percent of what
+// the device holds at once. In cluster mode `grid`
 // counts blocks (a multiple of `cluster`) and each cluster has one queue slab.
 size_t cta_max_vertices(int device);
 bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_records,
-                      size_t num_sources, CtaShape* out);
+                      size_t num_sources, uint32_t sm_share, CtaShape* out);
 void launch_cta(const CtaParams& p, const CtaShape& sh, int grid, cudaStream_t s);
 void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, uint2* erec,
                          cudaStream_t s);

@@ -597,9 +597,8 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
   if (reach_dev && path == MSBFS_PATH_CTA) path = MSBFS_PATH_HYBRID;
   CtaShape cta{};
   if (path == MSBFS_PATH_CTA &&
-      !cta_launch_shape((uint32_t)g->V, eng->device, true, g->erec != nullptr, S, &cta))
+      !cta_launch_shape((uint32_t)g->V, eng->device, true, g->erec != nullptr, S, eng->sm_share, &cta))
     path = MSBFS_PATH_HYBRID;
-  const int cta_grid = std::max(1, (int)((uint64_t)cta.grid * eng->sm_share / 100));
   if (!g->sym && path != MSBFS_PATH_CTA && !g->coff)
     return set_err(eng, MSBFS_ERR_INVALID_GRAPH, "missing transpose");
 
@@ -617,7 +616,7 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
     // Cluster mode: `blocks` stays a multiple of the cluster size, one
     // queue slab per cluster.
     const int cl = std::max(1, cta.cluster);
-    const int blocks = std::max(cl, std::min<int>(cta_grid, (int)std::min<size_t>(S * cl, 1u << 30)) / cl * cl);
+    const int blocks = std::max(cl, std::min<int>(cta.grid, (int)std::min<size_t>(S * cl, 1u << 30)) / cl * cl);
     if (V > cta.qh &&  // else every frontier fits the shared-memory halves
         (rc = grow(eng, &eng->d_cta_queue, &eng->d_cta_queue_cap, (size_t)(blocks / cl) * V)))
       return rc;
