@@ -202,3 +202,45 @@ def test_server_admits_row_launches_by_free_pool_bytes(native, oracle):
         assert info["launches"] == 1
     finally:
         srv.close()
+
+
+@pytest.mark.parametrize("percent", [85, 40])
+def test_express_requests_complete_beside_general_traversals(native, percent):
+    """While a general slot traverses a path of 350,000 levels, in a launch as
+    large as its share of the GPU allows, and another has the same to do, small
+    requests of both kinds are admitted and complete (their sources lie in a
+    component of their own)."""
+    n, k = 350_000, 64
+    path = np.arange(n - 1, dtype=np.int64)
+    i, j = np.triu_indices(k, 1)
+    e = np.concatenate([np.stack([path, path + 1], 1), np.stack([n + i, n + j], 1)])
+    g = native.CsrGraph.from_edge_list(n + k, np.concatenate([e, e[:, ::-1]]))
+    srv = native.BfsServer(g, slots=3, max_sources_per_launch=9, express_slots=1,
+                           small_sources=8, general_sm_percent=percent,
+                           method=native.GpuBfsMethod.MultiWordBitParallelPush)
+
+    def general(first):
+        src = np.full(9, first, np.uint32)
+        return [srv.submit(src), srv.submit(src)]
+
+    try:
+        for mode in (srv.STATS, srv.ROWS):  # workspaces built
+            srv.wait(srv.submit(np.arange(n, n + 4, dtype=np.uint32), mode))
+        for _ in range(2):
+            for t in general(n):
+                srv.wait(t)
+        large = general(0)
+        with pytest.raises(native.BfsError):
+            srv.wait(large[0], timeout_ms=20)
+        for _ in range(2):
+            res, info = srv.wait(srv.submit(np.array([n], np.uint32)))
+            assert info["status"] == 0 and res["eccentricity"][0] == 1 and res["reached"][0] == k
+            rows, info = srv.wait(srv.submit(np.array([n], np.uint32), srv.ROWS))
+            assert info["status"] == 0 and rows[n:].tolist() == [0] + [1] * (k - 1)
+        with pytest.raises(native.BfsError):  # the first large one is still running
+            srv.wait(large[0], timeout_ms=0.01)
+        for t in large:
+            res, info = srv.wait(t)
+            assert info["status"] == 0 and (res["eccentricity"] == n - 1).all()
+    finally:
+        srv.close()

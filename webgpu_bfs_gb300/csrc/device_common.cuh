@@ -176,20 +176,21 @@ constexpr int MAT_NPMAX = 8;
 // Launch helpers implemented in level_launch.cu / cta_kernel.cu.
 struct LevelKernelInfo {
   void* traverse;     // a pass's whole traversal, cooperative
-  int traverse_grid;  // its resident grid
+  int traverse_resident;  // its resident grid
+  int traverse_grid;  // blocks it is launched with at most
   void* init;         // the same level by level, driven by the host
   void* level[2][2];  // [direction: DIR_PUSH, DIR_PULL][with profiling counters]
   int level_grids[2]; // resident grid per direction
   void* materialize;
-  void* reduce;       // per-source reductions in place of materialize
+  void* reduce[2];    // per-source reductions in place of materialize: [in narrow blocks]
   void* cleanup;
   void* queue;        // a top-down level's queue after a bottom-up one (host-driven loop)
   int level_block;
   int mat_block;
   int mat_grid;
   size_t mat_smem;
-  int red_block;
-  int red_grid;
+  int red_block[2];
+  int red_grid[2];
 };
 // Fills kernel symbols and launch shapes for words-per-vertex W and NP level
 // planes (the materialisation stages 1 + NP arrays in shared memory).
@@ -199,8 +200,10 @@ size_t materialize_smem_bytes(uint32_t W, uint32_t NP);
 // W words per vertex: an upper bound on what a pass of fewer sources uses.
 size_t materialize_items(uint32_t V, uint32_t W);
 // A whole traversal (source init, levels, frontier cleanup) in one cooperative
-// launch of k.traverse_grid blocks.
-cudaError_t launch_traverse(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
+// launch of `blocks` blocks. leave_room: with shared memory for other streams'
+// kernels beside them.
+cudaError_t launch_traverse(const LevelParams& p, const LevelKernelInfo& k, int blocks,
+                            bool leave_room, cudaStream_t s);
 void launch_init(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
 // Launches the level kernel of direction `dir` (DIR_PUSH / DIR_PULL), or
 // both (pull, then push) when dir is DIR_BOTH; `count` picks the form that
@@ -208,7 +211,8 @@ void launch_init(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s)
 constexpr uint32_t DIR_BOTH = 2;
 void launch_level(const LevelParams& p, const LevelKernelInfo& k, uint32_t dir, bool count,
                   cudaStream_t s);
-// reduce: per-source reductions (reduce_kernel) instead of rows or bitmasks.
+// reduce: per-source reductions (reduce_kernel) instead of rows or bitmasks,
+// narrow: in blocks that find room beside another stream's traversal.
 // phase (materialisation only): MAT_ALL writes every row (bytes when the
 // pass allows) and clears the traversal state; MAT_BYTES writes only the
 // byte rows from PassDesc::row_split on and clears nothing (nothing at all
@@ -216,7 +220,7 @@ void launch_level(const LevelParams& p, const LevelKernelInfo& k, uint32_t dir, 
 // below the split (all rows when the pass did not go to bytes) and clears.
 enum : uint32_t { MAT_BYTES = 0, MAT_WIDE = 1, MAT_ALL = 2 };
 void launch_materialize(const LevelParams& p, const LevelKernelInfo& k, bool reduce,
-                        cudaStream_t s, uint32_t phase = MAT_ALL);
+                        cudaStream_t s, uint32_t phase = MAT_ALL, bool narrow = false);
 void launch_queue(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
 void launch_cleanup(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s);
 

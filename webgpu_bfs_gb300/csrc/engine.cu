@@ -163,6 +163,10 @@ struct msbfs_engine {
   uint32_t split = MSBFS_SPLIT;  // in-edge slice length of bottom-up steps
   uint32_t bits_div = 64;
   uint32_t sm_share = 100;  // percent of the resident grid the persistent kernels use
+  // Served form: most of it for the next traversals, and reductions in blocks
+  // that find room beside another stream's traversal.
+  uint32_t traverse_cap = 100;
+  bool narrow_reduce = false;
 #ifndef MSBFS_MAT_WAVES
 // R-MAT scale 22, S=512, materialisation ms: 1 wave (persistent) 1.82, 2
 // 1.81, 4 1.69, 8 1.65, one block per tile 1.59. Blocks of a long
@@ -311,6 +315,15 @@ bool wide_pass_fits(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_
   return need <= eng->total_mem / 8 && need <= free_mem / 2;
 }
 
+// Blocks of a traversal. Blocks that a small graph cannot feed only make the
+// grid barriers of its levels longer: a block per 1,024 lane loads (visited
+// pieces and edges).
+int traversal_blocks(const msbfs_engine* eng, const msbfs_graph* g, uint32_t W, int resident) {
+  const uint64_t loads = (uint64_t)g->V * std::max(1u, W / 4) + g->E;
+  const uint64_t blocks = std::min<uint64_t>(resident, std::max<uint64_t>(64, loads / 1024));
+  return std::max(1, (int)(blocks * eng->sm_share / 100));
+}
+
 int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t mode,
                   Workspace** out) {
   auto key = std::make_tuple(g->id, W, mode);
@@ -360,12 +373,8 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
     const size_t want = eng->mat_waves ? (size_t)w->k.mat_grid * eng->mat_waves : items;
     w->k.mat_grid = (int)std::max<size_t>(1, std::min(want, items));
   }
-  w->k.red_grid = std::max(1, (int)((uint64_t)w->k.red_grid * eng->sm_share / 100));
-  // Blocks that a small graph cannot feed only make the grid barriers of its
-  // levels longer: a block per 1,024 lane loads (visited pieces and edges).
-  const uint64_t loads = (uint64_t)g->V * std::max(1u, W / 4) + g->E;
-  w->k.traverse_grid = (int)std::min<uint64_t>(w->k.traverse_grid, std::max<uint64_t>(64, loads / 1024));
-  w->k.traverse_grid = std::max(1, (int)((uint64_t)w->k.traverse_grid * eng->sm_share / 100));
+  for (int& grid : w->k.red_grid) grid = std::max(1, (int)((uint64_t)grid * eng->sm_share / 100));
+  w->k.traverse_grid = traversal_blocks(eng, g, W, w->k.traverse_resident);
   if (eng->traverse_blocks) w->k.traverse_grid = (int)eng->traverse_blocks;
   LevelParams& p = w->p;
   p.V = (uint32_t)g->V;
@@ -717,7 +726,10 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
     } else if (!one_launch) {
       if ((rc = run_pass_host_loop(eng, w, reduce))) return rc;
     } else {
-      const cudaError_t launched = launch_traverse(w->p, w->k, eng->stream);
+      int blocks = w->k.traverse_grid;
+      if (eng->traverse_cap < 100)
+        blocks = std::min(blocks, std::max(1, (int)((uint64_t)w->k.traverse_resident * eng->traverse_cap / 100)));
+      const cudaError_t launched = launch_traverse(w->p, w->k, blocks, eng->traverse_cap < 100, eng->stream);
       const bool refused = launched == cudaErrorCooperativeLaunchTooLarge ||
                            launched == cudaErrorLaunchOutOfResources ||
                            launched == cudaErrorNotSupported;
@@ -739,7 +751,8 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
         CK(cudaEventRecord(eng->split_events[ps], eng->stream));
       }
       if (!refused)
-        launch_materialize(w->p, w->k, reduce, eng->stream, split ? MAT_WIDE : MAT_ALL);
+        launch_materialize(w->p, w->k, reduce, eng->stream, split ? MAT_WIDE : MAT_ALL,
+                           eng->narrow_reduce);
       CK(cudaGetLastError());
     }
     CK(cudaMemcpyAsync(&eng->h_ctl[ps], w->d_ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost,
@@ -1416,6 +1429,29 @@ int msbfs_graph_attach(msbfs_graph* g, msbfs_engine* e) {
   if (e != g->eng && std::find(g->users.begin(), g->users.end(), e) == g->users.end())
     g->users.push_back(e);
   return MSBFS_OK;
+}
+
+// The part of the device that a level-path traversal of S sources takes, in
+// percent of the blocks resident on all of it; 0 when the engine's method sends
+// the call to the CTA path. Not part of the C ABI.
+uint32_t msbfs_engine_traversal_share(msbfs_engine* e, const msbfs_graph* g, size_t S) {
+  std::lock_guard<std::mutex> lk(e->mu);
+  if (method_path(resolve_method(g, e->method, S)) == MSBFS_PATH_CTA) return 0;
+  uint32_t W = 1;
+  while (W < 64 && (size_t)W * 32 < S) W <<= 1;
+  LevelKernelInfo k{};
+  if (!level_kernel_info(W, level_planes(g), e->num_sms, &k)) return 100;
+  const int blocks = traversal_blocks(e, g, W, k.traverse_resident);
+  return (uint32_t)((100ull * blocks + k.traverse_resident - 1) / k.traverse_resident);
+}
+
+// The served form's cap on the blocks of the engine's next traversals, in
+// percent of those resident on the whole device, and whether its calls may have
+// to find room beside other traversals. Not part of the C ABI.
+void msbfs_engine_cap_traversal(msbfs_engine* e, uint32_t percent, bool beside) {
+  std::lock_guard<std::mutex> lk(e->mu);
+  e->traverse_cap = percent;
+  e->narrow_reduce = beside;
 }
 
 extern "C" {

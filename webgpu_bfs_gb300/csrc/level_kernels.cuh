@@ -1436,13 +1436,16 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
   return x;
 }
 
-constexpr int RED_BLOCK = 256;
+// Threads of a block. The narrow form is for the served form's express slots:
+// beside a traversal of five blocks an SM, 14,336 registers are free, less than
+// 256 threads take. us of a statistics call with 256 / 128 everywhere: R-MAT 21
+// S=64 898 / 916, R-MAT 16 S=64 191 / 203, R-MAT 23 S=2,048 29.2 / 28.8 ms.
+constexpr int RED_BLOCK = 256, RED_BLOCK_NARROW = 128;
 #ifndef MSBFS_RED_MIN_BLOCKS
 // R-MAT scale 22, S=512: 3 blocks (80 registers, a few spills) 0.82 ms,
 // 2 blocks (113 registers) 0.96 ms, 4 blocks (64 registers) 0.92 ms.
 #define MSBFS_RED_MIN_BLOCKS 3
 #endif
-constexpr int RED_MIN_BLOCKS = MSBFS_RED_MIN_BLOCKS;
 template <int VEC>
 __device__ __forceinline__ bool any_word(const Words<VEC>& x) {
   uint32_t a = 0;
@@ -1465,8 +1468,9 @@ __device__ __forceinline__ bool any_word(const Words<VEC>& x) {
 // non-zero are written back as zero (the next pass starts from clean
 // buffers). Lanes flagged in ovf (deeper than the planes encode) were folded
 // in by the level kernel.
-template <int W>
-__global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(const __grid_constant__ LevelParams p) {
+template <int W, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, MSBFS_RED_MIN_BLOCKS * RED_BLOCK / BLOCK)
+    reduce_kernel(const __grid_constant__ LevelParams p) {
   constexpr int G = W >= 4 ? 4 : W;
   SourceStats* st = p.d.stats;
   if (!st) return;
@@ -1494,7 +1498,7 @@ __global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(const
     if (begin >= p.V) continue;  // the same for the whole block
     const uint32_t v_end = (uint32_t)min(begin + per_share, (size_t)p.V);
     const uint32_t v0 = (uint32_t)begin + (threadIdx.x & ~31u);
-    for (uint32_t i = threadIdx.x; i < G * 32; i += RED_BLOCK) {
+    for (uint32_t i = threadIdx.x; i < G * 32; i += BLOCK) {
       s_sum[i] = 0;
       s_cnt[i] = s_ecc[i] = 0;
     }
@@ -1508,12 +1512,12 @@ __global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(const
     }
     Words<G> xn = zero;
     if (v0 + lane < v_end) xn = ld_words<G>(p.vis + (size_t)(v0 + lane) * W + (size_t)g * G);
-    for (uint32_t vb = v0; vb < v_end; vb += RED_BLOCK) {
+    for (uint32_t vb = v0; vb < v_end; vb += BLOCK) {
       const uint32_t v = vb + lane;
       const size_t a = (size_t)v * W + (size_t)g * G;
       const Words<G> x = xn;
       xn = zero;
-      if (v + RED_BLOCK < v_end) xn = ld_words<G>(p.vis + a + RED_BLOCK * (size_t)W);
+      if (v + BLOCK < v_end) xn = ld_words<G>(p.vis + a + BLOCK * (size_t)W);
       const bool any = any_word(x);
       if (__ballot_sync(FULL, any) == 0) continue;  // warp-uniform
       Words<G> o = zero, pl[MAT_NPMAX];
@@ -1559,7 +1563,7 @@ __global__ void __launch_bounds__(RED_BLOCK, RED_MIN_BLOCKS) reduce_kernel(const
       atomicAdd(&s_cnt[32 * i + lane], cnt[i]);
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < G * 32; i += RED_BLOCK) {
+    for (uint32_t i = threadIdx.x; i < G * 32; i += BLOCK) {
       const uint32_t s = 32 * g * G + i;
       if (s_cnt[i] && s < P) {
         atomicAdd(&st[s].sum, s_sum[i]);
@@ -1744,7 +1748,8 @@ void fill_level_info(int num_sms, uint32_t NP, LevelKernelInfo* k) {
   k->level[DIR_PULL][0] = (void*)level_kernel<W, DIR_PULL, false>;
   k->level[DIR_PULL][1] = (void*)level_kernel<W, DIR_PULL, true>;
   k->materialize = (void*)materialize_kernel<W>;
-  k->reduce = (void*)reduce_kernel<W>;
+  k->reduce[0] = (void*)reduce_kernel<W, RED_BLOCK>;
+  k->reduce[1] = (void*)reduce_kernel<W, RED_BLOCK_NARROW>;
   k->cleanup = (void*)cleanup_kernel<W>;
   k->queue = (void*)queue_kernel<W>;
   auto resident = [&](const void* fn, int block, size_t smem) {
@@ -1753,7 +1758,7 @@ void fill_level_info(int num_sms, uint32_t NP, LevelKernelInfo* k) {
     return num_sms * (occ < 1 ? 1 : occ);
   };
   k->level_block = LEVEL_BLOCK;
-  k->traverse_grid = resident(k->traverse, LEVEL_BLOCK, 0);
+  k->traverse_resident = k->traverse_grid = resident(k->traverse, LEVEL_BLOCK, 0);
   // The counting form runs at the production form's grid (it is only run
   // for its counters; the roofline's durations come from the production form).
   for (uint32_t d : {(uint32_t)DIR_PUSH, (uint32_t)DIR_PULL})
@@ -1761,8 +1766,10 @@ void fill_level_info(int num_sms, uint32_t NP, LevelKernelInfo* k) {
   k->mat_block = MAT_BLOCK;
   k->mat_smem = materialize_smem_bytes(W, NP);
   k->mat_grid = resident(k->materialize, MAT_BLOCK, k->mat_smem);
-  k->red_block = RED_BLOCK;
-  k->red_grid = resident(k->reduce, RED_BLOCK, 0);
+  for (int i = 0; i < 2; ++i) {
+    k->red_block[i] = i ? RED_BLOCK_NARROW : RED_BLOCK;
+    k->red_grid[i] = resident(k->reduce[i], k->red_block[i], 0);
+  }
 }
 
 }  // namespace msbfs

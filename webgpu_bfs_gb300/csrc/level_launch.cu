@@ -58,10 +58,26 @@ static void launch(void* fn, int grid, int block, size_t smem, const LevelParams
   cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, s);
 }
 
-cudaError_t launch_traverse(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s) {
+cudaError_t launch_traverse(const LevelParams& p, const LevelKernelInfo& k, int blocks,
+                            bool leave_room, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(k.level_block);
+  cfg.stream = s;
+  cudaLaunchAttribute attrs[2] = {};
+  attrs[0].id = cudaLaunchAttributeCooperative;
+  attrs[0].val.cooperative = 1;
+  // The part of an SM's L1 that is shared memory stays as it is while blocks are
+  // on it, and kernels of other streams start beside these only where it is large
+  // enough for them: at 72% (164 KB) all of a served request's kernels did, at
+  // 65% and by default none before this one's end. It costs the traversal 1-2%
+  // (R-MAT 21 S=512 2.42 -> 2.48 ms, R-MAT 22 S=2,048 14.92 -> 14.96; 86% 3.06 / 16.4).
+  attrs[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  attrs[1].val.sharedMemCarveout = 72;
+  cfg.attrs = attrs;
+  cfg.numAttrs = leave_room ? 2 : 1;
   void* args[] = {(void*)&p};
-  return cudaLaunchCooperativeKernel(k.traverse, dim3(k.traverse_grid), dim3(k.level_block), args,
-                                     0, s);
+  return cudaLaunchKernelExC(&cfg, k.traverse, args);
 }
 
 void launch_init(const LevelParams& p, const LevelKernelInfo& k, cudaStream_t s) {
@@ -80,9 +96,9 @@ void launch_level(const LevelParams& p, const LevelKernelInfo& k, uint32_t dir, 
 }
 
 void launch_materialize(const LevelParams& p, const LevelKernelInfo& k, bool reduce,
-                        cudaStream_t s, uint32_t phase) {
+                        cudaStream_t s, uint32_t phase, bool narrow) {
   if (reduce) {
-    launch(k.reduce, k.red_grid, k.red_block, 0, p, s);
+    launch(k.reduce[narrow], k.red_grid[narrow], k.red_block[narrow], 0, p, s);
     return;
   }
   void* args[] = {(void*)&p, &phase};

@@ -18,8 +18,13 @@
 
 #include "../../include/msbfs.h"
 
-// engine.cu: lets a second engine of the device run on a resident graph.
+// engine.cu: lets a second engine of the device run on a resident graph; the
+// part of the device that a level-path traversal of S sources takes, in percent
+// of the blocks it holds at once (0 on the CTA path); a cap on that part for an
+// engine's next calls, which may run beside other traversals.
 int msbfs_graph_attach(msbfs_graph* g, msbfs_engine* e);
+uint32_t msbfs_engine_traversal_share(msbfs_engine* e, const msbfs_graph* g, size_t S);
+void msbfs_engine_cap_traversal(msbfs_engine* e, uint32_t percent, bool beside);
 
 namespace {
 
@@ -52,6 +57,7 @@ struct Slot {
   msbfs_graph* g = nullptr;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev = nullptr;
+  cudaEvent_t traversed = nullptr;  // the running launch's traversal, before its copies
   size_t rows_off = 0;    // the running launch's rows in the server's pool
   size_t rows_bytes = 0;  // (0: none reserved)
   msbfs_source_stats* d_stats = nullptr;
@@ -62,6 +68,11 @@ struct Slot {
   bool express = false;  // takes small requests only, narrow launches
   bool busy = false;
   int launch_rc = MSBFS_OK;
+  bool traversing() const {
+    if (!busy || launch_rc || cudaEventQuery(traversed) != cudaErrorNotReady) return false;
+    cudaGetLastError();
+    return true;
+  }
 };
 
 size_t elem_bytes(int mode, size_t V) {
@@ -119,6 +130,17 @@ struct msbfs_server {
   int device = 0;
   size_t V = 0;
   msbfs_server_config cfg{};
+  // A level-path traversal starts only once all its blocks are resident, and
+  // while one waits for that, launches behind it wait too, whatever their
+  // priority. So that express requests never wait for a general one's end,
+  // general slots with a share below 100% have at most general_at_once
+  // traversals on the device, and express traversals beside them take
+  // express_percent of it, a part of what those leave. At 100% nothing is left,
+  // and general traversals keep the whole device. us of an express request beside
+  // a general traversal of 350,000 levels, statistics / rows: 250 / 140, with one
+  // or more general slots at work (4.5 s, that traversal, without this).
+  uint32_t general_at_once = 0;  // 0: no limit
+  uint32_t express_percent = 100;
   msbfs_graph* graph = nullptr;  // resident once, owned by slot 0's engine
   char* d_pool = nullptr;        // hbm_budget_bytes of distance-row staging
   RowPool pool;
@@ -147,7 +169,8 @@ void finish_part(msbfs_server* s, const Part& p, int rc) {
 
 // Issues one launch on slot `sl` (called without the lock; the slot is busy
 // so only the scheduler touches it).
-int launch_slot(msbfs_server* s, Slot& sl, const std::vector<uint32_t>& lanes) {
+int launch_slot(msbfs_server* s, Slot& sl, const std::vector<uint32_t>& lanes, uint32_t cap) {
+  msbfs_engine_cap_traversal(sl.eng, cap, s->general_at_once && sl.express);
   const size_t V = s->V, n = lanes.size();
   const size_t eb = elem_bytes(sl.mode, V);
   int rc;
@@ -158,6 +181,10 @@ int launch_slot(msbfs_server* s, Slot& sl, const std::vector<uint32_t>& lanes) {
     rc = msbfs_run_ms_bfs_stats_device(sl.eng, s->cfg.method, sl.g, lanes.data(), n,
                                        sl.d_stats);
   if (rc) return rc;
+  if (cudaEventRecord(sl.traversed, sl.stream) != cudaSuccess) {
+    cudaGetLastError();
+    return MSBFS_ERR_CUDA;
+  }
   bool need_stage = false;
   for (const Part& p : sl.parts) need_stage |= !p.r->out_pinned;
   if (need_stage && sl.h_stage_bytes < n * eb) {
@@ -186,6 +213,12 @@ int launch_slot(msbfs_server* s, Slot& sl, const std::vector<uint32_t>& lanes) {
     return MSBFS_ERR_CUDA;
   }
   return MSBFS_OK;
+}
+
+uint32_t traversing_general(const msbfs_server* s) {
+  uint32_t n = 0;
+  for (const Slot& sl : s->slots) n += !sl.express && sl.traversing();
+  return n;
 }
 
 void scheduler(msbfs_server* s) {
@@ -238,6 +271,7 @@ void scheduler(msbfs_server* s) {
     const size_t small = s->cfg.small_sources;
     for (Slot& sl : s->slots) {
       if (sl.busy || s->queue.empty()) continue;
+      if (!sl.express && s->general_at_once && traversing_general(s) >= s->general_at_once) continue;
       const bool have_express = s->cfg.express_slots > 0;
       bool want_small = sl.express;
       const Request* head = nullptr;
@@ -304,8 +338,13 @@ void scheduler(msbfs_server* s) {
       sl.busy = true;
       any_busy = true;
       progress = true;
+      uint32_t traversal_cap = 100;
+      if (s->general_at_once && sl.express)
+        traversal_cap = traversing_general(s) ? s->express_percent : 100;
+      else if (s->general_at_once)
+        traversal_cap = s->cfg.general_sm_percent;
       lk.unlock();
-      sl.launch_rc = reserved ? launch_slot(s, sl, lanes) : MSBFS_ERR_OOM;
+      sl.launch_rc = reserved ? launch_slot(s, sl, lanes, traversal_cap) : MSBFS_ERR_OOM;
       lk.lock();
     }
     if (s->stop && s->queue.empty() && !any_busy) break;
@@ -328,6 +367,7 @@ void destroy_slots(msbfs_server* s) {
     if (sl.d_stats) cudaFree(sl.d_stats);
     if (sl.h_stage) cudaFreeHost(sl.h_stage);
     if (sl.ev) cudaEventDestroy(sl.ev);
+    if (sl.traversed) cudaEventDestroy(sl.traversed);
     if (sl.stream) cudaStreamDestroy(sl.stream);
   }
   s->slots.clear();
@@ -377,7 +417,8 @@ int msbfs_server_create(int device, size_t V, size_t E, const uint32_t* ro, cons
     if ((rc = msbfs_engine_create(device, s->cfg.method, &sl.eng))) break;
     if (cudaStreamCreateWithPriority(&sl.stream, cudaStreamNonBlocking,
                                      sl.express ? prio_high : prio_low) != cudaSuccess ||
-        cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&sl.traversed, cudaEventDisableTiming) != cudaSuccess) {
       rc = MSBFS_ERR_CUDA;
       break;
     }
@@ -408,6 +449,15 @@ int msbfs_server_create(int device, size_t V, size_t E, const uint32_t* ro, cons
   if (rc) {
     destroy_slots(s.get());
     return rc;
+  }
+  if (s->cfg.express_slots && s->cfg.general_sm_percent < 100) {
+    const uint32_t general = s->cfg.slots - s->cfg.express_slots;
+    const uint32_t share =
+        msbfs_engine_traversal_share(s->slots.back().eng, s->graph, s->cfg.max_sources_per_launch);
+    const uint32_t most = std::max(s->cfg.general_sm_percent, 85u);  // of all general slots
+    s->general_at_once = share ? std::min(general, std::max(most / share, 1u)) : general;
+    s->express_percent =
+        std::max((100 - std::min(s->general_at_once * share, 99u)) / s->cfg.express_slots, 1u);
   }
   msbfs_server* raw = s.get();
   s->sched = std::thread(scheduler, raw);
