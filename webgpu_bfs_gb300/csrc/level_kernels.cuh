@@ -1078,8 +1078,7 @@ __global__ void __launch_bounds__(LEVEL_BLOCK) queue_kernel(const __grid_constan
 // run by the last block to arrive. Only valid in a cooperative launch (every
 // block resident). The wait is bounded: a block that gives up flags the pass,
 // the workspace and the engine (STATUS_STUCK, GridSync::stuck, h_stuck) and
-// returns false; blocks that come to a barrier of a stuck workspace do not
-// arrive, so it opens no more.
+// returns false; no block opens a barrier of a stuck workspace again.
 template <int W, typename Last>
 __device__ __forceinline__ bool level_barrier(const LevelParams& p, LevelShared<W>& sh,
                                               Last&& last_block) {
@@ -1091,9 +1090,10 @@ __device__ __forceinline__ bool level_barrier(const LevelParams& p, LevelShared<
     if (threadIdx.x == 0) {
       const uint2 s = __ldcg(reinterpret_cast<const uint2*>(&g->gen));
       gen = s.x;  // cannot advance before this block arrives
-      ok = s.y == 0;
       __threadfence();
-      if (ok) last = atomicAdd(&g->arrive, 1u) == gridDim.x - 1;
+      last = atomicAdd(&g->arrive, 1u) == gridDim.x - 1;
+      ok = s.y == 0;  // (looked at after the arrival, which need not wait for it)
+      if (!ok) last = 0;
     }
     last = __shfl_sync(FULL, last, 0);
     if (last) {
