@@ -16,6 +16,7 @@ distance matrix copied back to pinned host memory every step).
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import os
 import statistics
@@ -176,6 +177,19 @@ def level_bytes(rec, V, W, E):
     return (8 * rec["frontier_entries"] + rec["frontier_vertices"] * (8 + row)
             + rec["edges"] * (4 + row) + rec["new_vertices"] * (row + 8)
             + 4 * rec["new_pairs"])
+
+
+def level_traffic(workload, captures=ROOT / "profiles" / "traffic.json",
+                  source=ROOT / "webgpu_bfs_gb300" / "csrc" / "level_kernels.cuh"):
+    """DRAM bytes per level-kernel launch, as captured by ncu; None unless the
+    capture names the level kernels' present source by its hash."""
+    try:
+        entry = json.loads(Path(captures).read_text())[workload]
+        if entry["source_sha256"] != hashlib.sha256(Path(source).read_bytes()).hexdigest():
+            return None
+        return entry["level_kernel"]
+    except (OSError, ValueError, KeyError):
+        return None
 
 
 def cpu_model() -> str:
@@ -470,13 +484,7 @@ def run_ours(args, spec):
         mat_ms = sum(r["event_ms"] for r in mt)
         mat_b = 4 * S * V + sum(4 * W * V * (1 + max(1, r["level"]).bit_length())
                                 for r in mt)
-        traffic = None
-        tf = ROOT / "profiles" / "traffic.json"
-        if tf.exists():
-            try:
-                traffic = json.loads(tf.read_text()).get(args.workload, {}).get("level_kernel")
-            except Exception:
-                traffic = None
+        traffic = level_traffic(args.workload)
         ach = tot_b / (tot_ms / 1000.0) / 1e9 if tot_ms else 0.0
         roof = {"kernel": "level_kernel (push+pull launches)", "bound": "hbm",
                 "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,

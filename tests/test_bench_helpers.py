@@ -1,6 +1,9 @@
 """CPU checks of bench.py's host-side pieces: the served request stream, the
 Poisson arrivals, the latency summary and the algorithmic-bytes model of a
 level (the roofline's numerator)."""
+import hashlib
+import json
+
 import numpy as np
 
 import bench
@@ -130,3 +133,15 @@ def test_both_arms_print_the_same_config(native):
     a = bench.workload_config("road_s256", spec, g)
     b = bench.workload_config("road_s256", spec, g)
     assert a == b and "l2_policy" in a and a["sources"] == 256
+
+
+def test_level_traffic_is_of_the_present_kernels(tmp_path):
+    captures, source = tmp_path / "traffic.json", tmp_path / "kernels.cuh"
+    source.write_text("kernel v2")
+    entry = {"level_kernel": 5, "source_sha256": hashlib.sha256(b"kernel v2").hexdigest()}
+    captures.write_text(json.dumps({"now": entry, "before": {**entry, "source_sha256": "0"},
+                                    "unknown": {"level_kernel": 5}}))
+    assert bench.level_traffic("now", captures, source) == 5
+    for workload in ("before", "unknown", "absent"):
+        assert bench.level_traffic(workload, captures, source) is None
+    assert bench.level_traffic("now", tmp_path / "none.json", source) is None
