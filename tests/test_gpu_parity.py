@@ -592,3 +592,28 @@ def test_traversal_grids_that_do_and_do_not_launch(native, oracle, monkeypatch, 
             assert reach.total_reachable_pairs() == st["reached"].sum()
         finally:
             eng.close()
+
+
+def test_road_graph_of_more_than_2_28_edges(native):
+    """Edge records whose begin does not fit 28 bits: an 8,200 x 8,200 grid
+    (268.9 M edges), from its corners, its middle and a vertex listed twice."""
+    torch = pytest.importorskip("torch")
+    n = 8200
+    grid = native.Grid2D(n, n)
+    assert grid.graph.num_edges > 1 << 28
+    src = np.array([0, n * n - 1, n * n // 2 + n // 2, n - 1, 0], np.uint32)
+    xy = torch.arange(n, device="cuda", dtype=torch.int32)
+    eng = native.GpuBfsEngine()
+    try:
+        out = torch.empty((src.size, n, n), dtype=torch.int32, device="cuda")
+        eng.run_ms_bfs_device(grid.graph, src, out.data_ptr())
+        assert eng.synchronize()["path"] == 4
+        st = eng.run_ms_bfs_stats(grid.graph, src)
+        for s, row, stat in zip(src, out, st):
+            x, y = grid.coordinates(int(s))
+            want = (xy - y).abs()[:, None] + (xy - x).abs()[None, :]
+            assert torch.equal(row, want), s
+            assert stat["reached"] == n * n and stat["eccentricity"] == int(want.max())
+            assert stat["distance_sum"] == int(want.sum())
+    finally:
+        eng.close()

@@ -297,7 +297,7 @@ __device__ void cta_item(const BatchGraph& g, uint32_t s0, uint32_t n, uint32_t*
   const uint32_t bwords = (V + 31) / 32;
   const uint32_t sbits = smem_addr(bitmap), scnt = smem_addr(s_cnt);
   const uint32_t squeue = sbits + (bwords + 1) / 2 * 8, sbig = squeue + 8 * BATCH_QH;
-  const CtaQueue<false> q{squeue, scr, BATCH_QH, V, g.off};
+  const CtaQueue<ER_NONE> q{squeue, scr, BATCH_QH, V, g.off};
   auto mark = [&](uint32_t v, uint32_t bit) { return atoms_or(sbits + (v >> 5) * 4, bit); };
   for (uint32_t si = s0; si < s0 + n; ++si) {
     for (uint32_t i = tid; i < bwords; i += bs) bitmap[i] = 0;
@@ -316,8 +316,8 @@ __device__ void cta_item(const BatchGraph& g, uint32_t s0, uint32_t n, uint32_t*
       reached += n_in;
       const uint32_t nslot = slot == 8 ? 0 : slot + 4;
       if (tid == 0) sts32(scnt + nslot, 0);
-      cta_level<false, BATCH_BLOCK, 2>(nullptr, g.idx, q, level, n_in, scnt + slot, row, mark, sbig,
-                                       scnt + 12);
+      cta_level<ER_NONE, BATCH_BLOCK, 2>(nullptr, g.idx, q, level, n_in, scnt + slot, row, mark,
+                                         sbig, scnt + 12);
       n_in = lds32(scnt + slot);
       slot = nslot;
       ++level;
@@ -594,8 +594,10 @@ int msbfs_batch_create(int device, const msbfs_batch_graph* graphs, size_t n, ms
   // A kernel has one limit in the whole process, so it is the largest batch's,
   // whichever batches are alive.
   constexpr int SMEM_MAX = (int)batch_smem(MSBFS_BATCH_MAX_VERTICES);
-  BCK(cudaFuncSetAttribute(batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-  BCK(cudaFuncSetAttribute(batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+  BCK(cudaFuncSetAttribute(batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SMEM_MAX));
+  BCK(cudaFuncSetAttribute(batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SMEM_MAX));
   int occ = 0, occ_vt = 0, sms = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, BATCH_BLOCK, b->smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_vt, batch_kernel<true>, BATCH_BLOCK, b->smem);

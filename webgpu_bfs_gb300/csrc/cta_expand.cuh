@@ -9,8 +9,10 @@
 namespace msbfs {
 
 constexpr uint32_t CTA_FULL = 0xffffffffu;
+enum : int { ER_NONE = 0, ER_PACKED = 1, ER_WIDE = 2 };
+constexpr uint32_t ER_WIDE_ID = 0x0fffffffu;  // the target's bits of a wide record
 
-// Frontier entries. ER: the graph carries edge records, 8 bytes per edge
+// Frontier entries. ER_PACKED: the graph carries edge records, 8 bytes per edge
 // {target, target's edge range packed as begin << 4 | count} (built once per
 // road-like graph: at most 8 out-edges, fewer than 2^28 edges), and a queue
 // entry is the packed edge range of a frontier vertex instead of its id.
@@ -18,6 +20,11 @@ constexpr uint32_t CTA_FULL = 0xffffffffu;
 // edge records) instead of three (queue entry, offsets, adjacency): on a
 // ~4,000-level road graph the per-level latency chain is what a traversal's
 // time is made of.
+// ER_WIDE, for 2^28 edges and more (and at most 2^28 vertices): the records are
+// {target | its count << 28, target's edge begin}, and a queue entry is the
+// position of the record by which a vertex was found, which its expansion reads
+// again (from the L1, as a rule); the source, without one, is an id. 8200 x 8200
+// grid, S=1 / 32, ms: ids 576 / 1,731, these records 489 / 1,465.
 //
 // Queue: the first `qh` entries of a level's frontier sit in shared memory
 // (two halves, by level parity), the rest in one global slab of V words per
@@ -48,7 +55,7 @@ __device__ __forceinline__ uint32_t atoms_add(uint32_t a, uint32_t x) {
   return r;
 }
 
-template <bool ER>
+template <int ER>
 struct CtaQueue {
   uint32_t sq;     // shared-memory address of the halves
   uint32_t* slab;  // global memory
@@ -63,7 +70,7 @@ struct CtaQueue {
   // The frontier of level 0 (the halves may hold nothing: qh == 0).
   __device__ __forceinline__ void put_source(uint32_t u) const {
     uint32_t x = u;
-    if constexpr (ER) {
+    if constexpr (ER == ER_PACKED) {
       const uint32_t b = __ldg(off + u);
       x = b << 4 | (__ldg(off + u + 1) - b);
     }
@@ -80,7 +87,7 @@ struct CtaQueue {
 // (testing the bit first only adds a step: road 339x338 S=2,048 3.25 -> 3.08
 // ms without it). New vertices get their places with one shared-memory
 // atomicAdd per warp (ballot prefix sums).
-template <bool ER, int BATCH, typename Mark>
+template <int ER, int BATCH, typename Mark>
 __device__ __forceinline__ void cta_discover(const CtaQueue<ER>& q, uint32_t nd, uint32_t cnt,
                                              uint32_t* row, const uint32_t* v, const uint32_t* nx,
                                              bool* fresh, Mark&& mark) {
@@ -148,7 +155,7 @@ struct CtaNoBig {
 // is a multiple of 32, so a warp's entries past n_in are still inside it).
 // `big(e, n)` may take a vertex's edges [e, e + n) over (called by its first
 // lane): they are then left out here.
-template <bool ER, int THREADS, int LPV, int BATCH, typename Mark, typename Big = CtaNoBig>
+template <int ER, int THREADS, int LPV, int BATCH, typename Mark, typename Big = CtaNoBig>
 __device__ __forceinline__ void cta_expand(const uint2* erec, const uint32_t* idx,
                                            const CtaQueue<ER>& q, uint32_t level, uint32_t n_in,
                                            uint32_t cnt, uint32_t* row, Mark&& mark,
@@ -169,12 +176,18 @@ __device__ __forceinline__ void cta_expand(const uint2* erec, const uint32_t* id
       else
         x = *q.slab_at(level, i);
     }
-    if constexpr (ER) {
+    if constexpr (ER == ER_PACKED) {
       e = x >> 4;
       n = i < n_in ? x & 15u : 0u;
     } else if (i < n_in) {
-      e = __ldg(q.off + x);
-      n = __ldg(q.off + x + 1) - e;
+      if (ER == ER_WIDE && level) {
+        const uint2 r = __ldg(erec + x);
+        e = r.y;
+        n = r.x / (ER_WIDE_ID + 1);
+      } else {
+        e = __ldg(q.off + x);
+        n = __ldg(q.off + x + 1) - e;
+      }
     }
     if constexpr (HAS_BIG) {
       bool taken = false;
@@ -189,10 +202,13 @@ __device__ __forceinline__ void cta_expand(const uint2* erec, const uint32_t* id
         v[k] = nx[k] = 0;
         fresh[k] = sub + k * LPV < n;
         if (fresh[k]) {
-          if constexpr (ER) {
+          if constexpr (ER == ER_PACKED) {
             const uint2 r = __ldg(erec + e + sub + k * LPV);
             v[k] = r.x;
             nx[k] = r.y;
+          } else if constexpr (ER == ER_WIDE) {
+            nx[k] = e + sub + k * LPV;
+            v[k] = __ldg(erec + nx[k]).x & ER_WIDE_ID;
           } else {
             v[k] = nx[k] = __ldg(idx + e + sub + k * LPV);
           }
@@ -216,12 +232,12 @@ constexpr size_t BIG_BYTES = BIG_PIECES * 2 * sizeof(uint32_t);
 // edge records keep lists of more than BIG_DEGREE edges for a second sweep
 // (sbig: shared address of BIG_BYTES, 0 for none; spieces: of two counters, by
 // level parity, both 0 before level 0).
-template <bool ER, int THREADS, int LPV, typename Mark>
+template <int ER, int THREADS, int LPV, typename Mark>
 __device__ __forceinline__ void cta_level(const uint2* erec, const uint32_t* idx,
                                           const CtaQueue<ER>& q, uint32_t level, uint32_t n_in,
                                           uint32_t cnt, uint32_t* row, Mark&& mark, uint32_t sbig,
                                           uint32_t spieces) {
-  if constexpr (ER) {
+  if constexpr (ER != ER_NONE) {
     cta_expand<ER, THREADS, LPV, 4 / LPV>(erec, idx, q, level, n_in, cnt, row, mark);
     __syncthreads();
   } else {

@@ -88,7 +88,7 @@ constexpr int CTA_CLUSTER_LPV = 1;
 // s_cnt[(L+1) % 3] during level L (last read right after the barrier of
 // level L-2), so a level needs one block barrier. The per-source statistics
 // follow from the frontier sizes, which every thread knows.
-template <bool GB, bool ER, int FORM>
+template <bool GB, int ER, int FORM>
 __global__ void __launch_bounds__(CtaForm<FORM>::THREADS, CtaForm<FORM>::MINB)
     cta_bfs_kernel(CtaParams p) {
   constexpr int THREADS = CtaForm<FORM>::THREADS, LPV = CtaForm<FORM>::LPV;
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(CtaForm<FORM>::THREADS, CtaForm<FORM>::MINB)
 // index is in every block and every slice is zero, (2) the traversal is done.
 // The queue (shared-memory halves in rank 0, then one global slab of V words
 // per cluster) and the edge records work as in cta_bfs_kernel.
-template <int CL, bool ER>
+template <int CL, int ER>
 __global__ void __launch_bounds__(CTA_CLUSTER_THREADS, 1) cta_cluster_kernel(CtaParams p) {
   extern __shared__ __align__(16) uint32_t smem_dyn[];
   __shared__ uint32_t s_src_idx;  // written into every block by rank 0
@@ -255,20 +255,28 @@ __global__ void __launch_bounds__(CTA_CLUSTER_THREADS, 1) cta_cluster_kernel(Cta
 }
 
 // Edge records of a road-like graph: for every edge e = (u, v), {v, off[v] <<
-// 4 | out-degree of v}. One thread per vertex u.
+// 4 | out-degree of v}, or, wide, {v | out-degree of v << 28, off[v]}. One thread
+// per vertex u.
 __global__ void edge_records_kernel(uint32_t V, const uint32_t* __restrict__ off,
-                                    const uint32_t* __restrict__ idx, uint2* __restrict__ erec) {
+                                    const uint32_t* __restrict__ idx, uint2* __restrict__ erec,
+                                    bool wide) {
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < V; u += gridDim.x * blockDim.x) {
     for (uint32_t e = off[u]; e < off[u + 1]; ++e) {
       const uint32_t v = idx[e];
-      erec[e] = make_uint2(v, off[v] << 4 | (off[v + 1] - off[v]));
+      const uint32_t b = off[v], n = off[v + 1] - b;
+      erec[e] = wide ? make_uint2(n * (ER_WIDE_ID + 1) | v, b) : make_uint2(v, b << 4 | n);
     }
   }
 }
 
+int edge_record_kind(size_t V, size_t E) {
+  if (E < (size_t(1) << 28)) return ER_PACKED;
+  return V <= (size_t)ER_WIDE_ID + 1 ? ER_WIDE : ER_NONE;
+}
+
 void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, uint2* erec,
-                         cudaStream_t s) {
-  edge_records_kernel<<<1024, 256, 0, s>>>(V, off, idx, erec);
+                         int kind, cudaStream_t s) {
+  edge_records_kernel<<<1024, 256, 0, s>>>(V, off, idx, erec, kind == ER_WIDE);
 }
 
 constexpr size_t CTA_SMEM_RESERVE = 1024;  // static shared variables and slack
@@ -288,7 +296,7 @@ static cudaError_t allow_smem(void* fn, int optin) {
                               optin - (int)CTA_SMEM_RESERVE);
 }
 
-template <bool GB, bool ER>
+template <bool GB, int ER>
 static void* cta_fn(int form) {
   if constexpr (!GB) {
     if (form == CTA_TPUT) return (void*)cta_bfs_kernel<GB, ER, CTA_TPUT>;
@@ -299,21 +307,23 @@ static void* cta_fn(int form) {
 }
 
 static void* cta_kernel(const CtaShape& sh) {
-  if (sh.global_bits)
-    return sh.edge_records ? cta_fn<true, true>(sh.form) : cta_fn<true, false>(sh.form);
-  return sh.edge_records ? cta_fn<false, true>(sh.form) : cta_fn<false, false>(sh.form);
+  if (sh.global_bits)  // (the only mode of graphs with wide records: they have 2^26 vertices)
+    return sh.edge_records == ER_WIDE     ? cta_fn<true, ER_WIDE>(sh.form)
+           : sh.edge_records == ER_PACKED ? cta_fn<true, ER_PACKED>(sh.form)
+                                          : cta_fn<true, ER_NONE>(sh.form);
+  return sh.edge_records ? cta_fn<false, ER_PACKED>(sh.form) : cta_fn<false, ER_NONE>(sh.form);
 }
 
-template <int CL, bool ER>
+template <int CL, int ER>
 static void* cta_cluster_fn() {
   return (void*)cta_cluster_kernel<CL, ER>;
 }
 
 static void* cluster_kernel(int cl, bool er) {
   switch (cl) {
-    case 2: return er ? cta_cluster_fn<2, true>() : cta_cluster_fn<2, false>();
-    case 4: return er ? cta_cluster_fn<4, true>() : cta_cluster_fn<4, false>();
-    case 8: return er ? cta_cluster_fn<8, true>() : cta_cluster_fn<8, false>();
+    case 2: return er ? cta_cluster_fn<2, ER_PACKED>() : cta_cluster_fn<2, ER_NONE>();
+    case 4: return er ? cta_cluster_fn<4, ER_PACKED>() : cta_cluster_fn<4, ER_NONE>();
+    case 8: return er ? cta_cluster_fn<8, ER_PACKED>() : cta_cluster_fn<8, ER_NONE>();
     default: return nullptr;
   }
 }
@@ -349,7 +359,7 @@ static int cluster_capacity(int cl, bool er, size_t smem, int block, int optin) 
 // Cluster mode for a call of few sources: the smallest cluster whose slices
 // hold the bitmap next to rank 0's queue halves. MSBFS_CTA_CLUSTER=0 turns
 // it off, =1 uses it whatever the number of sources.
-static bool cta_cluster_shape(uint32_t V, int optin, bool edge_records, size_t num_sources,
+static bool cta_cluster_shape(uint32_t V, int optin, int edge_records, size_t num_sources,
                               uint32_t sm_share, CtaShape* out) {
   const char* env = getenv("MSBFS_CTA_CLUSTER");
   const int mode = env ? atoi(env) : -1;
@@ -383,7 +393,7 @@ static bool cta_cluster_shape(uint32_t V, int optin, bool edge_records, size_t n
   return false;
 }
 
-bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_records,
+bool cta_launch_shape(uint32_t V, int device, bool allow_global, int edge_records,
                       size_t num_sources, uint32_t sm_share, CtaShape* out) {
   int sms = 0, optin = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -555,7 +565,7 @@ extern "C" int msbfs_run_cta_noalloc(int device, size_t num_vertices,
   }
   const uint32_t V = (uint32_t)num_vertices;
   CtaShape sh{};
-  if (!cta_launch_shape(V, device, /*allow_global=*/false, /*edge_records=*/false, num_sources,
+  if (!cta_launch_shape(V, device, /*allow_global=*/false, /*edge_records=*/ER_NONE, num_sources,
                         /*sm_share=*/100, &sh))
     return MSBFS_ERR_SCRATCH_TOO_SMALL;
   const size_t slabs = (NOALLOC_WORDS - NOALLOC_Q_OFF) / (size_t)V;

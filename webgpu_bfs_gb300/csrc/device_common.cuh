@@ -237,7 +237,7 @@ struct CtaParams {
   uint32_t* gbits;       // global-bitmap mode: per resident block ceil(V/32) u32
   uint32_t big;          // long lists' pieces sit after the queue halves (set at launch)
   uint32_t qh;           // frontier entries per shared-memory queue half (set at launch)
-  const uint2* erec;     // per edge {target, target's edge begin << 4 | count}, or null
+  const uint2* erec;     // edge records (cta_expand.cuh), or null
 };
 struct CtaShape {
   int grid = 0;           // blocks: those resident at the SM share, or fewer
@@ -247,7 +247,7 @@ struct CtaShape {
   int form = 0;           // block form (threads, lanes per vertex) of cta_kernel.cu
   int minb = 1;           // resident blocks per SM the queue halves leave room for
   bool global_bits = false;
-  bool edge_records = false;
+  int edge_records = 0;   // their kind
   bool big = false;       // room for long lists' pieces after the queue halves
   int cluster = 0;        // > 1: blocks per cluster sharing one source's bitmap
 };
@@ -259,11 +259,13 @@ struct CtaShape {
 // the device holds at once. In cluster mode `grid`
 // counts blocks (a multiple of `cluster`) and each cluster has one queue slab.
 size_t cta_max_vertices(int device);
-bool cta_launch_shape(uint32_t V, int device, bool allow_global, bool edge_records,
+bool cta_launch_shape(uint32_t V, int device, bool allow_global, int edge_records,
                       size_t num_sources, uint32_t sm_share, CtaShape* out);
 void launch_cta(const CtaParams& p, const CtaShape& sh, int grid, cudaStream_t s);
+// Kind of the edge records of a road-like graph (0: too large for any).
+int edge_record_kind(size_t V, size_t E);
 void launch_edge_records(uint32_t V, const uint32_t* off, const uint32_t* idx, uint2* erec,
-                         cudaStream_t s);
+                         int kind, cudaStream_t s);
 
 void launch_traversed_edges(uint32_t V, const uint32_t* off, const uint32_t* dist,
                             uint32_t num_sources, unsigned long long* out, cudaStream_t s);

@@ -72,8 +72,8 @@ struct msbfs_graph {
   // Bottom-up work order: vertices with 0 < in-degree < heavy, ascending ids.
   uint32_t n_order = 0;
   uint4* order = nullptr;  // {vertex, in-edge begin, in-edge end, 0}
-  // Road-like graphs: per edge {target, target's edge begin << 4 | count}.
-  uint2* erec = nullptr;
+  uint2* erec = nullptr;  // edge records of road-like graphs (CTA path)
+  int erec_kind = 0;
   std::vector<uint32_t> h_coff;  // host CSC offsets (V + 1): rebuilds the tables above
 };
 
@@ -606,7 +606,7 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
   if (reach_dev && path == MSBFS_PATH_CTA) path = MSBFS_PATH_HYBRID;
   CtaShape cta{};
   if (path == MSBFS_PATH_CTA &&
-      !cta_launch_shape((uint32_t)g->V, eng->device, true, g->erec != nullptr, S, eng->sm_share, &cta))
+      !cta_launch_shape((uint32_t)g->V, eng->device, true, g->erec_kind, S, eng->sm_share, &cta))
     path = MSBFS_PATH_HYBRID;
   if (!g->sym && path != MSBFS_PATH_CTA && !g->coff)
     return set_err(eng, MSBFS_ERR_INVALID_GRAPH, "missing transpose");
@@ -1001,11 +1001,10 @@ int upload_graph(msbfs_engine* eng, size_t V, size_t E, const uint32_t* off, con
   if (rc) return rc;
   // Road-like graphs (the ones the router sends to the CTA path) get edge
   // records, 8 bytes per edge, so a CTA-path level costs one dependent L2
-  // round trip instead of three. The packed edge range holds 28 bits of edge
-  // index and at most 15 out-edges (road-like: at most 8).
-  if (is_road_like(g.get()) && E > 0 && E < (size_t(1) << 28)) {
+  // round trip instead of three.
+  if (is_road_like(g.get()) && E > 0 && (g->erec_kind = edge_record_kind(V, E))) {
     CK(device_alloc(eng, (void**)&g->erec, E * sizeof(uint2)));
-    launch_edge_records((uint32_t)V, g->off, g->idx, g->erec, eng->stream);
+    launch_edge_records((uint32_t)V, g->off, g->idx, g->erec, g->erec_kind, eng->stream);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(eng->stream));
   }
