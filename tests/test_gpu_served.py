@@ -244,3 +244,31 @@ def test_express_requests_complete_beside_general_traversals(native, percent):
             assert info["status"] == 0 and (res["eccentricity"] == n - 1).all()
     finally:
         srv.close()
+
+
+def test_sm_share_leaves_room_for_another_engine(native):
+    """Rows by an engine held to 15% of the SMs while one held to 85% traverses
+    a path of 350,000 levels: they do not wait for its end."""
+    torch = pytest.importorskip("torch")
+    path, small = native.path_graph(350_000), native.generate_graph500_rmat(12, 8, 1)
+    rows = [torch.empty(g.num_vertices, dtype=torch.int32, device="cuda") for g in (path, small)]
+    push = native.GpuBfsMethod.MultiWordBitParallelPush
+    a, b = native.GpuBfsEngine(push), native.GpuBfsEngine(push)
+    try:
+        a.set_sm_share(85)
+        b.set_sm_share(15)
+        for eng, g, out in ((a, path, rows[0]), (b, small, rows[1])):  # workspaces built
+            eng.run_ms_bfs_device(g, [1], out.data_ptr())
+            eng.synchronize()
+        a.run_ms_bfs_device(path, [0], rows[0].data_ptr())
+        a_end = threading.Thread(target=a.synchronize)
+        a_end.start()
+        for _ in range(3):
+            b.run_ms_bfs_device(small, [1], rows[1].data_ptr())
+            b.synchronize()
+        assert a_end.is_alive()
+        a_end.join()
+        assert int(rows[0].max()) == 349_999
+    finally:
+        a.close()
+        b.close()

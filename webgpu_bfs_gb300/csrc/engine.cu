@@ -729,7 +729,8 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
       int blocks = w->k.traverse_grid;
       if (eng->traverse_cap < 100)
         blocks = std::min(blocks, std::max(1, (int)((uint64_t)w->k.traverse_resident * eng->traverse_cap / 100)));
-      const cudaError_t launched = launch_traverse(w->p, w->k, blocks, eng->traverse_cap < 100, eng->stream);
+      const cudaError_t launched = launch_traverse(
+          w->p, w->k, blocks, eng->sm_share < 100 || eng->traverse_cap < 100, eng->stream);
       const bool refused = launched == cudaErrorCooperativeLaunchTooLarge ||
                            launched == cudaErrorLaunchOutOfResources ||
                            launched == cudaErrorNotSupported;
