@@ -487,6 +487,7 @@ def run_ours(args, spec):
         traffic = level_traffic(args.workload)
         ach = tot_b / (tot_ms / 1000.0) / 1e9 if tot_ms else 0.0
         roof = {"kernel": "level_kernel (push+pull launches)", "bound": "hbm",
+                "limited_by": "latency of dependent gathers (achieved counts the rows that caches serve)",
                 "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                 "peak_source": f"{peak_kind} hbm_gbs", "traffic": traffic,
                 "launches": len(lv), "avg_launch_ms": tot_ms / max(1, len(lv)),

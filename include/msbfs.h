@@ -168,8 +168,9 @@ int msbfs_engine_set_tuning(msbfs_engine *engine, uint32_t max_words_per_pass,
  * per vertex of a pass, alpha, beta, the in-edge slice length of bottom-up
  * steps, the frontier-bitmap threshold and the in-degree from which a whole
  * warp scans a vertex -- keeping a change only when it is
- * faster, then applies the best settings to the engine (and the slice length
- * to the graph). With a cache path, a class already in the file is applied
+ * faster, then applies the best settings to the engine (slice length and
+ * in-degree to the graph); words that stay at their default keep following
+ * each graph's size. With a cache path, a class already in the file is applied
  * without timing and new classes are appended. Results never depend on the
  * settings. Calls that the router sends to the CTA-per-source path are not
  * tuned (the settings do not apply to it). */
@@ -191,9 +192,13 @@ int msbfs_engine_autotune(msbfs_engine *engine, msbfs_graph *graph, const uint32
                           size_t num_sources, const char *cache_path, msbfs_tuning *out);
 
 /* Caps the persistent kernels' grids at `percent` (1..100, default 100) of
- * the blocks that fit the device at once, leaving the rest of the SMs to
- * kernels of other streams (the served form gives them to its express
- * slots). No reference counterpart. Results do not depend on it. */
+ * the blocks that fit the device at once, leaving the rest to kernels of other
+ * streams (the served form gives it to its express slots). A level-path
+ * traversal is one cooperative launch: it starts when all its blocks fit beside
+ * what runs, so the traversals of engines whose shares add up to more than 100
+ * run one after the other, and other kernels start beside it as far as their
+ * blocks fit what it leaves. No reference counterpart. Results do not depend
+ * on it. */
 int msbfs_engine_set_sm_share(msbfs_engine *engine, uint32_t percent);
 
 /* Caps the levels of one level-synchronous pass (0, the default, = V + 2,
@@ -210,10 +215,11 @@ int msbfs_engine_set_level_cap(msbfs_engine *engine, uint32_t max_levels);
 /* Profiling: 0 off; 1 keep a per-level record of every call (device timers
  * and the work counters of the algorithmic-bytes model; the level loop is
  * driven from the host, one launch of the level kernels' counting form a
- * level); 2 as 1, with CUDA events around each launch; 3 as 2 with the production level kernels, which keep
- * no work counters (the records carry durations, frontier sizes and
- * discovered pairs only). msbfs_engine_level_log copies the last call's
- * records. */
+ * level); 2 as 1, with CUDA events around each launch; 3 as 2 with the
+ * production level kernels, which keep no work counters (the records carry
+ * durations, frontier sizes and discovered pairs only). Bottom-up levels keep
+ * no queue: their frontier_entries are 0. msbfs_engine_level_log copies the
+ * last call's records. */
 int msbfs_engine_set_profiling(msbfs_engine *engine, int level);
 int msbfs_engine_level_log(const msbfs_engine *engine, msbfs_level_record *out,
                            size_t capacity, size_t *count);
@@ -315,7 +321,11 @@ int msbfs_run_ms_bfs_stats(msbfs_engine *engine, const msbfs_graph *graph,
  * highest-priority streams; the other slots take large requests first, in
  * arrival order, and small ones only when no large request waits. Their
  * persistent kernels use general_sm_percent of the resident grid
- * (msbfs_engine_set_sm_share) so express kernels find SMs free. */
+ * (msbfs_engine_set_sm_share). Below 100, with express slots, no more of their
+ * level-path traversals are on the device at once than fit that share (at
+ * least 85%), and express traversals beside them take what is left, so that an
+ * express request never waits for the end of a general one. At 100 nothing is
+ * left: it waits for the traversals under way. */
 #define MSBFS_SERVE_ROWS 0  /* out = S*V u32 distance rows          */
 #define MSBFS_SERVE_STATS 1 /* out = S msbfs_source_stats           */
 typedef struct msbfs_server msbfs_server;

@@ -62,8 +62,12 @@ struct CtaForm {
   static constexpr int MINB = FORM == CTA_WIDE ? 1 : FORM == CTA_TPUT ? MSBFS_CTA_TPUT_MINB : 3;
   static constexpr int LPV = FORM <= CTA_SMALL ? 4 : 2;
 };
-// Vertices from which one block per SM is the wide one: about the graph whose
-// frontiers (of the order of the square root) exceed the small one's sweep.
+// Vertices from which one block per SM is the wide one: where frontiers (of the
+// order of the square root) exceed the small one's sweep. us of a statistics call,
+// wide / small, grids S=1, S=64, roads S=1, S=64: 8,100 vertices 89 / 89, 126 / 125,
+// 104 / 101, 178 / 165; 16,384 114 / 128, 174 / 163, 166 / 164, 237 / 223; 25,600
+// 161 / 178, 212 / 225, 211 / 237, 326 / 311; 32,761 198 / 224, 248 / 275, 238 /
+// 265, 324 / 323; 65,536 324 / 383, 360 / 423, 362 / 447, 445 / 508.
 constexpr size_t CTA_WIDE_VERTICES = 32768;
 constexpr size_t CTA_MID_BLOCKS = 3;  // most blocks per SM of the middle form
 // Global-bitmap mode keeps its per-block scratch (queue slab + bitmap) within

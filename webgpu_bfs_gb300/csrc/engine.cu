@@ -860,7 +860,7 @@ int finish_call(msbfs_engine* eng, msbfs_stats* stats) {
 // (1.7) 0.421 / 0.467, R-MAT 13 S=200 (0.03) 0.110 / 0.133. Against 64, 128 is
 // 1-2% slower on R-MAT 21 and 22; 16 loses to 32 on R-MAT 20 and larger.
 uint32_t warp_scan_degree(const msbfs_engine* eng, const std::vector<uint32_t>& coff) {
-  constexpr size_t LEVEL_WARPS_PER_SM = 48;
+  constexpr size_t LEVEL_WARPS_PER_SM = 48;  // resident: 6 blocks of 8 (level_kernels.cuh)
   size_t mid = 0;
   for (size_t v = 0; v + 1 < coff.size(); ++v) mid += coff[v + 1] - coff[v] - 32 < 32;
   return mid >= 3 * LEVEL_WARPS_PER_SM * (size_t)eng->num_sms ? 64 : 32;
@@ -885,7 +885,7 @@ int build_bottom_up_tables(msbfs_engine* eng, msbfs_graph* g, uint32_t split, ui
   g->split = split;
   g->n_heavy = 0;
   // A slice is one warp's serial work. With less than a full slice of edges
-  // per resident warp, shorter ones: a level of a small graph lasts as long
+  // per warp slot of the device (64 an SM), shorter ones: a level of a small graph lasts as long
   // as its longest slice (directed R-MAT 18, S=333: bottom-up levels of 220 us
   // behind warps that scanned up to 16 vertices of <= 512 in-edges). Not below
   // 256: a list's slices meet in its candidate words, two fences and an atomic
