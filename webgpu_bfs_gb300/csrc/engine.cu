@@ -184,7 +184,7 @@ struct msbfs_engine {
   // Polls of a grid barrier before the traversal gives up (tens of seconds;
   // MSBFS_BARRIER_SPINS), and the word that it then sets (page-locked).
   uint32_t barrier_spins = 1u << 26;
-  uint32_t* h_stuck = nullptr;
+  uint32_t* h_stuck = nullptr;  // (comes with the first level-path call)
   bool zero_copy = true;  // MSBFS_ZERO_COPY=0 stages host output in HBM instead
   bool narrow = true;     // MSBFS_NARROW=0 keeps host-bound rows u32 over the link
   int profiling = 0;
@@ -222,7 +222,7 @@ struct msbfs_engine {
   unsigned long long* d_counter = nullptr;
   SourceStats* d_sstats = nullptr;  // per-source reductions of host-output calls
   size_t d_sstats_cap = 0;
-  LevelCtl* h_ctl = nullptr;  // pinned, one per pass of the last call
+  LevelCtl* h_ctl = nullptr;  // one per pass of the last call, in h_stuck's allocation
   size_t h_ctl_cap = 0;
   // last call
   msbfs_stats last{};
@@ -350,10 +350,6 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
         o = o->second->W > PLAIN_WORDS ? eng->ws.erase(o) : std::next(o);
     }
   }
-  if (!eng->h_stuck) {
-    CK(cudaHostAlloc((void**)&eng->h_stuck, sizeof(uint32_t), cudaHostAllocMapped));
-    *eng->h_stuck = 0;
-  }
   auto w = std::make_unique<Workspace>();
   w->graph_id = g->id;
   w->W = W;
@@ -431,7 +427,6 @@ int get_workspace(msbfs_engine* eng, const msbfs_graph* g, uint32_t W, uint32_t 
   if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(GridSync)))) return rc;
   p.sync = (GridSync*)ptr;
   p.spins = eng->barrier_spins;
-  CK(cudaHostGetDevicePointer((void**)&p.h_stuck, eng->h_stuck, 0));
   if ((rc = dev_alloc(eng, w.get(), &ptr, sizeof(LevelRec) * LOG_CAP))) return rc;
   w->d_log = (LevelRec*)ptr;
   p.log = w->d_log;
@@ -681,10 +676,16 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
   }
   if (passes > eng->h_ctl_cap) {
     CK(cudaStreamSynchronize(eng->stream));
-    if (eng->h_ctl) cudaFreeHost(eng->h_ctl);
+    const uint32_t stuck = eng->h_stuck ? *eng->h_stuck : 0u;
+    if (eng->h_stuck) cudaFreeHost(eng->h_stuck);
+    eng->h_stuck = nullptr;
     eng->h_ctl = nullptr;
     eng->h_ctl_cap = 0;
-    CK(cudaMallocHost((void**)&eng->h_ctl, passes * sizeof(LevelCtl)));
+    char* at = nullptr;
+    CK(cudaMallocHost((void**)&at, alignof(LevelCtl) + passes * sizeof(LevelCtl)));
+    eng->h_stuck = reinterpret_cast<uint32_t*>(at);
+    *eng->h_stuck = stuck;
+    eng->h_ctl = reinterpret_cast<LevelCtl*>(at + alignof(LevelCtl));
     eng->h_ctl_cap = passes;
   }
   eng->last.passes = (uint32_t)passes;
@@ -720,6 +721,7 @@ int enqueue_call(msbfs_engine* eng, int method, const msbfs_graph* g, const uint
     d.row_split = split ? (uint32_t)(split_frac * (double)np) / 32u * 32u : 0u;
     eng->split_rows[ps] = d.row_split;
     w->p.d = d;
+    w->p.h_stuck = eng->h_stuck;
     if ((rc = next_epoch(eng, w))) return rc;
     if (eng->profiling >= 2) {
       if ((rc = run_pass_profiled(eng, w, reduce, &eng->pass_event_ms[ps]))) return rc;
@@ -1312,7 +1314,6 @@ void msbfs_engine_destroy(msbfs_engine* e) {
   cudaFree(e->d_work);
   cudaFree(e->d_counter);
   cudaFree(e->d_sstats);
-  if (e->h_ctl) cudaFreeHost(e->h_ctl);
   if (e->h_log) cudaFreeHost(e->h_log);
   if (e->h_stuck) cudaFreeHost(e->h_stuck);
   for (cudaEvent_t ev : e->lvl_events) cudaEventDestroy(ev);

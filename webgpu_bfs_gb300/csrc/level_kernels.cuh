@@ -1766,10 +1766,10 @@ void fill_level_info(int num_sms, uint32_t NP, LevelKernelInfo* k) {
   k->mat_block = MAT_BLOCK;
   k->mat_smem = materialize_smem_bytes(W, NP);
   k->mat_grid = resident(k->materialize, MAT_BLOCK, k->mat_smem);
-  for (int i = 0; i < 2; ++i) {
-    k->red_block[i] = i ? RED_BLOCK_NARROW : RED_BLOCK;
-    k->red_grid[i] = resident(k->reduce[i], k->red_block[i], 0);
-  }
+  k->red_block[0] = RED_BLOCK;
+  k->red_block[1] = RED_BLOCK_NARROW;
+  k->red_grid[0] = resident(k->reduce[0], RED_BLOCK, 0);
+  k->red_grid[1] = k->red_grid[0] * (RED_BLOCK / RED_BLOCK_NARROW);  // as many threads
 }
 
 }  // namespace msbfs
